@@ -64,15 +64,14 @@ def parse():
 from gemini_unified_b200.pipeline import contiguous_runs, cost_blocks, zigzag  # noqa: E402  (frequency splits)
 
 
-def sched_names(tune):
+def sched_names(tune, backend):
     """Autotuned schedule per phase (toroidal, spheroidal, adjoint) as
-    'threads[+cache]/defer<lanes>,<steps>/q<lane run> or /qblock<block run>' strings."""
+    'threads/defer<lanes>,<steps>/q<lane run> or /qblock<block run>' strings."""
     from gemini_unified_b200.fk import DEFERRALS, GRANULARITIES, SCHEDULES
     def gran(q):
         lane, block = GRANULARITIES[q]
         return "q%d" % lane if not block else "qblock%d" % block
-    return ["%d%s/defer%d,%d/%s" % (SCHEDULES[s][0], "+cache" if SCHEDULES[s][1] else "", DEFERRALS[d][0],
-                                    DEFERRALS[d][1], gran(q))
+    return ["%d/defer%d,%d/%s" % (SCHEDULES[s][0 if backend == 2 else 1], DEFERRALS[d][0], DEFERRALS[d][1], gran(q))
             for s, d, q in zip(tune["schedule"], tune["defer"], tune["queue"])]
 
 
@@ -295,10 +294,8 @@ def main():
 
     # ---------------- batched + mixed-precision form (fast FP64 build): the headline
     fast = GeminiFK(m, ex, device=local, backend=2)
-    # the autotuner picks each phase's schedule (block size, matrix caching) and
-    # bookkeeping deferral on the whole band, untimed.  On the top quarter alone the two
-    # best spheroidal schedules differ by less than the run-to-run noise (262 against
-    # 265 ms) while over the whole band they differ by 5% (380 against 399 ms).
+    # the autotuner picks each phase's schedule (block size) and bookkeeping deferral on
+    # the whole band, untimed
     tune_fast = fast.autotune(w.params, jre, g.nf1, g.nf2)
     for _ in range(args.warmup):
         fk_step(fast)
@@ -358,7 +355,7 @@ def main():
             "config": {"workload": args.workload, "solves_per_step": total_items, "frequencies": int(g.nf2 - g.nf1 + 1),
                        "lmax": int(g.nwn.max() - 1), "nodes": int(ex.nnod), "parallelism": "frequency zig-zag over %d GPU(s)" % size,
                        "form": "fast FP64 build (FMA, Horner spline table, reciprocals); batched phase kernels",
-                       "schedule": {"fast": sched_names(tune_fast), "plain": sched_names(tune_plain),
+                       "schedule": {"fast": sched_names(tune_fast, 2), "plain": sched_names(tune_plain, 1),
                                     "tuned_on_jf": tune_fast["jf"]},
                        "l2": "flushed between steps (256 MiB write); outputs (1.9 GB) exceed L2"},
             "plain_fp64": {"value": plain_value, "unit": "solves/s", "ms_per_step": t_plain, "steps": plain_steps,

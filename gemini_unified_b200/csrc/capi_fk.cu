@@ -32,7 +32,7 @@ struct gem_ctx {
   // model (1-based host copies)
   bool have_model = false;
   double fref = 1, rearth = 0, ric = 0, roc = 0;
-  int aniflag = 0, fsflag = 0, equidis = 0, nlay = 0, nk = 0, nic = 0, noc = 0;
+  int aniflag = 0, iso = 0, fsflag = 0, equidis = 0, nlay = 0, nk = 0, nic = 0, noc = 0;
   std::vector<int> iflso, iktop, ikbot;
   std::vector<double> rb, drk, rk, ro, vpv, vph, vsv, vsh, eta, qkinv, qminv;
   // device copies of the knot arrays (1-based)
@@ -301,6 +301,9 @@ int gem_model_load(gem_ctx* ctx, const gem_model_desc* m) {
   } else {
     cp(ctx->vpv, m->vpv); cp(ctx->vph, m->vph); cp(ctx->vsv, m->vsv); cp(ctx->vsh, m->vsh); cp(ctx->eta, m->eta);
   }
+  ctx->iso = 1;
+  for (int i = 1; i <= K; ++i)
+    if (ctx->vph[i] != ctx->vpv[i] || ctx->vsh[i] != ctx->vsv[i] || ctx->eta[i] != 1.0) ctx->iso = 0;
   for (int i = 1; i <= K; ++i)
     if (!std::isfinite(ctx->ro[i]) || !std::isfinite(ctx->vpv[i]) || !std::isfinite(ctx->vsv[i]) ||
         !std::isfinite(ctx->rk[i]))
@@ -409,6 +412,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   P.rearth = ctx->rearth; P.ric = ctx->ric; P.roc = ctx->roc; P.rhs = ctx->rb[1];
   P.ruc = P.hasocean ? ctx->rb[ctx->nlay - 1] : ctx->rearth;
   P.eps = p->eps; P.sigma = g.sigma; P.df = g.df; P.dwn = g.dwn;
+  P.iso = ctx->iso;
   P.kopt = ctx->backend == GEM_BACKEND_GPU_FAST ? ctx->kopt : 6;
   for (int i = 1; i <= ctx->nlay; ++i) {
     P.rb[i] = ctx->rb[i]; P.drk[i] = ctx->drk[i]; P.iflso[i] = ctx->iflso[i]; P.iktop[i] = ctx->iktop[i];
@@ -482,7 +486,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
     S.defer[ph] = ctx->defer[fast ? 1 : 0][ph];
     S.qgran[ph] = ctx->qgran[fast ? 1 : 0][ph];
     S.grid[ph] = ctx->nsm * (fast ? gem_fast::fk_phase_blocks_per_sm(ph, sc) : gem_plain::fk_phase_blocks_per_sm(ph, sc));
-    nthreads = std::max(nthreads, (long long)S.grid[ph] * FK_SCHED_BLOCK[sc]);
+    nthreads = std::max(nthreads, (long long)S.grid[ph] * FK_SCHED_BLOCK[fast ? 1 : 0][sc]);
   }
   size_t scratch_n = (size_t)nthreads * ((ctx->nnod + 1) * gem_plain::fk_lane_slot_per_node() + FK_LANE_STEP_SLOTS);
   if (grow(ctx, ctx->d_scratch, ctx->scratch_cap, scratch_n)) return GEM_ERROR;
@@ -500,7 +504,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   L.adv_min = 1; L.adv_wait = 0; L.qgran = 1; L.qchunk = 0;
   L.nsrc = 0; L.src_blk = 0;
   ctx->last_grid = S.grid[1];
-  ctx->last_block = FK_SCHED_BLOCK[S.sched[1]];
+  ctx->last_block = FK_SCHED_BLOCK[fast ? 1 : 0][S.sched[1]];
   // ---- learned proposer: features / proposals per (phase, item) from the start radii
   S.propose = fast && ctx->prop_use != 0 && ctx->d_propw;
   if (ctx->dump_feat || S.propose) {
@@ -997,7 +1001,7 @@ int gem_proposer_dump_read(gem_ctx* ctx, float* out, long long cap, long long* n
 }
 
 // Solver schedules (no counterpart in the reference): per phase (toroidal,
-// spheroidal, adjoint) an index into FK_SCHED_BLOCK / FK_SCHED_BIGCACHE, kept
+// spheroidal, adjoint) an index into FK_SCHED_BLOCK, kept
 // per backend.  Every schedule gives bit-identical spectra; only the time differs.
 int gem_fk_schedule_set(gem_ctx* ctx, const int* sched3) {
   if (!ctx || !sched3) return GEM_ERROR;

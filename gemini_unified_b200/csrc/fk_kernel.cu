@@ -172,7 +172,8 @@ __global__ void poly_kernel(PrepArgs A, double* poly) {
       c2 = 0.5 * s1;
       c3 = (s2 - s1) / (6.0 * h);
     }
-    q[4 * v + 0] = c3; q[4 * v + 1] = c2; q[4 * v + 2] = c1; q[4 * v + 3] = c0;
+    double* o = q + 4 * (v == 0 ? 0 : poly_value((v - 1) / 2) + (v - 1) % 2);
+    o[0] = c3; o[1] = c2; o[2] = c1; o[3] = c0;
   }
 }
 

@@ -6,15 +6,15 @@
 
 namespace gem {
 
-// Schedules of a solver phase kernel (one block per SM): threads per block,
-// and whether the 4- and 5-variable systems keep their half- and end-step
-// matrices across the attempts of a Bulirsch-Stoer step (fast build; the
-// 2-variable systems always do, the plain build never).  The autotuner picks
-// one per phase; defaults measured at the batched configuration.
+// Schedules of a solver phase kernel: threads per block (one block per SM) of
+// the plain and of the fast build.  The autotuner picks one per phase; the
+// defaults are the fastest of the first three at the batched configuration
+// (fast build, toroidal / spheroidal / adjoint phase in ms: 256 threads 65.6 /
+// 203 / 107, 384 threads 56.2 / 210 / 99.8, 512 threads 55.3 / 210 / 108; of
+// small slabs every phase is fastest at 256).  The plain build tries 0..2 only.
 constexpr int FK_NSCHED = 6;
-constexpr int FK_SCHED_BLOCK[FK_NSCHED] = {384, 512, 256, 384, 512, 256};
-constexpr int FK_SCHED_BIGCACHE[FK_NSCHED] = {0, 0, 0, 1, 1, 1};
-constexpr int FK_SCHED_DEFAULT[3] = {1, 0, 1};   // toroidal 512, spheroidal 384, adjoint 512 threads
+constexpr int FK_SCHED_BLOCK[2][FK_NSCHED] = {{384, 512, 256, 384, 512, 256}, {256, 384, 512, 320, 448, 192}};
+constexpr int FK_SCHED_DEFAULT[3] = {1, 0, 1};   // toroidal, spheroidal, adjoint
 // candidate deferrals of the bookkeeping passes (lanes waiting, trips waited);
 // the last waits for the whole warp: its lanes, on adjacent degrees of one
 // frequency, reach their sub-interval ends within a few steps of each other
@@ -31,8 +31,8 @@ constexpr int FK_QCHUNK[FK_NGRAN] = {0, 0, 0, 1024};
 constexpr int FK_GRAN_DEFAULT = 0;
 constexpr int MAX_LAYER_KNOTS = 64;    // knots per layer handled by the spline kernel
 // per-lane scratch elements (double2) of one Bulirsch-Stoer step, after the
-// lane's node storage: A(x0) y0 and the last level of the Neville diagonal
-constexpr int FK_LANE_STEP_SLOTS = 10;
+// lane's node storage: A(x0) y0 and the results of the sixth and fourth attempt
+constexpr int FK_LANE_STEP_SLOTS = 15;
 
 struct PrepArgs {
   int nslot, nk, nlay, attmode;
@@ -122,7 +122,7 @@ cudaError_t launch_poly(const PrepArgs& A, double* poly, cudaStream_t st);
 #define GEM_DECLARE_SOLVER(NS)                                                                          \
   namespace NS {                                                                                     \
   /* phase < 0: start radii; 0 toroidal, 1 spheroidal minors, 2 adjoint + spheroidal spectra;     */ \
-  /* sched: index into FK_SCHED_BLOCK / FK_SCHED_BIGCACHE                                           */ \
+  /* sched: index into FK_SCHED_BLOCK[build]                                                     */ \
   cudaError_t launch_fk_phase(int phase, int sched, const gem::FKStatic& P, const gem::FKLaunch& L, int grid,  \
                               cudaStream_t st);                                                      \
   int fk_phase_blocks_per_sm(int phase, int sched);                                                  \

@@ -28,13 +28,16 @@
 #include "fk_solver.cuh"
 
 namespace GEM_NS {
+namespace {   // one copy per translation unit
 
 enum : int { PH_TOR = 0, PH_SPH = 1, PH_ADJ = 2 };
 template <int PH> struct PhaseNV { static constexpr int NV = PH == PH_TOR ? 2 : (PH == PH_SPH ? 5 : 4); };
-// levels 0..5 of the per-lane Neville diagonal feed the last attempt; the
-// levels below PhaseDiag::L live in shared memory, the rest (read only by the
-// seventh attempt) in the lane's registers or stack
-template <int PH, int BLK> struct PhaseDiag { static constexpr int L = (PH == PH_SPH && BLK > 384) ? 5 : 6; };
+// Shared-memory levels per lane of a phase kernel.  Fast build: the results of
+// the attempts 1, 2, 3 and 5 (those of 4 and 6 stay in registers until the
+// seventh attempt, which takes them from the lane's scratch).  Plain build: the
+// Neville diagonal, levels 0..5; the levels from L on, read only by the seventh
+// attempt, live in the lane's registers or stack.
+template <int PH, int BLK> struct PhaseDiag { static constexpr int L = GEM_FAST ? 4 : ((PH == PH_SPH && BLK > 384) ? 5 : 6); };
 
 // lane states
 enum : int {
@@ -124,48 +127,157 @@ __device__ __constant__ const StepWork STEPWORK = make_stepwork();
 //  Lockstep Bulirsch-Stoer step of all lanes with `active` set
 //  (complexBulirschStep.f90:111-170,180-238,297-340)
 // ------------------------------------------------------------------------
-template <int SYS, int NVD, int DL, bool BIG>
+#if GEM_FAST
+// Fast form.  The attempts run in pairs of n and 2 n sub-steps, (2, 4), (6, 12)
+// and (8, 16), then 24: a pair shares its system matrices (32 evaluations
+// instead of 48 for the six attempts most steps take).  The convergence tests
+// keep the order of the attempts, so steps are accepted as the reference does.
+//
+// Bound: FP64 latency and instruction supply at 2-3 warps per scheduler.  On the
+// upper frequencies of the batched configuration (310,474 solves) the spheroidal
+// kernel went from 82.9 to 56.1 G warp instructions and from 233 to 144 ms, its
+// FP64 pipe from 41 to 45 % busy; the whole band from 560 to 363 ms (658,944
+// solves).  What gave it, each measured on the band: pairs, three cubics instead
+// of eleven complex ones for an isotropic model, the knot interval once per step
+// and reciprocals without a branch (560 -> 489 ms); one evaluation per loop trip
+// instead of two, which fits the instruction caches (489 -> 382 ms); results of
+// four attempts in shared memory instead of six Neville levels, which leaves the
+// L1 to the cubics (hit rate 73 -> 84 %), and FMA chains into z0 (382 -> 363 ms).
+// Slower: 4 to 6 attempts sharing matrices through masks (a branch per attempt
+// and grid point: 650-800 ms); the seventh attempt put off to the lane's next
+// step, beside the attempts of the others (spilled registers: 363 -> 390 ms).
+template <int SYS, int NVD, int DL, bool ISO>
 __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool active, double h, double x,
                                      const dz* y0, dz* yext, int& result, double2* D, int lane, const Slot& xs,
                                      Counters& cnt_out) {
   constexpr int NV = SysNV<SYS>::NV;
   // the lane state lives in local memory: work on a register copy of the
   // environment; the counters follow from the attempts made (added at the end)
-#if GEM_FAST
-  const EnvF e = make_envf(P, e_in, active);
+  const double h48 = h / 48.0;   // grid spacing of the step's sub-steps
+  const EnvF e = make_envf(P, e_in, active, x, x + 48.0 * h48);
+  int lane_att = 0, warp_att = 0;
+  bool need = active;
+  int res = 0;   // 0: failed; > 0: number of attempts of a successful step
+  const dz zom2 = cmul(dz{e.omre, e.omim}, dz{e.omre, e.omim});
+  // y0 (in the lane state) and A(x) y0 (the lane's scratch elements 0..4) are
+  // read once per pair: they stay in memory
+  if (need) {
+    dz z[NV], t[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) { z[v] = y0[v]; t[v] = dz{0.0, 0.0}; }
+    SysE<SYS> E;
+    sys_at<SYS, ISO>(e, zom2, x, 1.0, E);
+    sys_mul<SYS>(E, z, t);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) xs.put(v, t[v]);
+  }
+  static_assert(DL == 4, "levels: attempts 1, 2, 3, 5");
+  // extrapolation and convergence test after attempt j with result yj: the
+  // attempts in shared memory, and from j = 5 on the fourth (c), for j = 7 the sixth (from the scratch)
+  auto test = [&](int j, const dz* yj, const dz* c) {
+    dz yy[NV], dy[NV];
+    auto add = [&](int i, int v, dz yi) {
+      const dz d = yi - yj[v];
+      cfma(yy[v], EXTRAP.w[j][i - 1], d);
+      cfma(dy[v], EXTRAP.e[j][i - 1], d);
+    };
+#pragma unroll
+    for (int v = 0; v < NV; ++v) { yy[v] = yj[v]; dy[v] = dz{0.0, 0.0}; }
+    const int nl = j == 3 ? 2 : (j < 6 ? 3 : 4);
+#pragma unroll 1
+    for (int l = 0; l < nl; ++l) {
+      const int i = l < 3 ? l + 1 : 5;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double2 q = D[(l * NVD + v) * 32 + lane];
+        add(i, v, dz{q.x, q.y});
+      }
+    }
+    if (j >= 5) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) add(4, v, c[v]);
+    }
+    if (j == 7) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) add(6, v, xs.get(5 + v));
+    }
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s1 = fma(dy[v].re, dy[v].re, fma(dy[v].im, dy[v].im, s1));
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s2 = fma(yy[v].re, yy[v].re, fma(yy[v].im, yy[v].im, s2));
+    if (s1 < (P.eps * P.eps) * s2) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) yext[v] = yy[v];
+      res = j;
+      need = false;
+    }
+  };
+#pragma unroll 1
+  for (int g = 0; g < 4; ++g) {
+    const unsigned needm = __ballot_sync(0xffffffffu, need);
+    if (!needm) break;
+    lane_att += (g < 3 ? 2 : 1) * __popc(needm);
+    warp_att += g < 3 ? 2 : 1;
+    if (!need) continue;
+    dz f[NV], c[NV];
+    midpoint<SYS, ISO>(e, zom2, g == 0 ? 4 : (g == 1 ? 12 : (g == 2 ? 16 : 24)), g < 3, h48, x, y0, xs, f, c);
+    if (g < 2) {   // attempts 1 and 2, then 3 and 5
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        D[((g == 0 ? 0 : 2) * NVD + v) * 32 + lane] = make_double2(c[v].re, c[v].im);
+        D[((g == 0 ? 1 : 3) * NVD + v) * 32 + lane] = make_double2(f[v].re, f[v].im);
+      }
+      if (g == 0) continue;
+    }
+    const int j0 = g == 1 ? 3 : (g == 2 ? 4 : 7), j1 = g == 1 ? 3 : (g == 2 ? 6 : 7);
+    if (g == 3) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) c[v] = xs.get(10 + v);
+    }
+#pragma unroll 1
+    for (int j = j0; j <= j1 && need; ++j) {
+      dz yj[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        yj[v] = (j == 3 || j == 4) ? c[v] : f[v];
+        if (j == 5) { const double2 q = D[(3 * NVD + v) * 32 + lane]; yj[v] = dz{q.x, q.y}; }
+      }
+      test(j, yj, c);
+    }
+    if (g == 2 && need) {   // attempts 4 and 6 for the test of the seventh
+#pragma unroll
+      for (int v = 0; v < NV; ++v) { xs.put(10 + v, c[v]); xs.put(5 + v, f[v]); }
+    }
+    if (g == 3) need = false;
+  }
+  result = res;
+  const int jdone = res ? res : (active ? 7 : 0);
+  const int mv = STEPWORK.mv[jdone], sm = STEPWORK.sm[jdone];
+  cnt_out.lane_attempts += lane_att;
+  cnt_out.warp_attempts += warp_att;
+  cnt_out.attempts += jdone;
+  cnt_out.matvecs += mv;
+  cnt_out.sysmats += sm;
+  cnt_out.flops += (long long)sm * FLOP_SYSMAT[SYS] + (long long)mv * FLOP_MV[SYS] + STEPWORK.ext[NV][jdone];
+}
 #else
+template <int SYS, int NVD, int DL, bool ISO>
+__device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool active, double h, double x,
+                                     const dz* y0, dz* yext, int& result, double2* D, int lane, const Slot& xs,
+                                     Counters& cnt_out) {
+  constexpr int NV = SysNV<SYS>::NV;
+  // the lane state lives in local memory: work on a register copy of the
+  // environment; the counters follow from the attempts made (added at the end)
   const Env e = e_in;
-#endif
   int lane_att = 0, warp_att = 0, jdone = 0;
   bool need = active;
   int res = 0;   // 0: failed; > 0: number of attempts of a successful step
-#if GEM_FAST
-  // What every attempt shares: y0 (read from the lane state), A(x) y0 and the
-  // matrices at x + h/2 and x + h.  y0 and A(x) y0 are read once per attempt,
-  // so they stay in memory (A(x) y0 in the lane's scratch elements 0..4)
-  // instead of holding 20 registers each through the sub-step loop.
-  constexpr bool CACHE = SysCache<SYS, BIG>::value;
-  SysM<SYS> Mh, Me;
-  const double h48 = h / 48.0;   // grid spacing of the step's sub-steps
-  if (need) {
-    dz ys[NV], t0[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) ys[v] = y0[v];
-    apply_sys<SYS>(P, e, x, ys, t0);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) xs.put(v, t0[v]);
-    if constexpr (CACHE) {
-      sys_eval<SYS>(P, e, x + 24.0 * h48, Mh);
-      sys_eval<SYS>(P, e, x + 48.0 * h48, Me);
-    }
-  }
-#else
   (void)xs;
   dz ys[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) ys[v] = y0[v];
-#endif
-  dz dlast[NV];   // diagonal level DL when DL < 6 (fast build: scratch elements 5..9)
+  dz dlast[NV];   // diagonal level DL when DL < 6
   for (int j = 1; j <= 7; ++j) {
     unsigned needm = __ballot_sync(0xffffffffu, need);
     if (!needm) break;
@@ -173,51 +285,28 @@ __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool ac
     warp_att += 1;
     if (!need) continue;
     dz Y[NV];
-#if GEM_FAST
-    midpoint<SYS, CACHE>(P, e, j, h48, x, y0, xs, Mh, Me, Y);
-#else
     midpoint<SYS>(P, e, j, h, x, ys, Y);
-#endif
     jdone = j;
     // new diagonal of the Neville tableau for point p = j-1 (0-based)
     const int p = j - 1;
     dz yy[NV], dy[NV], c[NV], pend[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) { yy[v] = Y[v]; c[v] = Y[v]; pend[v] = Y[v]; dy[v] = dz{0.0, 0.0}; }
-#if GEM_FAST
-    for (int m = 1; m <= p; ++m) {
-      const double na = NEV.a[p][m], nb = NEV.b[p][m];
-#else
     const double xp = h / (double)SEQDIV[p];
     for (int m = 1; m <= p; ++m) {
       const double xi = h / (double)SEQDIV[p - m];
       const double hh = xi - xp;
-#endif
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const bool shared_level = DL == 6 || m - 1 < DL;
         double2* slot = D + ((m - 1) * NVD + v) * 32 + lane;
-#if GEM_FAST
-        dz pv = shared_level ? dz{0.0, 0.0} : xs.get(5 + v);
-#else
         dz pv = dlast[v];
-#endif
         if (shared_level) { double2 q = *slot; pv = dz{q.x, q.y}; }
-#if GEM_FAST
-        const dz u = c[v] - pv;
-        c[v] = na * u;
-        dz nd = nb * u;
-#else
         dz u = (c[v] - pv) / hh;
         c[v] = xi * u;
         dz nd = xp * u;
-#endif
         if (shared_level) *slot = make_double2(pend[v].re, pend[v].im);   // level m-1 of the new diagonal
-#if GEM_FAST
-        else xs.put(5 + v, pend[v]);
-#else
         else dlast[v] = pend[v];
-#endif
         pend[v] = nd;
         yy[v] = yy[v] + nd;
         dy[v] = nd;
@@ -227,30 +316,17 @@ __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool ac
 #pragma unroll
       for (int v = 0; v < NV; ++v) D[(p * NVD + v) * 32 + lane] = make_double2(pend[v].re, pend[v].im);
     } else if (p < 6) {
-#if GEM_FAST
-#pragma unroll
-      for (int v = 0; v < NV; ++v) xs.put(5 + v, pend[v]);
-#else
 #pragma unroll
       for (int v = 0; v < NV; ++v) dlast[v] = pend[v];
-#endif
     }
     if (j >= 3) {
       double s1 = 0.0, s2 = 0.0;
-#if GEM_FAST
-#pragma unroll
-      for (int v = 0; v < NV; ++v) s1 += dy[v].re * dy[v].re + dy[v].im * dy[v].im;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) s2 += yy[v].re * yy[v].re + yy[v].im * yy[v].im;
-      const bool conv = s1 < (P.eps * P.eps) * s2;
-#else
 #pragma unroll
       for (int v = 0; v < NV; ++v) { double a = zabs(dy[v]); s1 += a * a; }
 #pragma unroll
       for (int v = 0; v < NV; ++v) { double a = zabs(yy[v]); s2 += a * a; }
       double errmax = sqrt(s1 / s2);
       const bool conv = errmax / P.eps < 1.0;
-#endif
       if (conv) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) yext[v] = yy[v];
@@ -269,6 +345,18 @@ __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool ac
   cnt_out.matvecs += mv;
   cnt_out.sysmats += sm;
   cnt_out.flops += (long long)sm * FLOP_SYSMAT[SYS] + (long long)mv * FLOP_MV[SYS] + STEPWORK.ext[NV][jdone];
+}
+#endif
+
+// the step of a system: the isotropic form when the whole model is isotropic (fast build)
+template <int SYS, int NVD, int DL>
+__device__ __forceinline__ void bs_step_of(const FKStatic& P, const Env& e, bool active, double h, double x, const dz* y0,
+                                           dz* yext, int& result, double2* D, int lane, const Slot& xs, Counters& cnt) {
+#if GEM_FAST
+  if (P.iso) bs_step<SYS, NVD, DL, true>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt);
+  else
+#endif
+    bs_step<SYS, NVD, DL, false>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt);
 }
 
 // ------------------------------------------------------------------------
@@ -1021,7 +1109,7 @@ __global__ void __launch_bounds__(128) fk_setup_kernel(const __grid_constant__ F
 // ------------------------------------------------------------------------
 //  Lockstep phase kernel
 // ------------------------------------------------------------------------
-template <int PH, int BLK, bool BIG>
+template <int PH, int BLK>
 __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant__ FKStatic P, FKLaunch LL) {
   constexpr int NVD = PhaseNV<PH>::NV;
   extern __shared__ double2 smem_diag[];
@@ -1036,6 +1124,15 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   }
   if (threadIdx.x == 0) { blk_q = 0ull; blk_lock = 0; }
   __syncthreads();
+#if GEM_FAST
+  for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.kb[i] = tab.rk[i];
+  __syncthreads();
+  if (P.equidis == 1) {
+    for (int nl = 2 + (int)threadIdx.x; nl <= P.nlay; nl += blockDim.x)
+      for (int j1 = tab.iktop[nl - 1] + 1, i = j1; i <= tab.iktop[nl]; ++i) tab.kb[i] = tab.rk[j1] + (i - j1) * tab.drk[nl];
+    __syncthreads();
+  }
+#endif
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   constexpr int DL = PhaseDiag<PH, BLK>::L;
@@ -1140,25 +1237,25 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
     dz yext[5];
     int result = 0;
     if (PH == PH_TOR) {
-      bs_step<SYS_TOROIDAL, NVD, DL, BIG>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
+      bs_step_of<SYS_TOROIDAL, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
     } else if (PH == PH_ADJ) {
-      bs_step<SYS_SOLIDT, NVD, DL, BIG>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
+      bs_step_of<SYS_SOLIDT, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
     } else {
       unsigned sysmask = __reduce_or_sync(FULL, integ ? (1u << L.sys) : 0u);
       mixed_trips += __popc(sysmask) > 1;
       if (sysmask & (1u << SYS_MINORS))
-        bs_step<SYS_MINORS, NVD, DL, BIG>(P, L.e, integ && L.sys == SYS_MINORS, L.h, L.x, L.y, yext, result, D, lane, xs,
+        bs_step_of<SYS_MINORS, NVD, DL>(P, L.e, integ && L.sys == SYS_MINORS, L.h, L.x, L.y, yext, result, D, lane, xs,
                                           cnt);
       const unsigned long long c2 = clock64();
       if (sysmask & (1u << SYS_FLUID)) {
         int r = 0;
-        bs_step<SYS_FLUID, NVD, DL, BIG>(P, L.e, integ && L.sys == SYS_FLUID, L.h, L.x, L.y, yext, r, D, lane, xs,
+        bs_step_of<SYS_FLUID, NVD, DL>(P, L.e, integ && L.sys == SYS_FLUID, L.h, L.x, L.y, yext, r, D, lane, xs,
                                           cnt);
         if (integ && L.sys == SYS_FLUID) result = r;
       }
       if (sysmask & (1u << SYS_RADIAL)) {
         int r = 0;
-        bs_step<SYS_RADIAL, NVD, DL, BIG>(P, L.e, integ && L.sys == SYS_RADIAL, L.h, L.x, L.y, yext, r, D, lane, xs,
+        bs_step_of<SYS_RADIAL, NVD, DL>(P, L.e, integ && L.sys == SYS_RADIAL, L.h, L.x, L.y, yext, r, D, lane, xs,
                                           cnt);
         if (integ && L.sys == SYS_RADIAL) result = r;
       }
@@ -1231,4 +1328,5 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   }
 }
 
+}  // namespace
 }  // namespace GEM_NS

@@ -4,7 +4,8 @@
 // function) in the same operation order; the control structure is the
 // GPU's own:
 //   * system matrices are evaluated at each modified-midpoint sub-step instead
-//     of being cached on the 1/48 grid (same values, no per-thread cache);
+//     of being cached on the 1/48 grid (same values, no per-thread cache); the
+//     fast build shares them between the two attempts of a pair;
 //   * matrix-vector products skip the structural zeros of each system (adding
 //     a zero product leaves a sum unchanged);
 //   * results at nodes go to a per-thread scratch slot laid out
@@ -25,6 +26,7 @@
 #endif
 
 namespace GEM_NS {
+namespace {   // one copy per translation unit
 using namespace gem;
 
 // Bulirsch-Stoer subdivision scheme (parametersBulirschStep.f90:28-48)
@@ -63,6 +65,21 @@ __device__ __forceinline__ void layer_index(const FKStatic& P, double r, int& nl
 //  Spline evaluation (splineEarthmodelCoefficients.f90:118-162).
 //  MASK selects the elastic constants (bit c -> constant c of A,C,F,L,N,K,M).
 // ------------------------------------------------------------------------
+#if GEM_FAST
+// values at t of the cubics of one knot interval: density and the constants of MASK
+template <unsigned MASK>
+__device__ __forceinline__ void horner_spline(const double* __restrict__ q, double t, double& ro, dz* el) {
+  auto horner = [&](int v) {
+    double2 c32 = __ldg(reinterpret_cast<const double2*>(q + 4 * v));
+    double2 c10 = __ldg(reinterpret_cast<const double2*>(q + 4 * v + 2));
+    return fma(fma(fma(c32.x, t, c32.y), t, c10.x), t, c10.y);
+  };
+  ro = horner(0);
+#pragma unroll
+  for (int c = 0; c < 7; ++c)
+    if (MASK & (1u << c)) el[c] = dz{horner(poly_value(c)), horner(poly_value(c) + 1)};
+}
+#endif
 template <unsigned MASK>
 __device__ __forceinline__ void eval_spline(const FKStatic& P, const Env& e, double r, int nl, double& ro,
                                             dz* el) {
@@ -94,16 +111,7 @@ __device__ __forceinline__ void eval_spline(const FKStatic& P, const Env& e, dou
       j = j < 1 ? 1 : (j > P.nk - 1 ? P.nk - 1 : j);
       t = r - T->rk[j];
     }
-    const double* __restrict__ q = e.poly + (long long)j * POLY_STRIDE;
-    auto horner = [&](int v) {
-      double2 c32 = __ldg(reinterpret_cast<const double2*>(q + 4 * v));
-      double2 c10 = __ldg(reinterpret_cast<const double2*>(q + 4 * v + 2));
-      return fma(fma(fma(c32.x, t, c32.y), t, c10.x), t, c10.y);
-    };
-    ro = horner(0);
-#pragma unroll
-    for (int c = 0; c < 7; ++c)
-      if (MASK & (1u << c)) el[c] = dz{horner(1 + 2 * c), horner(2 + 2 * c)};
+    horner_spline<MASK>(e.poly + (long long)j * POLY_STRIDE, t, ro, el);
     return;
   }
 #endif
@@ -155,58 +163,60 @@ __device__ __forceinline__ void eval_spline(const FKStatic& P, const Env& e, dou
 }
 
 #if GEM_FAST
-// The environment of one Bulirsch-Stoer step (fast build): the knot range of
-// the step's layer is looked up once per step instead of at every sub-step.
-// The interval and t = r - rk(j) are the ones eval_spline finds.
+// The environment of one Bulirsch-Stoer step (fast build): the knot intervals
+// jlo..jhi of the step's two ends are looked up once per step.  A step is a
+// fraction of a wavelength and mostly stays in one interval or crosses one
+// knot, so a sub-step finds its interval by one comparison with the knot above
+// jlo; a search runs only while a lane of the warp steps over several knots
+// (wide).  The interval is the last one of jlo..jhi whose lower bound kb is not
+// above r (kb: the knots, or with equidistant knots their regular grid, which
+// gives the interval int((r - rk(j1)) / drk) of eval_spline).
 struct EnvF : Env {
-  int sj1, sjhi;       // first and last knot interval of the layer
-  int sflat;           // layer 1: the homogeneous sphere, evaluated at its knot (t = 0)
-  int sequi;           // equidistant knots: direct index; else the search of eval_spline
-  double srk1, srdrk;  // rk(j1) and 1/drk of the layer
+  int jlo, jhi;
+  bool wide;               // a lane of the warp spans more than two intervals
+  double kb1, rk0, rk1;    // kb(jlo+1) (infinite when jlo = jhi), rk(jlo), rk(jlo+1)
 };
+// last interval j of j1..j2 with kb(j) <= r (j1 when there is none)
+__device__ __forceinline__ int knot_interval(const double* __restrict__ kb, int j1, int j2, double r) {
+  int lo = j1, hi = j2;
+  while (lo < hi) {
+    const int m = (lo + hi + 1) >> 1;
+    if (kb[m] <= r) lo = m; else hi = m - 1;
+  }
+  return lo;
+}
 // Lanes without a step (active false) may hold no layer yet (a lane that never
 // took an item): they read the tables of layer 1 and evaluate nothing.
-__device__ __forceinline__ EnvF make_envf(const FKStatic& P, const Env& e, bool active) {
+__device__ __forceinline__ EnvF make_envf(const FKStatic& P, const Env& e, bool active, double xa, double xb) {
   EnvF f;
   static_cast<Env&>(f) = e;
   const Tab* __restrict__ T = e.tab;
   const int nl = (active && e.nl >= 1 && e.nl <= P.nlay) ? e.nl : 1;
-  f.sflat = nl == 1;
-  f.sequi = P.equidis == 1;
-  if (nl == 1) {
-    f.sj1 = f.sjhi = T->iktop[1];
-    f.srk1 = 0.0; f.srdrk = 0.0;
+  if (nl == 1) {   // the homogeneous sphere: the constant cubic of its knot
+    f.jlo = f.jhi = T->iktop[1];
   } else {
-    const int j1 = T->iktop[nl - 1] + 1, j2 = T->iktop[nl];
-    f.sj1 = j1; f.sjhi = j2 - 1;
-    f.srk1 = T->rk[j1]; f.srdrk = T->rdrk[nl];
+    const int j1 = min(max(T->iktop[nl - 1] + 1, 1), P.nk - 1), j2 = min(T->iktop[nl] - 1, P.nk - 1);
+    f.jlo = knot_interval(T->kb, j1, j2, fmin(xa, xb));
+    f.jhi = knot_interval(T->kb, f.jlo, j2, fmax(xa, xb));
   }
+  f.rk0 = T->rk[f.jlo];
+  f.rk1 = T->rk[f.jlo + 1];
+  f.kb1 = f.jhi > f.jlo ? T->kb[f.jlo + 1] : __longlong_as_double(0x7ff0000000000000LL);
+  f.wide = __any_sync(0xffffffffu, active && f.jhi > f.jlo + 1);
   return f;
 }
-template <unsigned MASK>
-__device__ __forceinline__ void eval_spline(const FKStatic& P, const EnvF& e, double r, double& ro, dz* el) {
-  if (!e.sequi) { eval_spline<MASK>(P, static_cast<const Env&>(e), r, e.nl, ro, el); return; }
-  const Tab* __restrict__ T = e.tab;
-  int j = e.sj1;
-  double t = 0.0;
-  if (!e.sflat) {
-    if (e.sjhi > e.sj1) {
-      j = (int)((r - e.srk1) * e.srdrk) + e.sj1;
-      j = j < e.sj1 ? e.sj1 : (j > e.sjhi ? e.sjhi : j);
-    }
-    j = j < 1 ? 1 : (j > P.nk - 1 ? P.nk - 1 : j);
-    t = r - T->rk[j];
+// cubics and argument of the spline at r
+__device__ __forceinline__ const double* spline_at(const EnvF& e, double r, double& t) {
+  const bool up = r >= e.kb1;
+  int j = up ? e.jlo + 1 : e.jlo;
+  double rk = up ? e.rk1 : e.rk0;
+  if (e.wide) {
+    const Tab* __restrict__ T = e.tab;
+    while (j < e.jhi && r >= T->kb[j + 1]) ++j;
+    rk = T->rk[j];
   }
-  const double* __restrict__ q = e.poly + (long long)j * POLY_STRIDE;
-  auto horner = [&](int v) {
-    double2 c32 = __ldg(reinterpret_cast<const double2*>(q + 4 * v));
-    double2 c10 = __ldg(reinterpret_cast<const double2*>(q + 4 * v + 2));
-    return fma(fma(fma(c32.x, t, c32.y), t, c10.x), t, c10.y);
-  };
-  ro = horner(0);
-#pragma unroll
-  for (int c = 0; c < 7; ++c)
-    if (MASK & (1u << c)) el[c] = dz{horner(1 + 2 * c), horner(2 + 2 * c)};
+  t = r - rk;
+  return e.poly + j * POLY_STRIDE;
 }
 #endif
 
@@ -221,138 +231,171 @@ template <> struct SysNV<SYS_RADIAL> { static constexpr int NV = 2; };
 template <> struct SysNV<SYS_TOROIDAL> { static constexpr int NV = 2; };
 template <> struct SysNV<SYS_SOLIDT> { static constexpr int NV = 4; };
 
-// 1/z: Smith's division on the parity path, one reciprocal on the fast path
-__device__ __forceinline__ dz zinv(dz z) {
-#if GEM_FAST
-  return zinv_fast(z);
-#else
-  return 1.0 / z;
-#endif
-}
+// 1/x and 1/z: divisions (Smith's for z) on the parity path.  The fast path
+// takes one reciprocal without a branch: the PTX approximation (20 bits, rel.
+// error d) and one third-order Newton (Householder) update r (1 + d + d^2),
+// whose error d^3 is below the rounding.  A correctly rounded reciprocal has a
+// slow path behind a branch, which keeps the compiler from overlapping the
+// evaluations of a step.
 __device__ __forceinline__ double rinv(double x) {
 #if GEM_FAST
-  return __drcp_rn(x);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double d = fma(-x, r, 1.0);
+  return fma(r, fma(d, d, d), r);
 #else
   return 1.0 / x;
 #endif
 }
+__device__ __forceinline__ dz zinv(dz z) {
+#if GEM_FAST
+  const double r = rinv(z.re * z.re + z.im * z.im);
+  return {z.re * r, -z.im * r};
+#else
+  return 1.0 / z;
+#endif
+}
 
 #if GEM_FAST
-// Fast build: the system matrix at x in a compact form -- the quantities
-// that depend on x, from which the entries follow with a few products -- so
-// that a Bulirsch-Stoer step evaluates the positions all its attempts share
-// (x0, x0 + h/2, x0 + h) once.  Entries as in the plain build below.
-template <int SYS> struct SysM;
-template <> struct SysM<SYS_MINORS> { dz a, b, c, m23, m24; double rr, ro; };   // a = z2/r, b = 4 z1/r^2, c = N/r^2
-template <> struct SysM<SYS_FLUID> { dz m12; double m11, ro; };
-template <> struct SysM<SYS_RADIAL> { dz m11, m12, m21, m22; };
-template <> struct SysM<SYS_TOROIDAL> { dz m12, m21; double rr; };
-template <> struct SysM<SYS_SOLIDT> { dz z2, zrpc, w, c, a43; double rr, ro; };  // w = z1/r^2, c = N/r^2
+// acc + a b, four FMAs for a complex factor
+__device__ __forceinline__ void cfma(dz& acc, dz a, dz b) {
+  acc.re = fma(a.re, b.re, fma(-a.im, b.im, acc.re));
+  acc.im = fma(a.re, b.im, fma(a.im, b.re, acc.im));
+}
+__device__ __forceinline__ void cfma(dz& acc, double a, dz b) {
+  acc.re = fma(a, b.re, acc.re);
+  acc.im = fma(a, b.im, acc.im);
+}
+__device__ __forceinline__ dz cmul(dz a, dz b) {
+  return {fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re)};
+}
 
-template <int SYS>
-__device__ __forceinline__ void sys_eval(const FKStatic& P, const EnvF& e, double x, SysM<SYS>& M) {
+// Entries of w A(x) of the fast build, w the sub-step's weight: z0 + w A z1 is
+// then a chain of FMAs into z0.  w enters in the few factors every entry has one of.
+template <int SYS> struct SysE;
+template <> struct SysE<SYS_MINORS> { dz a, m12, m14, m23, m24, m32, m42, z4; double m11, m13, m22, m33, m55; };
+template <> struct SysE<SYS_FLUID> { dz m12, m21; double m11; };
+template <> struct SysE<SYS_RADIAL> { dz m11, m12, m21, m22; };
+template <> struct SysE<SYS_TOROIDAL> { dz m12, m21; double rr; };
+template <> struct SysE<SYS_SOLIDT> { dz a11, a12, a14, z2, zrpc, a31, a32, a34, a43; double rr, a22, a42; };
+
+// w A(x) from the cubics q at t.  ISO (every knot of the model isotropic:
+// A = C, N = L, F = C - 2 L): with m = L/C, A - F^2/C - N = L (3 - 4 m) and
+// F/C = 1 - 2 m, so only the density, C and L are evaluated (5 cubics instead
+// of 11).  zom2 = (omega - i sigma)^2.
+template <int SYS, bool ISO>
+__device__ __forceinline__ void sys_eval(const EnvF& e, dz zom2, const double* __restrict__ q, double t, double x,
+                                         double w, SysE<SYS>& E) {
   double ro;
   dz el[7];
-  const dz zom{e.omre, e.omim};
   const double dll1 = e.dll1;
-  if constexpr (SYS == SYS_MINORS) {          // minorsOdeSystem.f90:77-126
-    eval_spline<0x1Fu>(P, e, x, ro, el);
-    const double rr = rinv(x), rr2 = rr * rr;
-    const dz zrpc = zinv(el[1]);
-    const dz z1 = el[0] - (el[2] * el[2]) * zrpc - el[4];
-    M.a = ((2.0 * el[2]) * zrpc) * rr;
-    M.b = (4.0 * z1) * rr2;
-    M.c = el[4] * rr2;
-    M.m23 = zinv(el[3]);
-    M.m24 = zrpc;
-    M.rr = rr;
-    M.ro = ro;
+  if constexpr (SYS == SYS_MINORS || SYS == SYS_SOLIDT) {   // minorsOdeSystem.f90:77-126, solidtOdeSystem.f90:77-114
+    horner_spline<ISO ? 0x0Au : 0x1Fu>(q, t, ro, el);
+    const double rr = rinv(x), rs = w * rr, r2s = rs * rr;
+    const dz zrpc = zinv(el[1]), zom = (w * ro) * zom2;
+    const double rl = w * rinv(fma(el[3].re, el[3].re, el[3].im * el[3].im));
+    const dz m23{el[3].re * rl, -el[3].im * rl};
+    dz z1, fc, n;   // A - F^2/C - N, F/C, N
+    if constexpr (ISO) {
+      const dz m = cmul(el[3], zrpc);
+      n = el[3];
+      z1 = cmul(n, dz{fma(-4.0, m.re, 3.0), -4.0 * m.im});
+      fc = dz{fma(-2.0, m.re, 1.0), -2.0 * m.im};
+    } else {
+      n = el[4];
+      fc = cmul(el[2], zrpc);
+      z1 = el[0] - n;
+      cfma(z1, -el[2], fc);
+    }
+    const dz z = r2s * z1, c = r2s * n;
+    if constexpr (SYS == SYS_MINORS) {
+      E.a = (2.0 * rs) * fc;
+      E.m11 = -2.0 * rs;
+      E.m13 = dll1 * rs;
+      E.m12 = (-2.0 * dll1) * z;
+      E.m14 = (-0.5 * dll1) * E.a;
+      E.m22 = rs - E.a.re;               // the imaginary parts of m22, m33, m55 are -a, -a, +a
+      E.m33 = fma(-3.0, rs, -E.a.re);
+      E.m55 = fma(-5.0, rs, E.a.re);
+      E.m23 = m23;
+      E.m24 = w * zrpc;
+      E.z4 = 4.0 * z;
+      E.m42 = E.z4 - zom;
+      E.m32 = dz{fma(dll1, z.re, fma(dll1 - 2.0, c.re, -zom.re)), fma(dll1, z.im, fma(dll1 - 2.0, c.im, -zom.im))};
+    } else {
+      E.rr = rs;
+      E.z2 = rs * fc;
+      E.zrpc = (-w) * zrpc;
+      E.a43 = -m23;
+      E.a11 = 2.0 * E.z2;
+      E.a12 = dz{fma(-4.0, z.re, zom.re), fma(-4.0, z.im, zom.im)};
+      E.a14 = 2.0 * z;
+      E.a22 = fma(2.0, rs, -E.a11.re);   // its imaginary part is -a11
+      E.a31 = (-dll1) * E.z2;
+      E.a32 = (2.0 * dll1) * z;
+      E.a34 = dz{fma(-dll1, z.re, fma(2.0 - dll1, c.re, zom.re)), fma(-dll1, z.im, fma(2.0 - dll1, c.im, zom.im))};
+      E.a42 = (-dll1) * rs;
+    }
   } else if constexpr (SYS == SYS_FLUID) {   // fluidOdeSystem.f90:78-95
-    eval_spline<0x02u>(P, e, x, ro, el);
-    const dz zomro = zom * zom * ro;
-    M.m11 = -2.0 * rinv(x);
-    M.m12 = zinv(el[1]) - dll1 * zinv((zomro * x) * x);
-    M.ro = ro;
+    horner_spline<0x02u>(q, t, ro, el);
+    const dz zomro = ro * zom2;
+    const dz k = zinv(el[1]), g = zinv((zomro * x) * x);
+    E.m11 = (-2.0 * w) * rinv(x);
+    E.m12 = w * dz{fma(-dll1, g.re, k.re), fma(-dll1, g.im, k.im)};
+    E.m21 = (-w) * zomro;
   } else if constexpr (SYS == SYS_RADIAL) {  // radialOdeSystem.f90:78-99
-    eval_spline<0x17u>(P, e, x, ro, el);
-    const dz zomro = zom * zom * ro;
+    horner_spline<ISO ? 0x0Au : 0x17u>(q, t, ro, el);
+    if constexpr (ISO) { el[0] = el[1]; el[2] = el[1] - 2.0 * el[3]; el[4] = el[3]; }
+    const dz zomro = ro * zom2;
     const double rr = rinv(x), rr2 = rr * rr;
     const dz rc = zinv(el[1]);
-    M.m11 = ((-2.0 * el[2]) * rr) * rc;
-    M.m12 = rc;
-    M.m21 = (-zomro) + (4.0 * rr2) * ((el[0] - (el[2] * el[2]) * rc) - el[4]);
-    M.m22 = (2.0 * rr) * (el[2] * rc - 1.0);
-  } else if constexpr (SYS == SYS_TOROIDAL) {  // toroidalOdeSystem.f90:81-102
-    eval_spline<0x18u>(P, e, x, ro, el);
-    const dz zomro = zom * zom * ro;
-    const double rr = rinv(x), rr2 = rr * rr;
-    M.m12 = zinv(el[3]);
-    M.m21 = (-zomro) - (el[4] * rr2) * (2.0 - dll1);
-    M.rr = rr;
-  } else {                                    // solidtOdeSystem.f90:77-114
-    eval_spline<0x1Fu>(P, e, x, ro, el);
-    const double rr = rinv(x), rr2 = rr * rr;
-    const dz zrpc = zinv(el[1]);
-    M.z2 = (el[2] * rr) * zrpc;
-    M.zrpc = zrpc;
-    M.w = (el[0] - (el[2] * el[2]) * zrpc - el[4]) * rr2;
-    M.c = el[4] * rr2;
-    M.a43 = -zinv(el[3]);
-    M.rr = rr;
-    M.ro = ro;
+    E.m11 = ((-2.0 * w * rr) * el[2]) * rc;
+    E.m12 = w * rc;
+    E.m21 = w * ((-zomro) + (4.0 * rr2) * ((el[0] - (el[2] * el[2]) * rc) - el[4]));
+    E.m22 = (2.0 * w * rr) * (el[2] * rc - 1.0);
+  } else {                                   // toroidalOdeSystem.f90:81-102
+    horner_spline<ISO ? 0x08u : 0x18u>(q, t, ro, el);
+    const dz zom = (w * ro) * zom2;
+    const double rr = rinv(x), rs = w * rr, r2s = (dll1 - 2.0) * (rs * rr);
+    const dz n = el[ISO ? 3 : 4];
+    E.m12 = w * zinv(el[3]);
+    E.m21 = dz{fma(n.re, r2s, -zom.re), fma(n.im, r2s, -zom.im)};
+    E.rr = rs;
   }
 }
 
+// acc += E z
 template <int SYS>
-__device__ __forceinline__ void sys_apply(const SysM<SYS>& M, const Env& e, const dz* z, dz* y) {
-  const dz zom{e.omre, e.omim};
-  const double dll1 = e.dll1;
+__device__ __forceinline__ void sys_mul(const SysE<SYS>& E, const dz* z, dz* acc) {
   if constexpr (SYS == SYS_MINORS) {
-    const dz zomro = zom * zom * M.ro;
-    const double rr = M.rr, m11 = -2.0 * rr, m13 = dll1 * rr;
-    const dz m12 = (-0.5 * dll1) * M.b;
-    const dz m14 = (-0.5 * dll1) * M.a;
-    const dz m22 = rr - M.a;
-    const dz m32 = (-zomro) + (0.25 * dll1) * M.b + (dll1 - 2.0) * M.c;
-    const dz m33 = (-3.0 * rr) - M.a;
-    const dz m42 = (-zomro) + M.b;
-    const dz m55 = M.a - 5.0 * rr;
-    y[0] = m11 * z[0] + m12 * z[1] + m13 * z[2] + m14 * z[3];
-    y[1] = m22 * z[1] + M.m23 * z[2] + M.m24 * z[3];
-    y[2] = (-M.a) * z[0] + m32 * z[1] + m33 * z[2] + M.m24 * z[4];
-    y[3] = (-m11) * z[0] + m42 * z[1] + (-m22) * z[3] + M.m23 * z[4];
-    y[4] = M.b * z[0] + m42 * z[2] + m32 * z[3] + m55 * z[4];
+    const dz m22{E.m22, -E.a.im}, m33{E.m33, -E.a.im}, m55{E.m55, E.a.im};
+    cfma(acc[0], E.m11, z[0]); cfma(acc[1], m22, z[1]); cfma(acc[2], -E.a, z[0]); cfma(acc[3], -E.m11, z[0]); cfma(acc[4], E.z4, z[0]);
+    cfma(acc[0], E.m12, z[1]); cfma(acc[1], E.m23, z[2]); cfma(acc[2], E.m32, z[1]); cfma(acc[3], E.m42, z[1]); cfma(acc[4], E.m42, z[2]);
+    cfma(acc[0], E.m13, z[2]); cfma(acc[1], E.m24, z[3]); cfma(acc[2], m33, z[2]); cfma(acc[3], -m22, z[3]); cfma(acc[4], E.m32, z[3]);
+    cfma(acc[0], E.m14, z[3]); cfma(acc[2], E.m24, z[4]); cfma(acc[3], E.m23, z[4]); cfma(acc[4], m55, z[4]);
   } else if constexpr (SYS == SYS_FLUID) {
-    const dz zomro = zom * zom * M.ro;
-    y[0] = M.m11 * z[0] + M.m12 * z[1];
-    y[1] = (-zomro) * z[0];
+    cfma(acc[0], E.m11, z[0]); cfma(acc[1], E.m21, z[0]);
+    cfma(acc[0], E.m12, z[1]);
   } else if constexpr (SYS == SYS_RADIAL) {
-    y[0] = M.m11 * z[0] + M.m12 * z[1];
-    y[1] = M.m21 * z[0] + M.m22 * z[1];
+    cfma(acc[0], E.m11, z[0]); cfma(acc[1], E.m21, z[0]);
+    cfma(acc[0], E.m12, z[1]); cfma(acc[1], E.m22, z[1]);
   } else if constexpr (SYS == SYS_TOROIDAL) {
-    y[0] = M.rr * z[0] + M.m12 * z[1];
-    y[1] = M.m21 * z[0] + (-3.0 * M.rr) * z[1];
+    cfma(acc[0], E.rr, z[0]); cfma(acc[1], E.m21, z[0]);
+    cfma(acc[0], E.m12, z[1]); cfma(acc[1], -3.0 * E.rr, z[1]);
   } else {
-    const dz zomro = zom * zom * M.ro;
-    const double rr = M.rr, rr2 = rr * rr;
-    const dz a11 = 2.0 * M.z2;
-    const dz a12 = zomro - 4.0 * M.w;
-    const dz a22 = (-a11) + 2.0 * rr;
-    const dz a32 = (2.0 * dll1) * M.w;
-    const dz a34 = zomro - (dll1 * M.w + (dll1 - 2.0) * M.c);
-    (void)rr2;
-    y[0] = a11 * z[0] + a12 * z[1] + rr * z[2] + (2.0 * M.w) * z[3];
-    y[1] = (-M.zrpc) * z[0] + a22 * z[1] + M.z2 * z[3];
-    y[2] = ((-dll1) * M.z2) * z[0] + a32 * z[1] + (-rr) * z[2] + a34 * z[3];
-    y[3] = ((-dll1) * rr) * z[1] + M.a43 * z[2] + (3.0 * rr) * z[3];
+    const dz a22{E.a22, -E.a11.im};
+    cfma(acc[0], E.a11, z[0]); cfma(acc[1], E.zrpc, z[0]); cfma(acc[2], E.a31, z[0]); cfma(acc[3], E.a42, z[1]);
+    cfma(acc[0], E.a12, z[1]); cfma(acc[1], a22, z[1]); cfma(acc[2], E.a32, z[1]); cfma(acc[3], E.a43, z[2]);
+    cfma(acc[0], E.rr, z[2]); cfma(acc[1], E.z2, z[3]); cfma(acc[2], -E.rr, z[2]); cfma(acc[3], 3.0 * E.rr, z[3]);
+    cfma(acc[0], E.a14, z[3]); cfma(acc[2], E.a34, z[3]);
   }
 }
 
-template <int SYS>
-__device__ __forceinline__ void apply_sys(const FKStatic& P, const EnvF& e, double x, const dz* z, dz* y) {
-  SysM<SYS> M;
-  sys_eval<SYS>(P, e, x, M);
-  sys_apply<SYS>(M, e, z, y);
+template <int SYS, bool ISO>
+__device__ __forceinline__ void sys_at(const EnvF& e, dz zom2, double x, double w, SysE<SYS>& E) {
+  double t;
+  const double* q = spline_at(e, x, t);
+  sys_eval<SYS, ISO>(e, zom2, q, t, x, w, E);
 }
 #else
 template <int SYS>
@@ -442,67 +485,78 @@ __device__ __forceinline__ void apply_sys(const FKStatic& P, const Env& e, doubl
 //  Bulirsch-Stoer full step (complexBulirschStep.f90:111-240,297-340)
 // ------------------------------------------------------------------------
 #if GEM_FAST
-// The 2-variable systems keep the matrices at x0 + h/2 and x0 + h across the
-// attempts of a step; the 5- and 4-variable systems do when BIG is set (a
-// schedule choice: at 384-512 threads per block the held matrices cost more in
-// spilled registers than evaluating them again, at 256 they do not).
-template <int SYS, bool BIG> struct SysCache {
-  static constexpr bool value = BIG || SYS == SYS_TOROIDAL || SYS == SYS_FLUID || SYS == SYS_RADIAL;
+// Extrapolation of the attempts 1..j to step size 0 by the polynomial through
+// (x_i = h / n_i, Y_i): its value is Y_j + sum_{i<j} w_i (Y_i - Y_j) with the
+// Lagrange weights w_i = prod_{k != i} n_i / (n_i - n_k), in which h cancels, and
+// the last correction of the Neville recursion (the polynomial through all
+// attempts minus the one without the first) is sum_{i<j} e_i (Y_i - Y_j),
+// e_i = w_i - w_i of the attempts 2..j.  |w_i| <= 39.
+struct ExtrapTab {
+  double w[8][7], e[8][7];
 };
-
-// Neville coefficients of the fast build.  With x_k = h / n_k, the update of
-// level m of diagonal p, u = (c - d) / (x_{p-m} - x_p), c' = x_{p-m} u,
-// d' = x_p u, is c' = a (c - d), d' = b (c - d) with a = n_p / (n_p - n_{p-m})
-// and b = n_{p-m} / (n_p - n_{p-m}): h cancels, so no division is left.
-struct NevTab {
-  double a[7][7], b[7][7];
-};
-constexpr NevTab make_nev() {
+constexpr ExtrapTab make_extrap() {
   const int n[7] = {2, 4, 6, 8, 12, 16, 24};
-  NevTab t{};
-  for (int p = 1; p < 7; ++p)
-    for (int m = 1; m <= p; ++m) {
-      t.a[p][m] = (double)n[p] / (double)(n[p] - n[p - m]);
-      t.b[p][m] = (double)n[p - m] / (double)(n[p] - n[p - m]);
+  ExtrapTab t{};
+  for (int j = 2; j <= 7; ++j)
+    for (int i = 0; i < j; ++i) {
+      double w = 1.0, w1 = 1.0;
+      for (int k = 0; k < j; ++k) {
+        if (k == i) continue;
+        w *= (double)n[i] / (double)(n[i] - n[k]);
+        if (k > 0) w1 *= (double)n[i] / (double)(n[i] - n[k]);
+      }
+      t.w[j][i] = w;
+      t.e[j][i] = i == 0 ? w : w - w1;
     }
   return t;
 }
-__device__ __constant__ const NevTab NEV = make_nev();
+__device__ __constant__ const ExtrapTab EXTRAP = make_extrap();
 
-// Modified midpoint of attempt jtry with t0 = A(xstart) y0 given (in memory), and with
-// CACHE the matrices at xstart + h/2 (Mh) and xstart + h (Me): the parts every
-// attempt of a step shares.  The grid point g (in 48ths of the step) sits at
-// xstart + g h48, h48 = h / 48 rounded once per step.
-template <int SYS, bool CACHE>
-__device__ __forceinline__ void midpoint(const FKStatic& P, const EnvF& e, int jtry, double h48, double xstart,
-                                         const dz* y0, const Slot& t0, const SysM<SYS>& Mh, const SysM<SYS>& Me,
-                                         dz* out) {
+// Modified midpoint of n sub-steps, and with pair the one of n/2 sub-steps
+// beside it: its grid is every second point of the finer one, so both share
+// the system matrices.  t0 = A(xstart) y0 is given (in memory); the grid point g
+// (in 48ths of the step) sits at xstart + g h48, h48 = h / 48 rounded once per step.
+// A sub-step z2 = z0 + 2 hf A z1 accumulates into z0; the coarse one has twice
+// the weight, which its vector takes (exact).  The last sub-step takes half the
+// weight: z_{n-1} + hf A z_n, whose mean with z_n is the result.
+// One evaluation per loop trip: the loop stays small enough for the instruction
+// caches (with two per trip, warps waited longer for instructions than for data).
+template <int SYS, bool ISO>
+__device__ __forceinline__ void midpoint(const EnvF& e, dz zom2, int n, bool pair, double h48, double xstart, const dz* y0,
+                                         const Slot& t0, dz* fine, dz* coarse) {
   constexpr int NV = SysNV<SYS>::NV;
-  const int nstep = SEQDIV[jtry - 1];
-  const int dix = 48 / nstep;
-  const double hdiv = (double)dix * h48;
-  dz z0[NV], z1[NV], t[NV];
+  const int dix = 48 / n;
+  const double dg = (double)dix, hf = dg * h48;
+  dz f0[NV], c0[NV];
 #pragma unroll
-  for (int v = 0; v < NV; ++v) { z0[v] = y0[v]; z1[v] = y0[v] + hdiv * t0.get(v); }
-  const double h2 = 2.0 * hdiv;
-  for (int m = 1; m <= nstep - 1; ++m) {
-    if (CACHE && m * dix == 24) {
-      sys_apply<SYS>(Mh, e, z1, t);
-    } else {
-      const double x = xstart + (double)(m * dix) * h48;
-      apply_sys<SYS>(P, e, x, z1, t);
-    }
+  for (int v = 0; v < NV; ++v) {
+    const dz y = y0[v], t = t0.get(v);
+    f0[v] = y; fine[v] = y + hf * t;
+    c0[v] = y; coarse[v] = y + (2.0 * hf) * t;
+  }
+  double g = 0.0;
+#pragma unroll 1
+  for (int m = 1; m <= n; ++m) {
+    g += dg;
+    SysE<SYS> E;
+    sys_at<SYS, ISO>(e, zom2, xstart + g * h48, m == n ? hf : 2.0 * hf, E);
+    sys_mul<SYS>(E, fine, f0);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      dz z2 = z0[v] + h2 * t[v];
-      z0[v] = z1[v];
-      z1[v] = z2;
+    for (int v = 0; v < NV; ++v) { const dz z = f0[v]; f0[v] = fine[v]; fine[v] = z; }
+    if (pair && !(m & 1)) {
+      dz u[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) u[v] = 2.0 * coarse[v];
+      sys_mul<SYS>(E, u, c0);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) { const dz z = c0[v]; c0[v] = coarse[v]; coarse[v] = z; }
     }
   }
-  if constexpr (CACHE) sys_apply<SYS>(Me, e, z1, t);
-  else apply_sys<SYS>(P, e, xstart + 48.0 * h48, z1, t);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) out[v] = 0.5 * ((z1[v] + z0[v]) + hdiv * t[v]);
+  for (int v = 0; v < NV; ++v) {
+    fine[v] = 0.5 * (f0[v] + fine[v]);
+    coarse[v] = 0.5 * (c0[v] + coarse[v]);
+  }
 }
 #else
 template <int SYS>
@@ -795,4 +849,5 @@ __device__ int toroidal_surface_iv(const FKStatic& P, const Env& e, dz* ys, doub
   return ST_OK;
 }
 
+}  // namespace
 }  // namespace GEM_NS

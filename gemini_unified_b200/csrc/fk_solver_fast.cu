@@ -3,4 +3,5 @@
 // (compiled with --fmad=true).
 #define GEM_NS gem_fast
 #define GEM_FAST 1
+#define GEM_PHASE 2
 #include "fk_solver_tu.cuh"

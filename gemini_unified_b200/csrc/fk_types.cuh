@@ -14,6 +14,7 @@ struct FKStatic {
   double rearth, ric, roc, rhs, ruc, eps, sigma, df, dwn;
   int kopt;   // attempt the step-size control aims at (opttry, parametersBulirschStep.f90:28-48: 6)
   int dsv;    // 1: DSV spectra with radial derivatives of a source at node jre (no reciprocity)
+  int iso;    // 1: every knot is isotropic (A = C, N = L, F = C - 2 L)
   int jsl, jsr;   // node range of the minors (spheroidalMinors.f90:72-585): jre..jre, or a set of source nodes
   double rb[MAXLAY + 1];
   double drk[MAXLAY + 1];
@@ -34,12 +35,17 @@ struct Counters {
 // memory (lanes index them divergently)
 struct Tab {
   double rk[MAXKNOT + 1];
+  double kb[MAXKNOT + 1];    // lower bound of the radii that take interval j (fast variant)
   double drk[MAXLAY + 1];
   double rdrk[MAXLAY + 1];   // 1/drk (fast variant)
   int iktop[MAXLAY + 1];
 };
 
 constexpr int POLY_STRIDE = 64;   // doubles per knot interval in the polynomial table
+// position in the polynomial table of the real part of constant c (A, C, F, L, N,
+// K, M; the imaginary part follows it; position 0 is the density): C and L first,
+// so that what an isotropic model needs (density, C, L) is one run of 160 bytes
+__host__ __device__ constexpr int poly_value(int c) { return c == 1 ? 1 : (c == 3 ? 3 : (c == 0 ? 5 : (c == 2 ? 7 : 1 + 2 * c))); }
 
 struct Env {
   const Tab* tab;                   // shared-memory copy of the knot tables

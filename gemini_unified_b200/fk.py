@@ -22,9 +22,9 @@ LIB_PATH = os.path.join(_HERE, "_lib", "libgemini_fk.so")
 
 GEM_BACKEND_GPU_FP64 = 1
 GEM_BACKEND_GPU_FAST = 2
-# solver schedules (include/gemini_fk.h): threads per block and whether the 4-
-# and 5-variable systems keep their half- and end-step matrices (fast backend)
-SCHEDULES = [(384, False), (512, False), (256, False), (384, True), (512, True), (256, True)]
+# solver schedules (include/gemini_fk.h): threads per block of the fast and of the
+# plain backend (which tries the first three only)
+SCHEDULES = [(256, 384), (384, 512), (512, 256), (320, 384), (448, 512), (192, 256)]
 NSCHED = len(SCHEDULES)
 # bookkeeping deferrals (lanes waiting, steps waited)
 DEFERRALS = [(1, 0), (8, 6), (16, 10), (32, 24), (32, 48), (32, 1000000)]

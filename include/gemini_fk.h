@@ -226,9 +226,8 @@ int gem_fk_graph_launch(gem_ctx* ctx, void* stream);
 /* Solver schedules and their autotuner (no counterpart in the reference; the
  * reference runs one solve at a time).  Each phase kernel (toroidal,
  * spheroidal, adjoint) runs one block per SM under one of GEM_FK_NSCHED
- * schedules: threads per block (384, 512, 256, 384, 512, 256) and, for
- * schedules 3..5, the 4- and 5-variable systems of the fast backend keep their
- * half- and end-step matrices across the attempts of a Bulirsch-Stoer step.
+ * schedules: 256, 384, 512, 320, 448 or 192 threads per block with the fast
+ * backend, 384, 512, 256, 384, 512 or 256 with the plain one.
  * Every schedule gives bit-identical spectra.  sched3[ph] is kept per context
  * and backend; the default is {1, 0, 1}. */
 #define GEM_FK_NSCHED 6

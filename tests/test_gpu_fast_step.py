@@ -1,0 +1,59 @@
+"""The fast build's Bulirsch-Stoer step over the forms of an earth model it
+distinguishes: isotropic (density, C and L evaluated) or not, knots on a regular
+grid or searched, and steps that stay in one or two knot intervals or cross
+several (fine knots at low frequency).  Reference: the FP64 form, which repeats
+the reference's arithmetic and evaluates all constants; the spectra must agree
+to 1e-8 of each spectrum's largest value, the FP64 spectral bar."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from gemini_unified_b200 import configs, model as M
+
+pytestmark = pytest.mark.gpu
+
+
+def _refined(m, n):
+    """The model with n - 1 knots added in every knot interval of its layers (linear in between)."""
+    cols = ("depth", "ro", "vpv", "vph", "vsv", "vsh", "eta", "qk", "qm")
+    new = {c: [] for c in cols}
+    top = []
+    bot = m.ikbot
+    for nl in range(m.nlay):
+        a, b = (m.iktop[0] - 1, m.iktop[0] - 1) if nl == 0 else (bot[nl] - 1, m.iktop[nl] - 1)
+        k = 1 if nl == 0 or (b - a) * n + 1 > 60 else n
+        x = np.arange((b - a) * k + 1) / k + a
+        for c in cols:
+            new[c].append(np.interp(x, np.arange(m.nk), getattr(m, c)))
+        top.append(sum(len(v) for v in new["ro"]))
+    new = {c: np.concatenate(v) for c, v in new.items()}
+    return dataclasses.replace(m, nk=len(new["ro"]), iktop=np.asarray(top, np.int32), **new)
+
+
+MODELS = {
+    "isotropic": lambda: configs.prem(),
+    "transversely_isotropic": lambda: configs.prem(isotropic=False),
+    "searched_knots": lambda: dataclasses.replace(configs.prem(), equidis=0),
+    "fine_knots": lambda: _refined(configs.prem(), 2),
+    "fine_searched_knots_ti": lambda: dataclasses.replace(_refined(configs.prem(isotropic=False), 2), equidis=0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(MODELS))
+@pytest.mark.parametrize("source,stress", [("MOMENT", False), ("FORCE", True)])
+def test_fast_step_matches_the_fp64_form(gpu, name, source, stress):
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, GEM_BACKEND_GPU_FP64, GeminiFK
+    w = configs.WORKLOADS["global_small"]
+    m = MODELS[name]()
+    ex = w.nodes(m)
+    jre = ex.node_index(w.rec_radius)
+    p = dataclasses.replace(w.params, source_type=source, stressflag=stress)
+    for jf in (2, 9, 52):       # the lowest frequencies take the longest steps
+        ref = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FP64).run(p, jre, jf, jf, f32=False)
+        got = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST).run(p, jre, jf, jf, f32=False)
+        np.testing.assert_array_equal(got[3], ref[3])
+        np.testing.assert_array_equal(np.isnan(got[2]), np.isnan(ref[2]))
+        scale = np.nanmax(np.abs(ref[2]), axis=2, keepdims=True)
+        err = np.abs(got[2] - ref[2]) / np.where(scale > 0, scale, 1.0)
+        assert np.nanmax(err) <= 1e-8
