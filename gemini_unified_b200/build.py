@@ -62,7 +62,7 @@ def source_hash() -> str:
         h.update(os.path.relpath(f, ROOT).encode())
         with open(f, "rb") as fh:
             h.update(hashlib.sha256(fh.read()).digest())
-    h.update(repr((ARCH, FLAGS, sorted(FMAD_TRUE))).encode())
+    h.update(repr((ARCH, [f.replace(ROOT, ".") for f in FLAGS], sorted(FMAD_TRUE))).encode())   # not where the tree lies
     h.update(_nvcc_version().encode())
     return h.hexdigest()
 
