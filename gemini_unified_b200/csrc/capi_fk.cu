@@ -51,6 +51,7 @@ struct gem_ctx {
   int* d_order = nullptr; size_t order_cap = 0;
   int32_t* d_status = nullptr; size_t status_cap = 0;
   double* d_rstart = nullptr; size_t rstart_cap = 0;
+  double2* d_start = nullptr; size_t start_cap = 0;
   double2* d_um = nullptr; size_t um_cap = 0;
   double2* d_dm = nullptr; size_t dm_cap = 0;
   double2* d_dets = nullptr; size_t dets_cap = 0;
@@ -248,7 +249,7 @@ void gem_ctx_destroy(gem_ctx* ctx) {
   cudaFree(ctx->d_items); cudaFree(ctx->d_slots); cudaFree(ctx->d_queue); cudaFree(ctx->d_stats);
   cudaFree(ctx->d_err); cudaFree(ctx->d_prof); cudaFree(ctx->d_warp_ns);
   cudaFree(ctx->d_order); cudaFree(ctx->d_status); cudaFree(ctx->d_rstart); cudaFree(ctx->d_um);
-  cudaFree(ctx->d_dm); cudaFree(ctx->d_dets);
+  cudaFree(ctx->d_dm); cudaFree(ctx->d_dets); cudaFree(ctx->d_start);
   for (auto* a : ctx->d_aux) cudaFree(a);
   cudaFree(ctx->d_steplog); cudaFree(ctx->d_steplog_n);
   cudaFree(ctx->d_propw); cudaFree(ctx->d_propnorm); cudaFree(ctx->d_prop_kopt); cudaFree(ctx->d_prop_hs);
@@ -477,6 +478,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   if (grow(ctx, ctx->d_um, ctx->um_cap, S.nu)) return GEM_ERROR;
   if (grow(ctx, ctx->d_dm, ctx->dm_cap, S.nd)) return GEM_ERROR;
   if (grow(ctx, ctx->d_rstart, ctx->rstart_cap, 2 * (size_t)nkf)) return GEM_ERROR;
+  if (grow(ctx, ctx->d_start, ctx->start_cap, (size_t)nslot * 2 * START_ENTRIES)) return GEM_ERROR;
   if (grow(ctx, ctx->d_dets, ctx->dets_cap, S.ndet)) return GEM_ERROR;
   // ---- grid: the largest of the three phases sets the per-lane scratch
   long long nthreads = 0;
@@ -496,6 +498,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   L.nitems = nitems; L.nkf = nkf; L.gf64 = (double2*)d_gf64; L.gfre = d_gfre; L.gfim = d_gfim;
   L.status = status; L.scratch = ctx->d_scratch; L.nthreads = nthreads; L.queue = ctx->d_queue;
   L.stats = ctx->d_stats;
+  L.start_tab = ctx->d_start; L.nslot = nslot;
   L.rstart = ctx->d_rstart; L.um = (double2*)ctx->d_um; L.dm = (double2*)ctx->d_dm; L.dets = (double2*)ctx->d_dets;
   L.prof = nullptr;
   L.warp_ns = nullptr;

@@ -34,6 +34,10 @@ constexpr int MAX_LAYER_KNOTS = 64;    // knots per layer handled by the spline 
 // lane's node storage: A(x0) y0 and the results of the sixth and fourth attempt
 constexpr int FK_LANE_STEP_SLOTS = 15;
 
+// radii of the turning-radius search per frequency and motion type: 400 steps of
+// (R - r0) / 400 reach the top within rounding, in whole warps
+constexpr int START_ENTRIES = 416;
+
 struct PrepArgs {
   int nslot, nk, nlay, attmode;
   double df, fref;
@@ -68,6 +72,8 @@ struct FKLaunch {
   double2* scratch;     // per-thread node storage, element-major
   long long nthreads;   // scratch stride
   unsigned int* queue;  // work-queue counters, one per phase (zeroed before launch)
+  double2* start_tab;   // [nslot][2][START_ENTRIES] (radius, velocity) of the turning-radius search
+  int nslot;
   double* rstart;       // [2][nkf] start radius, toroidal then spheroidal
   double2* um;          // [jre*6][nkf] upward minors at nodes 1..jre
   double2* dm;          // [(nnod-jre+1)*6][nkf] downward minors at nodes jre..nnod

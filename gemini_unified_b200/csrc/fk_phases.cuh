@@ -5,7 +5,8 @@
 // (computeGreenFKSpectraForSynthetics.f90:424-494).  Here each of the three
 // becomes its own persistent kernel over all items of a frequency slab:
 //
-//   fk_setup_kernel   start radii of both motion types (initialValues.f90:71-192)
+//   start_table_kernel, fk_setup_kernel
+//                     start radii of both motion types (initialValues.f90:71-192)
 //   PH_TOR            toroidal minors (toroidalMinors.f90:71-268), toroidal
 //                     unit-jump Green functions (unitJumpGreenFunctions.f90:147-175)
 //                     and the toroidal spectra of every node;
@@ -1087,22 +1088,48 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
 #undef FAIL
 
 // ------------------------------------------------------------------------
-//  Start radii of all items (one thread per item)
+//  Start radii of all items
 // ------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) fk_setup_kernel(const __grid_constant__ FKStatic P, FKLaunch LL) {
-  __shared__ Tab tab;
+__device__ __forceinline__ void load_tab(const FKStatic& P, Tab& tab) {
   for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.rk[i] = P.rk[i];
   for (int i = threadIdx.x; i <= MAXLAY; i += blockDim.x) {
     tab.drk[i] = P.drk[i]; tab.iktop[i] = P.iktop[i]; tab.rdrk[i] = 1.0 / P.drk[i];
   }
   __syncthreads();
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < LL.nitems; k += (long long)gridDim.x * blockDim.x) {
-    int2 w = LL.items[k];
+}
+
+// start_tab[(slot * 2 + type) * START_ENTRIES + i], type 0 toroidal; one block per (slot, type)
+__global__ void __launch_bounds__(START_ENTRIES) start_table_kernel(const __grid_constant__ FKStatic P, FKLaunch LL) {
+  __shared__ Tab tab;
+  load_tab(P, tab);
+  const int slot = blockIdx.x >> 1;
+  const bool tor = (blockIdx.x & 1) == 0;
+  Env e;
+  e.tab = &tab;
+  set_env(P, LL, slot, 1, e);
+  LL.start_tab[(long long)blockIdx.x * START_ENTRIES + threadIdx.x] = start_entry(P, e, start_grid(P, tor), threadIdx.x);
+}
+
+// One warp per (item, type).  The walk over up to 400 radii and the integration
+// over up to 400 more are serial chains of spline evaluations, which bound a
+// thread per item whatever the slab: 7.8 ms for a single frequency (96 solves),
+// 10.7 ms for the small global band.  A warp evaluates 32 radii at once and adds
+// their terms in order, so the radii are the same bits: 0.04 and 0.15 ms.
+__global__ void __launch_bounds__(128) fk_setup_kernel(const __grid_constant__ FKStatic P, FKLaunch LL) {
+  __shared__ Tab tab;
+  load_tab(P, tab);
+  const int lane = threadIdx.x & 31;
+  const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < 2LL * LL.nitems; w += nw) {
+    const long long k = w >> 1;
+    const bool tor = (w & 1) == 0;
+    const int2 it = LL.items[k];
     Env e;
     e.tab = &tab;
-    set_env(P, LL, w.x, w.y, e);
-    LL.rstart[k] = start_radius(P, e, true);
-    LL.rstart[LL.nkf + k] = start_radius(P, e, false);
+    set_env(P, LL, it.x, it.y, e);
+    const double r = start_radius(P, e, start_grid(P, tor), tor,
+                                  LL.start_tab + (2LL * it.x + (tor ? 0 : 1)) * START_ENTRIES, lane);
+    if (lane == 0) LL.rstart[(tor ? 0 : LL.nkf) + k] = r;
   }
 }
 
@@ -1118,12 +1145,8 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   // refilled from the phase's queue under blk_lock
   __shared__ unsigned long long blk_q;
   __shared__ int blk_lock;
-  for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.rk[i] = P.rk[i];
-  for (int i = threadIdx.x; i <= MAXLAY; i += blockDim.x) {
-    tab.drk[i] = P.drk[i]; tab.iktop[i] = P.iktop[i]; tab.rdrk[i] = 1.0 / P.drk[i];
-  }
   if (threadIdx.x == 0) { blk_q = 0ull; blk_lock = 0; }
-  __syncthreads();
+  load_tab(P, tab);
 #if GEM_FAST
   for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.kb[i] = tab.rk[i];
   __syncthreads();

@@ -629,42 +629,78 @@ __device__ __forceinline__ double velocity_at(const FKStatic& P, const Env& e, d
 __device__ __forceinline__ double vslow(double om, double dll1, double r, double v) {
   return dll1 / (r * r) - (om / v) * (om / v);
 }
-__device__ double integrate_slowness(const FKStatic& P, const Env& e, double rturn, double dr, bool tor) {
-  double q = 0.0, r = rturn;
-  double rbot = (tor && P.hascore) ? P.roc : P.rhs - TENTH_F * dr;
-  const double qmax = -log(1.e-5);
-  while (q < qmax) {
-    if (r - dr < rbot) { r = rbot; break; }
-    r = r - dr;
-    int nl, top;
-    layer_index(P, r, nl, top);
-    double v = velocity_at(P, e, r, nl);
-    q = q + dr * sqrt(vslow(e.omre, e.dll1, r, v));
-  }
-  return r;
+// The search for the turning radius walks the same radii r_i, r_{i+1} =
+// min(r_i + dr, rmax), for every degree of a frequency: start_table_kernel lists
+// them with their velocities once per frequency and motion type.
+struct StartGrid {
+  double r0, dr, rmax, rbot;
+  int nl0;
+};
+__device__ __forceinline__ StartGrid start_grid(const FKStatic& P, bool tor) {
+  StartGrid g;
+  if (tor && P.hascore) { g.r0 = P.roc; g.nl0 = P.noc + 1; } else { g.r0 = P.rhs; g.nl0 = 1; }
+  g.dr = (P.rearth - g.r0) / 400.0;
+  g.rmax = (tor && P.hasocean) ? P.ruc : P.rearth;
+  g.rbot = (tor && P.hascore) ? P.roc : P.rhs - TENTH_F * g.dr;
+  return g;
 }
-__device__ double start_radius(const FKStatic& P, const Env& e, bool tor) {
-  double r; int nl;
-  if (tor && P.hascore) { r = P.roc; nl = P.noc + 1; } else { r = P.rhs; nl = 1; }
-  double dr = (P.rearth - r) / 400.0;
-  double v = velocity_at(P, e, r, nl);
-  double p = vslow(e.omre, e.dll1, r, v), pold = p;
-  if (p <= 0.0) {
-    if (tor && P.hascore) return P.roc;
-    return P.rhs - TENTH_F * dr;
+// entry i of the table; r_i is rmax from some i <= 402 on
+__device__ __forceinline__ double2 start_entry(const FKStatic& P, const Env& e, const StartGrid& g, int i) {
+  double r = g.r0;
+  for (int j = 0; j < i; ++j) r = fmin(r + g.dr, g.rmax);
+  int nl = g.nl0, top;
+  if (i > 0) layer_index(P, r, nl, top);
+  return make_double2(r, velocity_at(P, e, r, nl));
+}
+// integrate the vertical slowness downwards from rturn until its decay reaches
+// 1e-5 or the bottom (initialValues.f90:158-192): one warp evaluates 32 radii at
+// a time and adds their terms in order
+__device__ __forceinline__ double integrate_slowness(const FKStatic& P, const Env& e, const StartGrid& g, double rturn,
+                                                     int lane) {
+  const double qmax = -log(1.e-5);
+  double q = 0.0, r = rturn;
+  for (;;) {
+    double rl = r, prev = r;
+    for (int j = 0; j < 32; ++j)
+      if (j <= lane) { prev = rl; rl = rl - g.dr; }
+    const bool bottom = prev - g.dr < g.rbot;
+    double c = 0.0;
+    if (!bottom) {
+      int nl, top;
+      layer_index(P, rl, nl, top);
+      const double v = velocity_at(P, e, rl, nl);
+      c = g.dr * sqrt(vslow(e.omre, e.dll1, rl, v));
+    }
+    const unsigned bm = __ballot_sync(0xffffffffu, bottom);
+    for (int l = 0; l < 32; ++l) {
+      if (!(q < qmax)) return r;
+      if (bm >> l & 1u) return g.rbot;
+      r = __shfl_sync(0xffffffffu, rl, l);
+      q = q + __shfl_sync(0xffffffffu, c, l);
+    }
   }
-  double rmax = (tor && P.hasocean) ? P.ruc : P.rearth;
-  while (p > 0.0) {
-    pold = p;
-    if (fabs(1.0 - r / rmax) < EPS_D) return integrate_slowness(P, e, rmax, dr, tor);
-    r = fmin(r + dr, rmax);
-    int top;
-    layer_index(P, r, nl, top);
-    v = velocity_at(P, e, r, nl);
-    p = vslow(e.omre, e.dll1, r, v);
+}
+// Start radius of one (omega, l) and motion type, by one warp (initialValues.f90:71-150)
+__device__ double start_radius(const FKStatic& P, const Env& e, const StartGrid& g, bool tor,
+                               const double2* __restrict__ tab, int lane) {
+  double plast = 0.0;   // the value before the current 32
+  for (int base = 0; base < START_ENTRIES; base += 32) {
+    const double2 rv = tab[base + lane];
+    const double p = vslow(e.omre, e.dll1, rv.x, rv.y);
+    const bool attop = fabs(1.0 - rv.x / g.rmax) < EPS_D;
+    const unsigned m = __ballot_sync(0xffffffffu, !(p > 0.0) || attop);
+    if (m) {
+      const int l = __ffs(m) - 1;
+      const double r = __shfl_sync(0xffffffffu, rv.x, l), pi = __shfl_sync(0xffffffffu, p, l);
+      double pold = __shfl_sync(0xffffffffu, p, max(l - 1, 0));
+      if (l == 0) pold = plast;
+      if (base + l == 0 && !(pi > 0.0)) return (tor && P.hascore) ? P.roc : P.rhs - TENTH_F * g.dr;
+      if (pi > 0.0) return integrate_slowness(P, e, g, g.rmax, lane);
+      return integrate_slowness(P, e, g, r - g.dr * pi / (pi - pold), lane);
+    }
+    plast = __shfl_sync(0xffffffffu, p, 31);
   }
-  double rturn = r - dr * p / (p - pold);
-  return integrate_slowness(P, e, rturn, dr, tor);
+  return g.rmax;   // not reached: the table ends at rmax
 }
 
 // ------------------------------------------------------------------------

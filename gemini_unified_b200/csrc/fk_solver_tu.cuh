@@ -95,6 +95,7 @@ cudaError_t launch_fk_phase(int phase, int sched, const FKStatic& P, const FKLau
     case PH_SPH: return launch_fk_sph(sched, P, L, grid, st);
     case PH_ADJ: return launch_sched<PH_ADJ>(sched, P, L, grid, st);
     default:
+      start_table_kernel<<<2 * L.nslot, START_ENTRIES, 0, st>>>(P, L);
       fk_setup_kernel<<<grid, 128, 0, st>>>(P, L);
       return cudaGetLastError();
   }

@@ -57,3 +57,46 @@ def test_fast_step_matches_the_fp64_form(gpu, name, source, stress):
         scale = np.nanmax(np.abs(ref[2]), axis=2, keepdims=True)
         err = np.abs(got[2] - ref[2]) / np.where(scale > 0, scale, 1.0)
         assert np.nanmax(err) <= 1e-8
+
+
+def _ocean(m):
+    """The model with its top layer made an ocean."""
+    sel = slice(int(m.ikbot[-1]) - 1, int(m.iktop[-1]))
+    new = {}
+    for c, v in (("ro", 1020.0), ("vpv", 1450.0), ("vph", 1450.0), ("vsv", 0.0), ("vsh", 0.0)):
+        new[c] = getattr(m, c).copy()
+        new[c][sel] = v
+    iflso = m.iflso.copy()
+    iflso[-1] = 1
+    return dataclasses.replace(m, iflso=iflso, **new)
+
+
+# The start radii (a warp per solve and motion type) with and without a fluid core, with an
+# ocean (toroidal motion ends at its bottom) and in a full space; the first and last degree
+# of the lowest, a middle and the highest frequency.  The FP64 form repeats the reference's
+# arithmetic: 1e-10 of each frequency's largest value, as for the other models.
+START_MODELS = {"core": lambda: configs.prem(), "ocean": lambda: _ocean(configs.prem()), "crust": configs.regional_crust,
+                "full_space": lambda: dataclasses.replace(configs.prem(), fsflag=1)}
+
+
+@pytest.mark.parametrize("name", sorted(START_MODELS))
+def test_start_radii_of_other_models_match_oracle(gpu, name):
+    import oracle
+    from gemini_unified_b200.fk import GeminiFK
+    w = configs.WORKLOADS["global_small"]
+    m = START_MODELS[name]()
+    ex = w.nodes(m)
+    jre = next(j for j in range(ex.nnod, 0, -1) if ex.state[j - 1] == 0)
+    g = M.frequency_grid(w.params, m.rearth)
+    fk, o = GeminiFK(m, ex), oracle.Oracle(m, ex)
+    pc = M.fk_params_c(w.params, jre)
+    for jf in (g.nf1, 20, g.nf2):
+        n = int(g.nwn[jf - 1])
+        _, _, got, st = fk.run(w.params, jre, jf, jf, f32=False, raise_on_failure=False)
+        for iwn in (1, 2, n // 2, n):
+            ref, sto, _ = o.fk_frequency(pc, jf, n, 10, iwn, iwn)
+            a, b = got[:, :, iwn - 1], ref[:, :, iwn - 1]
+            assert st[iwn - 1] == sto[iwn - 1]
+            assert np.array_equal(np.isnan(a), np.isnan(b))
+            ok = ~np.isnan(b)
+            assert np.abs(a[ok] - b[ok]).max(initial=0.0) <= 1e-10 * max(np.abs(b[ok]).max(initial=0.0), 1e-300)
