@@ -52,6 +52,7 @@ struct gem_ctx {
   int32_t* d_status = nullptr; size_t status_cap = 0;
   double* d_rstart = nullptr; size_t rstart_cap = 0;
   double2* d_start = nullptr; size_t start_cap = 0;
+  int* d_status_src = nullptr; size_t status_src_cap = 0;
   double2* d_um = nullptr; size_t um_cap = 0;
   double2* d_dm = nullptr; size_t dm_cap = 0;
   double2* d_dets = nullptr; size_t dets_cap = 0;
@@ -249,7 +250,7 @@ void gem_ctx_destroy(gem_ctx* ctx) {
   cudaFree(ctx->d_items); cudaFree(ctx->d_slots); cudaFree(ctx->d_queue); cudaFree(ctx->d_stats);
   cudaFree(ctx->d_err); cudaFree(ctx->d_prof); cudaFree(ctx->d_warp_ns);
   cudaFree(ctx->d_order); cudaFree(ctx->d_status); cudaFree(ctx->d_rstart); cudaFree(ctx->d_um);
-  cudaFree(ctx->d_dm); cudaFree(ctx->d_dets); cudaFree(ctx->d_start);
+  cudaFree(ctx->d_dm); cudaFree(ctx->d_dets); cudaFree(ctx->d_start); cudaFree(ctx->d_status_src);
   for (auto* a : ctx->d_aux) cudaFree(a);
   cudaFree(ctx->d_steplog); cudaFree(ctx->d_steplog_n);
   cudaFree(ctx->d_propw); cudaFree(ctx->d_propnorm); cudaFree(ctx->d_prop_kopt); cudaFree(ctx->d_prop_hs);
@@ -495,7 +496,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   FKLaunch& L = S.L;
   L.spl = ctx->d_spl; L.poly = fast ? ctx->d_poly : nullptr; L.jf = ctx->d_slots; L.koff = ctx->d_slots + nslot; L.items = ctx->d_items;
   L.order = ctx->d_order;
-  L.nitems = nitems; L.nkf = nkf; L.gf64 = (double2*)d_gf64; L.gfre = d_gfre; L.gfim = d_gfim;
+  L.nitems = nitems; L.nqueue = (unsigned)nitems; L.nkf = nkf; L.gf64 = (double2*)d_gf64; L.gfre = d_gfre; L.gfim = d_gfim;
   L.status = status; L.scratch = ctx->d_scratch; L.nthreads = nthreads; L.queue = ctx->d_queue;
   L.stats = ctx->d_stats;
   L.start_tab = ctx->d_start; L.nslot = nslot;
@@ -505,7 +506,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   L.steplog = ctx->d_steplog; L.steplog_cap = ctx->steplog_cap; L.steplog_n = ctx->d_steplog_n;
   L.prop_kopt = nullptr; L.prop_hs = nullptr;
   L.adv_min = 1; L.adv_wait = 0; L.qgran = 1; L.qchunk = 0;
-  L.nsrc = 0; L.src_blk = 0;
+  L.nsrc = 0; L.src_blk = 0; L.status_src = nullptr;
   ctx->last_grid = S.grid[1];
   ctx->last_block = FK_SCHED_BLOCK[fast ? 1 : 0][S.sched[1]];
   // ---- learned proposer: features / proposals per (phase, item) from the start radii
@@ -594,9 +595,9 @@ int fk_enqueue(gem_ctx* ctx, SlabPlan& S, cudaStream_t st, bool timed) {
 // (computeGreenFKSpectraForASKI.f90:439-560): start radii; the toroidal phase
 // once, with the minors over the node range jsl..jsr of the plan and the
 // toroidal spectra of every source; the spheroidal minors once over the range;
-// then per source node (the moment or force sources jsnod[b], then the force at
-// jre) the adjoint phase with that node as the source.  Each source writes its
-// own output block (block b at b * blk_m; the force block is blk_f long).
+// then the adjoint phase of every source node (the moment or force sources
+// jsnod[b], then the force at jre) as one queue.  Each source writes its own
+// output block (block b at b * blk_m; the force block is blk_f long).
 int fk_enqueue_aski(gem_ctx* ctx, SlabPlan& S, int nsnod, const int* jsnod, int jre, int istyp, float* gre,
                     float* gim, double* g64, size_t blk_m, size_t blk_f, cudaStream_t st) {
   CK(cudaMemsetAsync(ctx->d_spl, 0, S.spl_n * sizeof(double), st));
@@ -616,13 +617,13 @@ int fk_enqueue_aski(gem_ctx* ctx, SlabPlan& S, int nsnod, const int* jsnod, int 
   if (ctx->d_steplog_n) CK(cudaMemsetAsync(ctx->d_steplog_n, 0, sizeof(unsigned long long), st));
   if (ctx->d_prof) CK(cudaMemsetAsync(ctx->d_prof, 0, 32 * sizeof(unsigned long long), st));
   auto launch = [&](int ph, const FKStatic& PX, FKLaunch LX) {
-    const int sc = ph >= 0 ? S.sched[ph] : 0;
-    if (ph >= 0) {
+    const int sc = ph >= 0 && ph < 3 ? S.sched[ph] : 0;
+    if (ph >= 0 && ph < 3) {
       LX.adv_min = FK_DEFER_MIN[S.defer[ph]]; LX.adv_wait = FK_DEFER_WAIT[S.defer[ph]];
       LX.qgran = FK_GRAN[S.qgran[ph]];
       LX.qchunk = FK_QCHUNK[S.qgran[ph]];
     }
-    const int g = ph >= 0 ? S.grid[ph] : ctx->nsm * 8;
+    const int g = ph >= 0 && ph < 3 ? S.grid[ph] : ctx->nsm * 8;
     return S.fast ? gem_fast::launch_fk_phase(ph, sc, PX, LX, g, st) : gem_plain::launch_fk_phase(ph, sc, PX, LX, g, st);
   };
   FKLaunch L0 = S.L;
@@ -648,22 +649,33 @@ int fk_enqueue_aski(gem_ctx* ctx, SlabPlan& S, int nsnod, const int* jsnod, int 
   le = launch(1, S.P, L0);
   nvtxRangePop();
   CK(le);
-  for (int b = 0; b <= nsnod; ++b) {
-    const bool force = b == nsnod;
-    const int js = force ? jre : jsnod[b], ty = force ? 0 : istyp;
-    FKStatic Pb = S.P;
-    Pb.jre = js; Pb.istyp = ty;
-    Pb.njsph = ty == 0 ? 2 : 4; Pb.njtor = ty == 0 ? 1 : 2;
-    Pb.nsp = 4 * Pb.njsph + 2 * Pb.njtor;
-    FKLaunch Lb = L0;
-    const size_t off = (size_t)b * blk_m;
-    Lb.gf64 = g64 ? reinterpret_cast<double2*>(g64) + off : nullptr;
-    Lb.gfre = gre ? gre + off : nullptr;
-    Lb.gfim = gim ? gim + off : nullptr;
-    Lb.dets = reinterpret_cast<double2*>(ctx->d_dets) + (size_t)(js - S.P.jsl) * S.nkf;
-    CK(cudaMemsetAsync(ctx->d_queue, 0, 4 * sizeof(unsigned int), st));
-    CK(launch(2, Pb, Lb));
+  // the adjoint phases of all sources as one queue: a slab of a few frequencies
+  // fills a fraction of the lanes, so the sources one after another each paid
+  // the latency of a whole phase (9 sources and the force, 12,669 degrees: 267
+  // -> 86 ms for the call).  Queue positions are 32 bits: the sources go in
+  // groups that fit.
+  FKLaunch La = Lt;
+  La.status_src = ctx->d_status_src;
+  CK(cudaMemsetAsync(ctx->d_status_src, 0, (size_t)nsrc * S.nkf * sizeof(int), st));
+  const int per = (int)std::max<long long>(1, std::min<long long>(nsrc, 0x7fffffffLL / std::max(S.nitems, 1)));
+  nvtxRangePushA("gem_fk: adjoint phase of the set of sources");
+  le = cudaSuccess;
+  for (int b0 = 0; b0 < nsrc && le == cudaSuccess; b0 += per) {
+    FKLaunch Lg = La;
+    Lg.nsrc = std::min(per, nsrc - b0);
+    Lg.nqueue = (unsigned)Lg.nsrc * (unsigned)S.nitems;
+    for (int b = 0; b < Lg.nsrc; ++b) { Lg.src_node[b] = La.src_node[b0 + b]; Lg.src_type[b] = La.src_type[b0 + b]; }
+    Lg.status_src = La.status_src + (size_t)b0 * S.nkf;
+    const size_t off = (size_t)b0 * blk_m;
+    Lg.gf64 = g64 ? reinterpret_cast<double2*>(g64) + off : nullptr;
+    Lg.gfre = gre ? gre + off : nullptr;
+    Lg.gfim = gim ? gim + off : nullptr;
+    le = cudaMemsetAsync(ctx->d_queue, 0, 4 * sizeof(unsigned int), st);
+    if (le == cudaSuccess) le = launch(2, S.P, Lg);
   }
+  if (le == cudaSuccess) le = launch(3, S.P, La);
+  nvtxRangePop();
+  CK(le);
   // totals only: the per-phase split is not recorded for a set of sources
   for (int ph = 0; ph < 3; ++ph)
     CK(cudaMemcpyAsync(ctx->d_stats + 8 * (ph + 1), ctx->d_stats, 8 * sizeof(unsigned long long),
@@ -856,6 +868,7 @@ int gem_fk_run_aski_device(gem_ctx* ctx, const gem_fk_params* p, int nsnod, cons
   SlabPlan S;
   int rc = fk_prepare(ctx, p, jf_first, jf_last, nullptr, nullptr, nullptr, d_status, S);
   if (rc) return rc;
+  if (grow(ctx, ctx->d_status_src, ctx->status_src_cap, (size_t)(nsnod + 1) * S.nkf)) return GEM_ERROR;
   const size_t blk_m = (size_t)S.nkf * gem_fk_aski_nsp(p->istyp) * ctx->nnod;
   const size_t blk_f = (size_t)S.nkf * gem_fk_aski_nsp(0) * ctx->nnod;
   cudaStream_t st = (cudaStream_t)stream;

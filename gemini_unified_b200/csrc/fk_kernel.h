@@ -64,6 +64,7 @@ struct FKLaunch {
   const int2* items;    // (slot, iwn) of each output index k
   const int* order;     // queue position -> k, most expensive first
   int nitems;
+  unsigned nqueue;      // queue positions: nitems, or nsrc * nitems in the adjoint phase of a set of sources
   long long nkf;        // extent of the wavenumber-frequency index in the outputs
   double2* gf64;        // optional FP64 output (nkf, nsp, nnod)
   float* gfre;          // optional FP32 real part
@@ -91,10 +92,11 @@ struct FKLaunch {
   int adv_min, adv_wait;
   int qgran;            // queue positions reserved per fetch (FK_GRAN)
   int qchunk;           // > 0: runs of queue positions shared by the warps of a block (FK_QCHUNK)
-  // toroidal phase of a set of source nodes (nsrc > 0): per source b its node and
-  // type (0 force, 1 moment), passed by value; its output block starts at
-  // element b * src_blk
+  // toroidal and adjoint phase of a set of source nodes (nsrc > 0): per source b
+  // its node and type (0 force, 1 moment), passed by value; its output block
+  // starts at element b * src_blk; status_src [nsrc][nkf]: adjoint status per source
   int nsrc;
+  int* status_src;
   long long src_blk;
   unsigned char src_node[MAXNOD + 2];
   unsigned char src_type[MAXNOD + 2];
@@ -128,6 +130,7 @@ cudaError_t launch_poly(const PrepArgs& A, double* poly, cudaStream_t st);
 #define GEM_DECLARE_SOLVER(NS)                                                                          \
   namespace NS {                                                                                     \
   /* phase < 0: start radii; 0 toroidal, 1 spheroidal minors, 2 adjoint + spheroidal spectra;     */ \
+  /* 3: status of a set of sources after its adjoint phase;                                       */ \
   /* sched: index into FK_SCHED_BLOCK[build]                                                     */ \
   cudaError_t launch_fk_phase(int phase, int sched, const gem::FKStatic& P, const gem::FKLaunch& L, int grid,  \
                               cudaStream_t st);                                                      \

@@ -62,6 +62,10 @@ struct LaneLayout {
 struct Lane {
   int st, status;
   int k;                // item index = output index k of the slab
+  // adjoint phase: source node and type, the source's index in a set and the
+  // offset of its output block
+  int jre, istyp, src;
+  long long off;
   int iwn;
   Env e;
   double rstart_t, rstart_s;
@@ -536,24 +540,29 @@ __device__ void dsv_tor_derivative(const FKStatic& P, const Env& e, double r, in
     }
 }
 
-// spheroidal part of node n: U, V for every jump, then dU/dr, dV/dr
+// spheroidal part of node n for the source at node jsh (type ty, output block
+// at element off): U, V for every jump, then dU/dr, dV/dr
 __device__ void output_dsv_sph_node(const FKStatic& P, const Env& e, const Slot& s, const LaneLayout& lay, int n,
-                                    const FKLaunch& LL, int k) {
+                                    const FKLaunch& LL, int k, int jsh, int ty, long long off) {
   dz zsph[4][4], ztor[2][2];
-  source_terms(P, e, P.jre, zsph, ztor);
+  source_terms_of(P, e, jsh, ty, zsph, ztor);
+  const int njsph = ty == 0 ? 2 : 4, njtor = ty == 0 ? 1 : 2, nsp = 4 * njsph + 2 * njtor;
   dz g[4][4], d[4][4];
-  for (int j = 0; j < P.njsph; ++j)
+  for (int j = 0; j < njsph; ++j)
     for (int i = 0; i < 4; ++i) {
       dz v{0.0, 0.0};
       for (int kk = 0; kk < 4; ++kk) v = v + s.get(lay.sph(n, kk, i)) * zsph[kk][j];
       g[i][j] = v;
     }
-  dsv_sph_derivative(P, e, P.rnod[n], P.njsph, g, d);
-  int isp = 0;
-  for (int i = 0; i < 4; i += 2)
-    for (int j = 0; j < P.njsph; ++j) put_out(P, LL, k, isp++, n, g[i][j]);
-  for (int i = 0; i < 4; i += 2)
-    for (int j = 0; j < P.njsph; ++j) put_out(P, LL, k, isp++, n, d[i][j]);
+  dsv_sph_derivative(P, e, P.rnod[n], njsph, g, d);
+  for (int q = 0; q < 4 * njsph; ++q) {
+    const int i = 2 * ((q / njsph) & 1), j = q % njsph;
+    const dz v = q < 2 * njsph ? g[i][j] : d[i][j];
+    const long long o = off + k + LL.nkf * ((long long)q + (long long)nsp * (n - 1));
+    if (LL.gf64) LL.gf64[o] = make_double2(v.re, v.im);
+    if (LL.gfre) LL.gfre[o] = (float)v.re;
+    if (LL.gfim) LL.gfim[o] = (float)v.im;
+  }
 }
 
 // toroidal part of node n: W for every jump, then dW/dr
@@ -592,9 +601,11 @@ __device__ void output_dsv_tor_src(const FKStatic& P, const Env& e, const dz ti[
 
 // spheroidal spectra of node n: reciprocity (reciprocity.f90:82-153) and
 // gfsph = bgsph * zsph (computeGreenFKSpectraForSynthetics.f90:445-494)
-__device__ void output_sph_node(const FKStatic& P, const Env& e, const Slot& s, const LaneLayout& lay, int n,
-                                const FKLaunch& LL, int k) {
-  if (P.dsv) { output_dsv_sph_node(P, e, s, lay, n, LL, k); return; }
+__device__ void output_sph_node(const FKStatic& P, const Slot& s, const LaneLayout& lay, int n, const FKLaunch& LL,
+                                const Lane& L) {
+  const Env& e = L.e;
+  const int k = L.k;
+  if (P.dsv) { output_dsv_sph_node(P, e, s, lay, n, LL, k, L.jre, L.istyp, L.off); return; }
   const double re = P.rnod[P.jre], r = P.rnod[n];
   const double elp1 = e.dll1, rlp1 = 1.0 / elp1, f = (r / re) * (r / re);
   const bool fluid = P.state[n] == 1;
@@ -675,8 +686,8 @@ __device__ void sink_node(const FKStatic& P, const FKLaunch& LL, const Slot& s, 
     default: {   // K_ADJ_UP / K_ADJ_DN: UJGF = mtil * adjoint (unitJumpGreenFunctions.f90:359-372)
       const bool up = L.sink == K_ADJ_UP;
       bool use;
-      if (up) use = n >= P.jre && P.state[n] == 0 && P.rnod[n] < P.ruc;
-      else use = n < P.jre && P.state[n] == 0 && P.rnod[n] >= L.rstart_s && P.rnod[n] > P.roc;
+      if (up) use = n >= L.jre && P.state[n] == 0 && P.rnod[n] < P.ruc;
+      else use = n < L.jre && P.state[n] == 0 && P.rnod[n] >= L.rstart_s && P.rnod[n] > P.roc;
       if (!use) return;
       dz m[6], out[4];
       for (int c = 0; c < 6; ++c) m[c] = up ? IS.dm(L.k, n, c, P.jsl) : IS.um(L.k, n, c);
@@ -729,7 +740,8 @@ __device__ void prop_begin(const FKStatic& P, const FKLaunch& LL, const Slot& s,
 template <int PH>
 __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, const Slot& s, const LaneLayout& lay,
                                      Lane& L) {
-  const int jre = P.jre, nnod = P.nnod;
+  int jre = PH == PH_ADJ ? L.jre : P.jre;
+  const int nnod = P.nnod;
   const ItemStore IS{&LL};
   for (int guard = 0; guard < 100000; ++guard) {
     switch (L.st) {
@@ -738,6 +750,11 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
 
       case S_ITEM_INIT: {
         const int2 w = LL.items[L.k];
+        if (PH == PH_ADJ) {
+          L.jre = P.jre; L.istyp = P.istyp; L.off = 0;
+          if (LL.nsrc > 0) { L.jre = LL.src_node[L.src]; L.istyp = LL.src_type[L.src]; L.off = (long long)L.src * LL.src_blk; }
+          jre = L.jre;
+        }
         set_env(P, LL, w.x, w.y, L.e);
         L.iwn = w.y;
         L.status = ST_OK;
@@ -771,7 +788,7 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
           L.st = S_SPH_GROUP;
         } else {   // unitJumpGreenFunctions.f90:194-372
           for (int el = 0; el < LaneLayout::PER_NODE * lay.NN; ++el) s.put(el, dz{0.0, 0.0});
-          double2 d = LL.dets[L.k];
+          double2 d = LL.dets[(long long)(jre - P.jsl) * LL.nkf + L.k];
           L.det = dz{d.x, d.y};
           if (!(zabs(L.det) > TINY_D)) { L.st = L.e.dll1 < EPS_D ? S_OUTPUT : S_ITEM_END; break; }
           if (L.e.dll1 < EPS_D) {   // l = 0 (:201-220)
@@ -967,7 +984,7 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
       }
       case S_ADJ_NEXT: {   // stage = 2*jump + (0 up, 1 down)  (:303-372)
         // jumps 2 and 4 only without stresses, and for the DSV spectra of a force
-        const int sph_mask = (P.dsv ? P.istyp == 1 : P.stressflag) ? 15 : 10;
+        const int sph_mask = (P.dsv ? L.istyp == 1 : P.stressflag) ? 15 : 10;
         int stg = L.stage + 1;
         for (; stg < 8; ++stg) {
           int j = stg >> 1;
@@ -1017,12 +1034,15 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
         break;
       }
       case S_OUTPUT:
-        for (int n = 1; n <= nnod; ++n) output_sph_node(P, L.e, s, lay, n, LL, L.k);
+        for (int n = 1; n <= nnod; ++n) output_sph_node(P, s, lay, n, LL, L);
         L.st = S_ITEM_END;
         break;
 
       case S_ITEM_END:
-        if (L.status != ST_OK && LL.status) LL.status[L.k] = L.status;
+        if (L.status != ST_OK) {
+          if (PH == PH_ADJ && LL.nsrc > 0) LL.status_src[(long long)L.src * LL.nkf + L.k] = L.status;
+          else if (LL.status) LL.status[L.k] = L.status;
+        }
         L.st = S_FETCH;
         return;
 
@@ -1133,6 +1153,28 @@ __global__ void __launch_bounds__(128) fk_setup_kernel(const __grid_constant__ F
   }
 }
 
+// After the adjoint phase of a set of sources: an item's status is that of the
+// first source that failed, and the spheroidal spectra of the sources after it
+// stay zero, as when the sources run one after another.
+__global__ void __launch_bounds__(128) fk_set_status_kernel(FKLaunch LL, int nnod) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= LL.nkf || LL.status[k] != ST_OK) return;
+  int b = 0;
+  while (b < LL.nsrc && LL.status_src[b * LL.nkf + k] == ST_OK) ++b;
+  if (b == LL.nsrc) return;
+  LL.status[k] = LL.status_src[b * LL.nkf + k];
+  for (++b; b < LL.nsrc; ++b) {
+    const int njsph = LL.src_type[b] == 0 ? 2 : 4, nsp = LL.src_type[b] == 0 ? 10 : 20;
+    for (int n = 0; n < nnod; ++n)
+      for (int q = 0; q < 4 * njsph; ++q) {
+        const long long o = b * LL.src_blk + k + LL.nkf * ((long long)q + (long long)nsp * n);
+        if (LL.gf64) LL.gf64[o] = make_double2(0.0, 0.0);
+        if (LL.gfre) LL.gfre[o] = 0.0f;
+        if (LL.gfim) LL.gfim[o] = 0.0f;
+      }
+  }
+}
+
 // ------------------------------------------------------------------------
 //  Lockstep phase kernel
 // ------------------------------------------------------------------------
@@ -1174,6 +1216,15 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   L.st = S_FETCH;
   L.qnext = 0; L.qend = 0;
   const unsigned qg = LL.qgran > 1 ? (unsigned)LL.qgran : 1u;
+  // queue position -> item (a set of sources: source after source, each in cost order)
+  auto take = [&](unsigned pos) {
+    if (PH == PH_ADJ && LL.nsrc > 0) {
+      L.src = (int)(pos / (unsigned)LL.nitems);
+      pos -= (unsigned)L.src * (unsigned)LL.nitems;
+    }
+    L.k = LL.order[pos];
+    L.st = S_ITEM_INIT;
+  };
   unsigned long long cyc_adv = 0, cyc_step = 0, mixed_trips = 0, cyc_minor_sys = 0;
   int waited = 0;   // trips this lane has waited for its bookkeeping
   for (;;) {
@@ -1196,7 +1247,7 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
     for (int round = 0; go && round < 64; ++round) {
       // the next position of the lane's reserved run, without the queue
       if (L.st == S_FETCH && L.qnext < L.qend) {
-        if (L.qnext < (unsigned)LL.nitems) { L.k = LL.order[L.qnext++]; L.st = S_ITEM_INIT; }
+        if (L.qnext < LL.nqueue) take(L.qnext++);
         else L.qnext = L.qend;
       }
       unsigned fm = __ballot_sync(FULL, L.st == S_FETCH);
@@ -1228,7 +1279,7 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
           const unsigned r = (unsigned)__popc(fm & ((1u << lane) - 1u));
           if (r < got) {
             const unsigned my = base + r;
-            if (my < (unsigned)LL.nitems) { L.k = LL.order[my]; L.st = S_ITEM_INIT; }
+            if (my < LL.nqueue) take(my);
             else L.st = S_IDLE;
           }
         }
@@ -1239,7 +1290,7 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
         base = __shfl_sync(FULL, base, leader);
         if (L.st == S_FETCH) {
           const unsigned my = base + (unsigned)__popc(fm & ((1u << lane) - 1u)) * qg;
-          if (my < (unsigned)LL.nitems) { L.k = LL.order[my]; L.st = S_ITEM_INIT; L.qnext = my + 1; L.qend = my + qg; }
+          if (my < LL.nqueue) { take(my); L.qnext = my + 1; L.qend = my + qg; }
           else L.st = S_IDLE;
         }
       }

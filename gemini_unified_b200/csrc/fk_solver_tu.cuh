@@ -94,6 +94,9 @@ cudaError_t launch_fk_phase(int phase, int sched, const FKStatic& P, const FKLau
     case PH_TOR: return launch_fk_tor(sched, P, L, grid, st);
     case PH_SPH: return launch_fk_sph(sched, P, L, grid, st);
     case PH_ADJ: return launch_sched<PH_ADJ>(sched, P, L, grid, st);
+    case 3:
+      fk_set_status_kernel<<<(unsigned)((L.nkf + 127) / 128), 128, 0, st>>>(L, P.nnod);
+      return cudaGetLastError();
     default:
       start_table_kernel<<<2 * L.nslot, START_ENTRIES, 0, st>>>(P, L);
       fk_setup_kernel<<<grid, 128, 0, st>>>(P, L);
