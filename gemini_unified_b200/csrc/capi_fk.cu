@@ -535,6 +535,13 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   return GEM_OK;
 }
 
+// Whether a phase runs in the group form (fk_group.cuh): few queue positions, and
+// none of the instruments of the thread form.
+bool use_groups(const gem_ctx* ctx, const SlabPlan& S, int ph, const FKLaunch& L) {
+  if (!S.fast || ctx->d_prof || ctx->d_warp_ns || ctx->d_steplog) return false;
+  return (long long)L.nqueue <= FK_GROUP_MAX[S.P.hascore][ph];
+}
+
 // The device work of one slab on stream st: zeroing, model preparation, start
 // radii, proposals, the three phases and the per-phase counter snapshots.
 // timed: record the context's events (not inside a graph capture).
@@ -560,6 +567,7 @@ int fk_enqueue(gem_ctx* ctx, SlabPlan& S, cudaStream_t st, bool timed) {
   if (timed) CK(cudaEventRecord(ctx->ev[2], st));
   auto launch = [&](int ph, const FKLaunch& LX, int g) {
     const int sc = ph >= 0 ? S.sched[ph] : 0;
+    if (ph >= 0 && use_groups(ctx, S, ph, LX)) return gem_fast::launch_fk_group(ph, P, LX, ctx->nsm, st);
     return S.fast ? gem_fast::launch_fk_phase(ph, sc, P, LX, g, st) : gem_plain::launch_fk_phase(ph, sc, P, LX, g, st);
   };
   CK(launch(-1, S.L, ctx->nsm * 8));
@@ -623,6 +631,7 @@ int fk_enqueue_aski(gem_ctx* ctx, SlabPlan& S, int nsnod, const int* jsnod, int 
       LX.qgran = FK_GRAN[S.qgran[ph]];
       LX.qchunk = FK_QCHUNK[S.qgran[ph]];
     }
+    if (ph >= 0 && ph < 3 && use_groups(ctx, S, ph, LX)) return gem_fast::launch_fk_group(ph, PX, LX, ctx->nsm, st);
     const int g = ph >= 0 && ph < 3 ? S.grid[ph] : ctx->nsm * 8;
     return S.fast ? gem_fast::launch_fk_phase(ph, sc, PX, LX, g, st) : gem_plain::launch_fk_phase(ph, sc, PX, LX, g, st);
   };

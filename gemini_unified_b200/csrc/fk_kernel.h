@@ -15,6 +15,21 @@ namespace gem {
 constexpr int FK_NSCHED = 6;
 constexpr int FK_SCHED_BLOCK[2][FK_NSCHED] = {{384, 512, 256, 384, 512, 256}, {256, 384, 512, 320, 448, 192}};
 constexpr int FK_SCHED_DEFAULT[3] = {1, 0, 1};   // toroidal, spheroidal, adjoint
+// Largest number of solves a phase of the fast build runs in the group form, 16
+// or 8 lanes per solve (models without and with a fluid core; toroidal,
+// spheroidal, adjoint).  The thread form takes the time of the longest solve
+// whatever the number below its 37,888 lanes, the group form's grows with the
+// solves once its 3,552 groups are busy.  Thread and group form in ms:
+//   PREM to 0.2 Hz    3,206 solves 11.8 / 49 / 12.8 and 4.1 / 16.8 / 4.3,
+//                    22,278 solves 11.1 / 53 / 15.1 and 6.3 / 30 / 15.6;
+//   PREM to 0.05 Hz   4,601 solves 2.6 / 14.0 / 0.35 and 1.1 / 4.1 / 0.28,
+//                    17,961 solves 2.8 / 13.7 / 0.37 and 1.5 / 7.1 / 0.76;
+//   crust to 2 Hz     9,517 solves 2.0 / 4.7 / 7.5 and 0.9 / 3.1 / 4.4,
+//                    21,988 solves 2.1 / 4.8 / 7.7 and 1.9 / 6.7 / 9.3.
+// The lines lie where the slowest model of the kind breaks even: solves of a
+// model with a core differ more in length, and short integrations (adjoints,
+// a crust) spend more in the bookkeeping, which one lane of a group does.
+constexpr int FK_GROUP_MAX[2][3] = {{16000, 9000, 8000}, {24000, 22000, 8000}};
 // candidate deferrals of the bookkeeping passes (lanes waiting, trips waited);
 // the last waits for the whole warp: its lanes, on adjacent degrees of one
 // frequency, reach their sub-interval ends within a few steps of each other
@@ -139,6 +154,10 @@ cudaError_t launch_poly(const PrepArgs& A, double* poly, cudaStream_t st);
   }
 GEM_DECLARE_SOLVER(gem_plain)
 GEM_DECLARE_SOLVER(gem_fast)
+namespace gem_fast {
+// group form of a phase (fk_group.cuh): 16 or 8 lanes per solve, one block per SM
+cudaError_t launch_fk_group(int phase, const gem::FKStatic& P, const gem::FKLaunch& L, int grid, cudaStream_t st);
+}
 namespace gem_ray {
 // travel-time table by ray tracing (raytable.cu): one thread per turning radius
 cudaError_t launch_ray_table(const gem::FKStatic& P, const double* spl, int ntp, int stype, double eps, double drtp,

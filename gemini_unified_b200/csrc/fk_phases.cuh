@@ -43,7 +43,8 @@ template <int PH, int BLK> struct PhaseDiag { static constexpr int L = GEM_FAST 
 // lane states
 enum : int {
   S_FETCH = 0, S_IDLE, S_ITEM_INIT, S_TOR_UP, S_TOR_DONE, S_SPH_GROUP, S_SPH_GROUP_END, S_ADJ_PLAN,
-  S_ADJ_NEXT, S_ADJ_END, S_OUTPUT, S_ITEM_END, S_PROP_NEXT, S_SUB_END, S_INTEG
+  S_ADJ_NEXT, S_ADJ_END, S_OUTPUT, S_ITEM_END, S_PROP_NEXT, S_SUB_END, S_INTEG,
+  S_ITEM_NEW, S_TOR_OUT, S_SPH_NORM, S_SPH_NORMED
 };
 // node sinks
 enum : int { K_DT = 0, K_UT, K_UM, K_DM, K_ADJIC, K_ADJ_UP, K_ADJ_DN };
@@ -81,6 +82,7 @@ struct Lane {
   int sys, nv, sink, after, do_norm;
   int jl, jr, dl, dr, nnodp, ndp, jnod, jd, kmin, nstep;
   double x1, x2, xa, xe, x, h, hdid, lgnorm, s0, s1, idir;
+  int jknot;  // knot interval of the last step (fast build)
   int kopt;   // target attempt of the step-size control
   double hs;  // multiplier of the initial steps given by the initial-value formulas
   dz y[5];
@@ -154,12 +156,14 @@ __device__ __constant__ const StepWork STEPWORK = make_stepwork();
 template <int SYS, int NVD, int DL, bool ISO>
 __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool active, double h, double x,
                                      const dz* y0, dz* yext, int& result, double2* D, int lane, const Slot& xs,
-                                     Counters& cnt_out) {
+                                     Counters& cnt_out, int& jknot) {
   constexpr int NV = SysNV<SYS>::NV;
   // the lane state lives in local memory: work on a register copy of the
   // environment; the counters follow from the attempts made (added at the end)
   const double h48 = h / 48.0;   // grid spacing of the step's sub-steps
-  const EnvF e = make_envf(P, e_in, active, x, x + 48.0 * h48);
+  int jk = jknot;
+  const EnvF e = make_envf(P, e_in, active, x, fma(48.0, h48, x), jk);
+  jknot = jk;
   int lane_att = 0, warp_att = 0;
   bool need = active;
   int res = 0;   // 0: failed; > 0: number of attempts of a successful step
@@ -171,7 +175,7 @@ __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool ac
 #pragma unroll
     for (int v = 0; v < NV; ++v) { z[v] = y0[v]; t[v] = dz{0.0, 0.0}; }
     SysE<SYS> E;
-    sys_at<SYS, ISO>(e, zom2, x, 1.0, E);
+    sys_at<SYS, ISO>(e, zom2, x, E);
     sys_mul<SYS>(E, z, t);
 #pragma unroll
     for (int v = 0; v < NV; ++v) xs.put(v, t[v]);
@@ -356,12 +360,14 @@ __device__ __noinline__ void bs_step(const FKStatic& P, const Env& e_in, bool ac
 // the step of a system: the isotropic form when the whole model is isotropic (fast build)
 template <int SYS, int NVD, int DL>
 __device__ __forceinline__ void bs_step_of(const FKStatic& P, const Env& e, bool active, double h, double x, const dz* y0,
-                                           dz* yext, int& result, double2* D, int lane, const Slot& xs, Counters& cnt) {
+                                           dz* yext, int& result, double2* D, int lane, const Slot& xs, Counters& cnt,
+                                           int& jknot) {
 #if GEM_FAST
-  if (P.iso) bs_step<SYS, NVD, DL, true>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt);
-  else
+  if (P.iso) bs_step<SYS, NVD, DL, true>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt, jknot);
+  else bs_step<SYS, NVD, DL, false>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt, jknot);
+#else
+  bs_step<SYS, NVD, DL, false>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt);
 #endif
-    bs_step<SYS, NVD, DL, false>(P, e, active, h, x, y0, yext, result, D, lane, xs, cnt);
 }
 
 // ------------------------------------------------------------------------
@@ -732,12 +738,91 @@ __device__ void prop_begin(const FKStatic& P, const FKLaunch& LL, const Slot& s,
   L.st = S_PROP_NEXT;
 }
 
+// determinant, toroidal unit-jump Green functions (unitJumpGreenFunctions.f90:147-175)
+// and spectra of the nodes first + 1, first + 1 + step, ...
+template <int PH>
+__device__ void tor_output(const FKStatic& P, const FKLaunch& LL, const Slot& s, const LaneLayout& lay, const Lane& L,
+                           int first, int step) {
+  const int jre = P.jre, nnod = P.nnod;
+  if (LL.nsrc > 0) {   // every source node of a set, each into its own output block
+    for (int b = 0; b < LL.nsrc; ++b) {
+      const int jsh = LL.src_node[b], ty = LL.src_type[b];
+      const dz det = s.get(lay.ut(jsh, 0)) * s.get(lay.dt(jsh, 1)) - s.get(lay.dt(jsh, 0)) * s.get(lay.ut(jsh, 1));
+      if (!(zabs(det) > TINY_D)) continue;
+      const int mask = ty == 1 ? 3 : 2;
+      dz dcoef[2], ecoef[2];
+      for (int j = 0; j < 2; ++j) {
+        double u1 = j == 0 ? 1.0 : 0.0, u2 = j == 1 ? 1.0 : 0.0;
+        dcoef[j] = (u2 * s.get(lay.dt(jsh, 0)) - u1 * s.get(lay.dt(jsh, 1))) / det;
+        ecoef[j] = (u2 * s.get(lay.ut(jsh, 0)) - u1 * s.get(lay.ut(jsh, 1))) / det;
+      }
+      for (int n = 1 + first; n <= nnod; n += step) {
+        dz ti[2][2] = {{{0, 0}, {0, 0}}, {{0, 0}, {0, 0}}};   // [comp][jump]
+        for (int j = 0; j < 2; ++j) {
+          if (!(mask & (1 << j))) continue;
+          if (n < jsh) {
+            if (P.state[n] == 0 && P.rnod[n] > L.rstart_t)
+              for (int c = 0; c < 2; ++c) ti[c][j] = dcoef[j] * s.get(lay.ut(n, c));
+          } else if (P.state[n] == 0) {
+            for (int c = 0; c < 2; ++c) ti[c][j] = ecoef[j] * s.get(lay.dt(n, c));
+          }
+        }
+        output_dsv_tor_src(P, L.e, ti, n, LL, L.k, jsh, ty, (long long)b * LL.src_blk);
+      }
+    }
+    return;
+  }
+  const dz det = s.get(lay.ut(jre, 0)) * s.get(lay.dt(jre, 1)) - s.get(lay.dt(jre, 0)) * s.get(lay.ut(jre, 1));
+  if (!(zabs(det) > TINY_D)) return;
+  // jumps whose Green functions are stored: the DSV spectra of a moment
+  // source use both, those of a force only the second
+  const int tor_mask = (P.dsv ? P.istyp == 1 : P.stressflag) ? 3 : 2;
+  dz dcoef[2], ecoef[2];
+  for (int j = 0; j < 2; ++j) {
+    double u1 = j == 0 ? 1.0 : 0.0, u2 = j == 1 ? 1.0 : 0.0;
+    dcoef[j] = (u2 * s.get(lay.dt(jre, 0)) - u1 * s.get(lay.dt(jre, 1))) / det;
+    ecoef[j] = (u2 * s.get(lay.ut(jre, 0)) - u1 * s.get(lay.ut(jre, 1))) / det;
+  }
+  for (int n = 1 + first; n <= nnod; n += step) {
+    dz ti[2][2] = {{{0, 0}, {0, 0}}, {{0, 0}, {0, 0}}};   // [comp][jump]
+    for (int j = 0; j < 2; ++j) {
+      if (!(tor_mask & (1 << j))) continue;
+      if (n < jre) {
+        if (P.state[n] == 0 && P.rnod[n] > L.rstart_t)
+          for (int c = 0; c < 2; ++c) ti[c][j] = dcoef[j] * s.get(lay.ut(n, c));
+      } else if (P.state[n] == 0) {
+        for (int c = 0; c < 2; ++c) ti[c][j] = ecoef[j] * s.get(lay.dt(n, c));
+      }
+    }
+    output_tor_node(P, L.e, ti, n, LL, L.k);
+  }
+}
+
+// minors of the direction just integrated to its final normalisation factor
+// (spheroidalMinors.f90:360-365,552-557), every step-th node
+__device__ void sph_normalise(const FKStatic& P, const FKLaunch& LL, const Slot& s, const LaneLayout& lay, const Lane& L,
+                              int first, int step) {
+  const ItemStore IS{&LL};
+  const bool up = L.up == 1;
+  const int n0 = up ? 1 : P.jsl, n1 = up ? P.jsr : P.nnod;
+  for (int n = n0 + first; n <= n1; n += step) {
+    double fct = pow(10.0, s.get(lay.lg(n)).re - L.lgnormend);
+    for (int c = 0; c < 6; ++c) {
+      if (up) IS.put_um(L.k, n, c, IS.um(L.k, n, c) * fct);
+      else IS.put_dm(L.k, n, c, P.jsl, IS.dm(L.k, n, c, P.jsl) * fct);
+    }
+  }
+}
+
 #define FAIL(code) do { L.status = (code); L.st = S_ITEM_END; } while (0)
 
 // ------------------------------------------------------------------------
 //  Per-lane bookkeeping of one phase
 // ------------------------------------------------------------------------
-template <int PH>
+// GROUP (a group of lanes per item): called by the group's first lane, returns in
+// the states S_TOR_OUT, S_SPH_NORM and S_OUTPUT, whose loops over the nodes the
+// group shares
+template <int PH, bool GROUP = false>
 __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, const Slot& s, const LaneLayout& lay,
                                      Lane& L) {
   int jre = PH == PH_ADJ ? L.jre : P.jre;
@@ -766,7 +851,8 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
         L.rstart_t = LL.rstart[L.k];
         L.rstart_s = LL.rstart[LL.nkf + L.k];
         if (PH == PH_TOR) {   // toroidalMinors.f90:150-199
-          for (int el = 0; el < 4 * lay.NN; ++el) s.put(el, dz{0.0, 0.0});
+          if (!GROUP)
+            for (int el = 0; el < 4 * lay.NN; ++el) s.put(el, dz{0.0, 0.0});
           L.up = 0;
           L.st = S_TOR_DONE;
           // minors over the source-node range jsl..jsr (toroidalMinors.f90:129-160)
@@ -787,7 +873,8 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
           L.lgnorm_g = 0.0; L.lgnormend = 0.0; L.htry_g = 0.0; L.liq_old = 0;
           L.st = S_SPH_GROUP;
         } else {   // unitJumpGreenFunctions.f90:194-372
-          for (int el = 0; el < LaneLayout::PER_NODE * lay.NN; ++el) s.put(el, dz{0.0, 0.0});
+          if (!GROUP)
+            for (int el = 0; el < LaneLayout::PER_NODE * lay.NN; ++el) s.put(el, dz{0.0, 0.0});
           double2 d = LL.dets[(long long)(jre - P.jsl) * LL.nkf + L.k];
           L.det = dz{d.x, d.y};
           if (!(zabs(L.det) > TINY_D)) { L.st = L.e.dll1 < EPS_D ? S_OUTPUT : S_ITEM_END; break; }
@@ -834,97 +921,20 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
         L.up = 1;
         break;
       }
-      case S_TOR_DONE: {   // determinant and toroidal UJGF (unitJumpGreenFunctions.f90:147-175)
+      case S_TOR_DONE:
         if (L.jr - L.jl < 0) { FAIL(ST_BOOKKEEPING); break; }
-        if constexpr (PH == PH_TOR) {
-          if (LL.nsrc > 0) {   // every source node of a set, each into its own output block
-            for (int b = 0; b < LL.nsrc; ++b) {
-              const int jsh = LL.src_node[b], ty = LL.src_type[b];
-              const dz det =
-                  s.get(lay.ut(jsh, 0)) * s.get(lay.dt(jsh, 1)) - s.get(lay.dt(jsh, 0)) * s.get(lay.ut(jsh, 1));
-              if (!(zabs(det) > TINY_D)) continue;
-              const int mask = ty == 1 ? 3 : 2;
-              dz dcoef[2], ecoef[2];
-              for (int j = 0; j < 2; ++j) {
-                double u1 = j == 0 ? 1.0 : 0.0, u2 = j == 1 ? 1.0 : 0.0;
-                dcoef[j] = (u2 * s.get(lay.dt(jsh, 0)) - u1 * s.get(lay.dt(jsh, 1))) / det;
-                ecoef[j] = (u2 * s.get(lay.ut(jsh, 0)) - u1 * s.get(lay.ut(jsh, 1))) / det;
-              }
-              for (int n = 1; n <= nnod; ++n) {
-                dz ti[2][2] = {{{0, 0}, {0, 0}}, {{0, 0}, {0, 0}}};   // [comp][jump]
-                for (int j = 0; j < 2; ++j) {
-                  if (!(mask & (1 << j))) continue;
-                  if (n < jsh) {
-                    if (P.state[n] == 0 && P.rnod[n] > L.rstart_t)
-                      for (int c = 0; c < 2; ++c) ti[c][j] = dcoef[j] * s.get(lay.ut(n, c));
-                  } else if (P.state[n] == 0) {
-                    for (int c = 0; c < 2; ++c) ti[c][j] = ecoef[j] * s.get(lay.dt(n, c));
-                  }
-                }
-                output_dsv_tor_src(P, L.e, ti, n, LL, L.k, jsh, ty, (long long)b * LL.src_blk);
-              }
-            }
-            L.st = S_ITEM_END;
-            break;
-          }
-        }
-        L.det = s.get(lay.ut(jre, 0)) * s.get(lay.dt(jre, 1)) - s.get(lay.dt(jre, 0)) * s.get(lay.ut(jre, 1));
-        if (!(zabs(L.det) > TINY_D)) { L.st = S_ITEM_END; break; }
-        // jumps whose Green functions are stored: the DSV spectra of a moment
-        // source use both, those of a force only the second
-        const int tor_mask = (P.dsv ? P.istyp == 1 : P.stressflag) ? 3 : 2;
-        dz dcoef[2], ecoef[2];
-        for (int j = 0; j < 2; ++j) {
-          double u1 = j == 0 ? 1.0 : 0.0, u2 = j == 1 ? 1.0 : 0.0;
-          dcoef[j] = (u2 * s.get(lay.dt(jre, 0)) - u1 * s.get(lay.dt(jre, 1))) / L.det;
-          ecoef[j] = (u2 * s.get(lay.ut(jre, 0)) - u1 * s.get(lay.ut(jre, 1))) / L.det;
-        }
-        for (int n = 1; n <= nnod; ++n) {
-          dz ti[2][2] = {{{0, 0}, {0, 0}}, {{0, 0}, {0, 0}}};   // [comp][jump]
-          for (int j = 0; j < 2; ++j) {
-            if (!(tor_mask & (1 << j))) continue;
-            if (n < jre) {
-              if (P.state[n] == 0 && P.rnod[n] > L.rstart_t)
-                for (int c = 0; c < 2; ++c) ti[c][j] = dcoef[j] * s.get(lay.ut(n, c));
-            } else if (P.state[n] == 0) {
-              for (int c = 0; c < 2; ++c) ti[c][j] = ecoef[j] * s.get(lay.dt(n, c));
-            }
-          }
-          output_tor_node(P, L.e, ti, n, LL, L.k);
-        }
+        if (GROUP) { L.st = S_TOR_OUT; return; }
+        tor_output<PH>(P, LL, s, lay, L, 0, 1);
         L.st = S_ITEM_END;
         break;
-      }
 
       // ---------------- spheroidal phase
       case S_SPH_GROUP: {
         const bool up = L.up == 1;
         if (!(up ? L.rend < L.rlim : L.rend > L.rlim)) {
-          // normalise to the final normalisation factor (spheroidalMinors.f90:360-365,552-557)
-          int n0 = up ? 1 : P.jsl, n1 = up ? P.jsr : nnod;
-          for (int n = n0; n <= n1; ++n) {
-            double fct = pow(10.0, s.get(lay.lg(n)).re - L.lgnormend);
-            for (int c = 0; c < 6; ++c) {
-              if (up) IS.put_um(L.k, n, c, IS.um(L.k, n, c) * fct);
-              else IS.put_dm(L.k, n, c, P.jsl, IS.dm(L.k, n, c, P.jsl) * fct);
-            }
-          }
-          if (up) {
-            for (int el = 0; el < lay.NN; ++el) s.put(lay.lg(el), dz{0.0, 0.0});
-            L.up = 0;
-            L.rbeg = P.rearth; L.rend = P.rearth; L.rlim = fmax(L.rstart_s, P.rnod[P.jsl]);
-            L.lgnorm_g = 0.0; L.lgnormend = 0.0; L.liq_old = 0;
-            break;
-          }
-          // determinants at the source nodes jsl..jsr (spheroidalMinors.f90:566-575)
-          for (int js = P.jsl; js <= P.jsr; ++js) {
-            dz u[6], d[6];
-            for (int c = 0; c < 6; ++c) { u[c] = IS.um(L.k, js, c); d[c] = IS.dm(L.k, js, c, P.jsl); }
-            if (P.state[js] == 1 || L.e.dll1 < EPS_D) L.det = u[0] * d[1] - d[0] * u[1];
-            else L.det = ((((u[0] * d[5] + u[5] * d[0]) - u[1] * d[4]) + u[2] * d[3]) + u[3] * d[2]) - u[4] * d[1];
-            LL.dets[(long long)(js - P.jsl) * LL.nkf + L.k] = make_double2(L.det.re, L.det.im);
-          }
-          L.st = S_ITEM_END;
+          if (GROUP) { L.st = S_SPH_NORM; return; }
+          sph_normalise(P, LL, s, lay, L, 0, 1);
+          L.st = S_SPH_NORMED;
           break;
         }
         int nl, top;
@@ -950,6 +960,27 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
         }
         prop_begin<PH>(P, LL, s, lay, L, sys, L.rbeg, L.rend, L.htry_g, ys, true, L.lgnorm_g, up ? K_UM : K_DM,
                        S_SPH_GROUP_END);
+        break;
+      }
+      case S_SPH_NORMED: {
+        const bool up = L.up == 1;
+        if (up) {
+          for (int el = 0; el < lay.NN; ++el) s.put(lay.lg(el), dz{0.0, 0.0});
+          L.up = 0;
+          L.rbeg = P.rearth; L.rend = P.rearth; L.rlim = fmax(L.rstart_s, P.rnod[P.jsl]);
+          L.lgnorm_g = 0.0; L.lgnormend = 0.0; L.liq_old = 0;
+          L.st = S_SPH_GROUP;
+          break;
+        }
+        // determinants at the source nodes jsl..jsr (spheroidalMinors.f90:566-575)
+        for (int js = P.jsl; js <= P.jsr; ++js) {
+          dz u[6], d[6];
+          for (int c = 0; c < 6; ++c) { u[c] = IS.um(L.k, js, c); d[c] = IS.dm(L.k, js, c, P.jsl); }
+          if (P.state[js] == 1 || L.e.dll1 < EPS_D) L.det = u[0] * d[1] - d[0] * u[1];
+          else L.det = ((((u[0] * d[5] + u[5] * d[0]) - u[1] * d[4]) + u[2] * d[3]) + u[3] * d[2]) - u[4] * d[1];
+          LL.dets[(long long)(js - P.jsl) * LL.nkf + L.k] = make_double2(L.det.re, L.det.im);
+        }
+        L.st = S_ITEM_END;
         break;
       }
       case S_SPH_GROUP_END: {
@@ -1034,6 +1065,7 @@ __device__ __noinline__ void advance(const FKStatic& P, const FKLaunch& LL, cons
         break;
       }
       case S_OUTPUT:
+        if (GROUP) return;
         for (int n = 1; n <= nnod; ++n) output_sph_node(P, s, lay, n, LL, L);
         L.st = S_ITEM_END;
         break;
@@ -1118,6 +1150,19 @@ __device__ __forceinline__ void load_tab(const FKStatic& P, Tab& tab) {
   __syncthreads();
 }
 
+// lower bounds of the knot intervals (fast build)
+__device__ __forceinline__ void load_bounds(const FKStatic& P, Tab& tab) {
+#if GEM_FAST
+  for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.kb[i] = tab.rk[i];
+  __syncthreads();
+  if (P.equidis == 1) {
+    for (int nl = 2 + (int)threadIdx.x; nl <= P.nlay; nl += blockDim.x)
+      for (int j1 = tab.iktop[nl - 1] + 1, i = j1; i <= tab.iktop[nl]; ++i) tab.kb[i] = tab.rk[j1] + (i - j1) * tab.drk[nl];
+    __syncthreads();
+  }
+#endif
+}
+
 // start_tab[(slot * 2 + type) * START_ENTRIES + i], type 0 toroidal; one block per (slot, type)
 __global__ void __launch_bounds__(START_ENTRIES) start_table_kernel(const __grid_constant__ FKStatic P, FKLaunch LL) {
   __shared__ Tab tab;
@@ -1189,15 +1234,7 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   __shared__ int blk_lock;
   if (threadIdx.x == 0) { blk_q = 0ull; blk_lock = 0; }
   load_tab(P, tab);
-#if GEM_FAST
-  for (int i = threadIdx.x; i <= MAXKNOT; i += blockDim.x) tab.kb[i] = tab.rk[i];
-  __syncthreads();
-  if (P.equidis == 1) {
-    for (int nl = 2 + (int)threadIdx.x; nl <= P.nlay; nl += blockDim.x)
-      for (int j1 = tab.iktop[nl - 1] + 1, i = j1; i <= tab.iktop[nl]; ++i) tab.kb[i] = tab.rk[j1] + (i - j1) * tab.drk[nl];
-    __syncthreads();
-  }
-#endif
+  load_bounds(P, tab);
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   constexpr int DL = PhaseDiag<PH, BLK>::L;
@@ -1214,6 +1251,7 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
   Lane L;
   L.e.tab = &tab;
   L.st = S_FETCH;
+  L.jknot = 1;
   L.qnext = 0; L.qend = 0;
   const unsigned qg = LL.qgran > 1 ? (unsigned)LL.qgran : 1u;
   // queue position -> item (a set of sources: source after source, each in cost order)
@@ -1311,26 +1349,26 @@ __global__ void __launch_bounds__(BLK, 1) fk_phase_kernel(const __grid_constant_
     dz yext[5];
     int result = 0;
     if (PH == PH_TOR) {
-      bs_step_of<SYS_TOROIDAL, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
+      bs_step_of<SYS_TOROIDAL, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt, L.jknot);
     } else if (PH == PH_ADJ) {
-      bs_step_of<SYS_SOLIDT, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt);
+      bs_step_of<SYS_SOLIDT, NVD, DL>(P, L.e, integ, L.h, L.x, L.y, yext, result, D, lane, xs, cnt, L.jknot);
     } else {
       unsigned sysmask = __reduce_or_sync(FULL, integ ? (1u << L.sys) : 0u);
       mixed_trips += __popc(sysmask) > 1;
       if (sysmask & (1u << SYS_MINORS))
         bs_step_of<SYS_MINORS, NVD, DL>(P, L.e, integ && L.sys == SYS_MINORS, L.h, L.x, L.y, yext, result, D, lane, xs,
-                                          cnt);
+                                          cnt, L.jknot);
       const unsigned long long c2 = clock64();
       if (sysmask & (1u << SYS_FLUID)) {
         int r = 0;
         bs_step_of<SYS_FLUID, NVD, DL>(P, L.e, integ && L.sys == SYS_FLUID, L.h, L.x, L.y, yext, r, D, lane, xs,
-                                          cnt);
+                                          cnt, L.jknot);
         if (integ && L.sys == SYS_FLUID) result = r;
       }
       if (sysmask & (1u << SYS_RADIAL)) {
         int r = 0;
         bs_step_of<SYS_RADIAL, NVD, DL>(P, L.e, integ && L.sys == SYS_RADIAL, L.h, L.x, L.y, yext, r, D, lane, xs,
-                                          cnt);
+                                          cnt, L.jknot);
         if (integ && L.sys == SYS_RADIAL) result = r;
       }
       cyc_minor_sys += clock64() - c2;

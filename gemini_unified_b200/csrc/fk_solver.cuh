@@ -176,18 +176,18 @@ struct EnvF : Env {
   bool wide;               // a lane of the warp spans more than two intervals
   double kb1, rk0, rk1;    // kb(jlo+1) (infinite when jlo = jhi), rk(jlo), rk(jlo+1)
 };
-// last interval j of j1..j2 with kb(j) <= r (j1 when there is none)
-__device__ __forceinline__ int knot_interval(const double* __restrict__ kb, int j1, int j2, double r) {
-  int lo = j1, hi = j2;
-  while (lo < hi) {
-    const int m = (lo + hi + 1) >> 1;
-    if (kb[m] <= r) lo = m; else hi = m - 1;
-  }
-  return lo;
+// last interval j of j1..j2 with kb(j) <= r (j1 when there is none), searched
+// from j: a solve's steps move through the intervals one by one
+__device__ __forceinline__ int knot_interval(const double* __restrict__ kb, int j1, int j2, double r, int j) {
+  j = max(j1, min(j, j2));
+  while (j < j2 && kb[j + 1] <= r) ++j;
+  while (j > j1 && kb[j] > r) --j;
+  return j;
 }
+// jknot: interval of the solve's last step (any value gives the same result).
 // Lanes without a step (active false) may hold no layer yet (a lane that never
 // took an item): they read the tables of layer 1 and evaluate nothing.
-__device__ __forceinline__ EnvF make_envf(const FKStatic& P, const Env& e, bool active, double xa, double xb) {
+__device__ __forceinline__ EnvF make_envf(const FKStatic& P, const Env& e, bool active, double xa, double xb, int& jknot) {
   EnvF f;
   static_cast<Env&>(f) = e;
   const Tab* __restrict__ T = e.tab;
@@ -196,8 +196,9 @@ __device__ __forceinline__ EnvF make_envf(const FKStatic& P, const Env& e, bool 
     f.jlo = f.jhi = T->iktop[1];
   } else {
     const int j1 = min(max(T->iktop[nl - 1] + 1, 1), P.nk - 1), j2 = min(T->iktop[nl] - 1, P.nk - 1);
-    f.jlo = knot_interval(T->kb, j1, j2, fmin(xa, xb));
-    f.jhi = knot_interval(T->kb, f.jlo, j2, fmax(xa, xb));
+    f.jlo = knot_interval(T->kb, j1, max(j1, j2), fmin(xa, xb), jknot);
+    f.jhi = knot_interval(T->kb, f.jlo, max(f.jlo, j2), fmax(xa, xb), f.jlo);
+    jknot = f.jlo;
   }
   f.rk0 = T->rk[f.jlo];
   f.rk1 = T->rk[f.jlo + 1];
@@ -249,7 +250,7 @@ __device__ __forceinline__ double rinv(double x) {
 }
 __device__ __forceinline__ dz zinv(dz z) {
 #if GEM_FAST
-  const double r = rinv(z.re * z.re + z.im * z.im);
+  const double r = rinv(fma(z.re, z.re, __dmul_rn(z.im, z.im)));
   return {z.re * r, -z.im * r};
 #else
   return 1.0 / z;
@@ -267,11 +268,12 @@ __device__ __forceinline__ void cfma(dz& acc, double a, dz b) {
   acc.im = fma(a, b.im, acc.im);
 }
 __device__ __forceinline__ dz cmul(dz a, dz b) {
-  return {fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re)};
+  return {fma(a.re, b.re, -__dmul_rn(a.im, b.im)), fma(a.re, b.im, __dmul_rn(a.im, b.re))};
 }
 
-// Entries of w A(x) of the fast build, w the sub-step's weight: z0 + w A z1 is
-// then a chain of FMAs into z0.  w enters in the few factors every entry has one of.
+// Matrix entries of the fast build.  Products and sums are written so that the
+// compiler has no choice in contracting them (fma, or the _rn products): the
+// thread form and the group form of a step give the same bits.
 template <int SYS> struct SysE;
 template <> struct SysE<SYS_MINORS> { dz a, m12, m14, m23, m24, m32, m42, z4; double m11, m13, m22, m33, m55; };
 template <> struct SysE<SYS_FLUID> { dz m12, m21; double m11; };
@@ -279,22 +281,21 @@ template <> struct SysE<SYS_RADIAL> { dz m11, m12, m21, m22; };
 template <> struct SysE<SYS_TOROIDAL> { dz m12, m21; double rr; };
 template <> struct SysE<SYS_SOLIDT> { dz a11, a12, a14, z2, zrpc, a31, a32, a34, a43; double rr, a22, a42; };
 
-// w A(x) from the cubics q at t.  ISO (every knot of the model isotropic:
+// A(x) from the cubics q at t.  ISO (every knot of the model isotropic:
 // A = C, N = L, F = C - 2 L): with m = L/C, A - F^2/C - N = L (3 - 4 m) and
 // F/C = 1 - 2 m, so only the density, C and L are evaluated (5 cubics instead
 // of 11).  zom2 = (omega - i sigma)^2.
 template <int SYS, bool ISO>
 __device__ __forceinline__ void sys_eval(const EnvF& e, dz zom2, const double* __restrict__ q, double t, double x,
-                                         double w, SysE<SYS>& E) {
+                                         SysE<SYS>& E) {
   double ro;
   dz el[7];
   const double dll1 = e.dll1;
+  auto scale = [](double a, dz z) { return dz{__dmul_rn(a, z.re), __dmul_rn(a, z.im)}; };
   if constexpr (SYS == SYS_MINORS || SYS == SYS_SOLIDT) {   // minorsOdeSystem.f90:77-126, solidtOdeSystem.f90:77-114
     horner_spline<ISO ? 0x0Au : 0x1Fu>(q, t, ro, el);
-    const double rr = rinv(x), rs = w * rr, r2s = rs * rr;
-    const dz zrpc = zinv(el[1]), zom = (w * ro) * zom2;
-    const double rl = w * rinv(fma(el[3].re, el[3].re, el[3].im * el[3].im));
-    const dz m23{el[3].re * rl, -el[3].im * rl};
+    const double rr = rinv(x), rr2 = __dmul_rn(rr, rr);
+    const dz zrpc = zinv(el[1]), zom = scale(ro, zom2), rl = zinv(el[3]);
     dz z1, fc, n;   // A - F^2/C - N, F/C, N
     if constexpr (ISO) {
       const dz m = cmul(el[3], zrpc);
@@ -307,60 +308,65 @@ __device__ __forceinline__ void sys_eval(const EnvF& e, dz zom2, const double* _
       z1 = el[0] - n;
       cfma(z1, -el[2], fc);
     }
-    const dz z = r2s * z1, c = r2s * n;
+    const dz z = scale(rr2, z1), c = scale(rr2, n);
     if constexpr (SYS == SYS_MINORS) {
-      E.a = (2.0 * rs) * fc;
-      E.m11 = -2.0 * rs;
-      E.m13 = dll1 * rs;
-      E.m12 = (-2.0 * dll1) * z;
-      E.m14 = (-0.5 * dll1) * E.a;
-      E.m22 = rs - E.a.re;               // the imaginary parts of m22, m33, m55 are -a, -a, +a
-      E.m33 = fma(-3.0, rs, -E.a.re);
-      E.m55 = fma(-5.0, rs, E.a.re);
-      E.m23 = m23;
-      E.m24 = w * zrpc;
-      E.z4 = 4.0 * z;
-      E.m42 = E.z4 - zom;
+      E.a = scale(2.0 * rr, fc);
+      E.m11 = -2.0 * rr;
+      E.m13 = __dmul_rn(dll1, rr);
+      E.m12 = scale(-2.0 * dll1, z);
+      E.m14 = scale(-0.5 * dll1, E.a);
+      E.m22 = __dsub_rn(rr, E.a.re);     // the imaginary parts of m22, m33, m55 are -a, -a, +a
+      E.m33 = fma(-3.0, rr, -E.a.re);
+      E.m55 = fma(-5.0, rr, E.a.re);
+      E.m23 = rl;
+      E.m24 = zrpc;
+      E.z4 = dz{4.0 * z.re, 4.0 * z.im};
+      E.m42 = dz{__dsub_rn(E.z4.re, zom.re), __dsub_rn(E.z4.im, zom.im)};
       E.m32 = dz{fma(dll1, z.re, fma(dll1 - 2.0, c.re, -zom.re)), fma(dll1, z.im, fma(dll1 - 2.0, c.im, -zom.im))};
     } else {
-      E.rr = rs;
-      E.z2 = rs * fc;
-      E.zrpc = (-w) * zrpc;
-      E.a43 = -m23;
-      E.a11 = 2.0 * E.z2;
+      E.rr = rr;
+      E.z2 = scale(rr, fc);
+      E.zrpc = -zrpc;
+      E.a43 = -rl;
+      E.a11 = dz{2.0 * E.z2.re, 2.0 * E.z2.im};
       E.a12 = dz{fma(-4.0, z.re, zom.re), fma(-4.0, z.im, zom.im)};
-      E.a14 = 2.0 * z;
-      E.a22 = fma(2.0, rs, -E.a11.re);   // its imaginary part is -a11
-      E.a31 = (-dll1) * E.z2;
-      E.a32 = (2.0 * dll1) * z;
+      E.a14 = dz{2.0 * z.re, 2.0 * z.im};
+      E.a22 = fma(2.0, rr, -E.a11.re);   // its imaginary part is -a11
+      E.a31 = scale(-dll1, E.z2);
+      E.a32 = scale(2.0 * dll1, z);
       E.a34 = dz{fma(-dll1, z.re, fma(2.0 - dll1, c.re, zom.re)), fma(-dll1, z.im, fma(2.0 - dll1, c.im, zom.im))};
-      E.a42 = (-dll1) * rs;
+      E.a42 = __dmul_rn(-dll1, rr);
     }
   } else if constexpr (SYS == SYS_FLUID) {   // fluidOdeSystem.f90:78-95
     horner_spline<0x02u>(q, t, ro, el);
-    const dz zomro = ro * zom2;
-    const dz k = zinv(el[1]), g = zinv((zomro * x) * x);
-    E.m11 = (-2.0 * w) * rinv(x);
-    E.m12 = w * dz{fma(-dll1, g.re, k.re), fma(-dll1, g.im, k.im)};
-    E.m21 = (-w) * zomro;
+    const dz zomro = scale(ro, zom2);
+    const dz k = zinv(el[1]), g = zinv(scale(__dmul_rn(x, x), zomro));
+    E.m11 = -2.0 * rinv(x);
+    E.m12 = dz{fma(-dll1, g.re, k.re), fma(-dll1, g.im, k.im)};
+    E.m21 = -zomro;
   } else if constexpr (SYS == SYS_RADIAL) {  // radialOdeSystem.f90:78-99
     horner_spline<ISO ? 0x0Au : 0x17u>(q, t, ro, el);
-    if constexpr (ISO) { el[0] = el[1]; el[2] = el[1] - 2.0 * el[3]; el[4] = el[3]; }
-    const dz zomro = ro * zom2;
-    const double rr = rinv(x), rr2 = rr * rr;
-    const dz rc = zinv(el[1]);
-    E.m11 = ((-2.0 * w * rr) * el[2]) * rc;
-    E.m12 = w * rc;
-    E.m21 = w * ((-zomro) + (4.0 * rr2) * ((el[0] - (el[2] * el[2]) * rc) - el[4]));
-    E.m22 = (2.0 * w * rr) * (el[2] * rc - 1.0);
+    if constexpr (ISO) {
+      el[0] = el[1]; el[4] = el[3];
+      el[2] = dz{fma(-2.0, el[3].re, el[1].re), fma(-2.0, el[3].im, el[1].im)};
+    }
+    const dz zomro = scale(ro, zom2);
+    const double rr = rinv(x), rr2 = __dmul_rn(rr, rr);
+    const dz rc = zinv(el[1]), fc = cmul(el[2], rc);
+    dz z1 = el[0] - el[4];   // A - F^2/C - N
+    cfma(z1, -el[2], fc);
+    E.m11 = scale(-2.0 * rr, fc);
+    E.m12 = rc;
+    E.m21 = dz{fma(4.0 * rr2, z1.re, -zomro.re), fma(4.0 * rr2, z1.im, -zomro.im)};
+    E.m22 = scale(2.0 * rr, dz{__dsub_rn(fc.re, 1.0), fc.im});
   } else {                                   // toroidalOdeSystem.f90:81-102
     horner_spline<ISO ? 0x08u : 0x18u>(q, t, ro, el);
-    const dz zom = (w * ro) * zom2;
-    const double rr = rinv(x), rs = w * rr, r2s = (dll1 - 2.0) * (rs * rr);
+    const dz zom = scale(ro, zom2);
+    const double rr = rinv(x), k = __dmul_rn(dll1 - 2.0, __dmul_rn(rr, rr));
     const dz n = el[ISO ? 3 : 4];
-    E.m12 = w * zinv(el[3]);
-    E.m21 = dz{fma(n.re, r2s, -zom.re), fma(n.im, r2s, -zom.im)};
-    E.rr = rs;
+    E.m12 = zinv(el[3]);
+    E.m21 = dz{fma(n.re, k, -zom.re), fma(n.im, k, -zom.im)};
+    E.rr = rr;
   }
 }
 
@@ -392,10 +398,10 @@ __device__ __forceinline__ void sys_mul(const SysE<SYS>& E, const dz* z, dz* acc
 }
 
 template <int SYS, bool ISO>
-__device__ __forceinline__ void sys_at(const EnvF& e, dz zom2, double x, double w, SysE<SYS>& E) {
+__device__ __forceinline__ void sys_at(const EnvF& e, dz zom2, double x, SysE<SYS>& E) {
   double t;
   const double* q = spline_at(e, x, t);
-  sys_eval<SYS, ISO>(e, zom2, q, t, x, w, E);
+  sys_eval<SYS, ISO>(e, zom2, q, t, x, E);
 }
 #else
 template <int SYS>
@@ -516,9 +522,8 @@ __device__ __constant__ const ExtrapTab EXTRAP = make_extrap();
 // beside it: its grid is every second point of the finer one, so both share
 // the system matrices.  t0 = A(xstart) y0 is given (in memory); the grid point g
 // (in 48ths of the step) sits at xstart + g h48, h48 = h / 48 rounded once per step.
-// A sub-step z2 = z0 + 2 hf A z1 accumulates into z0; the coarse one has twice
-// the weight, which its vector takes (exact).  The last sub-step takes half the
-// weight: z_{n-1} + hf A z_n, whose mean with z_n is the result.
+// A sub-step z2 = z0 + A (2 hf z1) accumulates into z0.  The last sub-step takes
+// half the weight: z_{n-1} + A (hf z_n), whose mean with z_n is the result.
 // One evaluation per loop trip: the loop stays small enough for the instruction
 // caches (with two per trip, warps waited longer for instructions than for data).
 template <int SYS, bool ISO>
@@ -531,22 +536,26 @@ __device__ __forceinline__ void midpoint(const EnvF& e, dz zom2, int n, bool pai
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     const dz y = y0[v], t = t0.get(v);
-    f0[v] = y; fine[v] = y + hf * t;
-    c0[v] = y; coarse[v] = y + (2.0 * hf) * t;
+    f0[v] = c0[v] = fine[v] = coarse[v] = y;
+    cfma(fine[v], hf, t);
+    cfma(coarse[v], 2.0 * hf, t);
   }
   double g = 0.0;
 #pragma unroll 1
   for (int m = 1; m <= n; ++m) {
     g += dg;
     SysE<SYS> E;
-    sys_at<SYS, ISO>(e, zom2, xstart + g * h48, m == n ? hf : 2.0 * hf, E);
-    sys_mul<SYS>(E, fine, f0);
+    const double w = m == n ? hf : 2.0 * hf;
+    sys_at<SYS, ISO>(e, zom2, fma(g, h48, xstart), E);
+    dz u[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u[v] = w * fine[v];
+    sys_mul<SYS>(E, u, f0);
 #pragma unroll
     for (int v = 0; v < NV; ++v) { const dz z = f0[v]; f0[v] = fine[v]; fine[v] = z; }
     if (pair && !(m & 1)) {
-      dz u[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) u[v] = 2.0 * coarse[v];
+      for (int v = 0; v < NV; ++v) u[v] = (2.0 * w) * coarse[v];
       sys_mul<SYS>(E, u, c0);
 #pragma unroll
       for (int v = 0; v < NV; ++v) { const dz z = c0[v]; c0[v] = coarse[v]; coarse[v] = z; }

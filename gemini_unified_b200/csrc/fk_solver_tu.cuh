@@ -8,6 +8,9 @@
 #include "fk_kernel.h"
 #include "fk_solver.cuh"
 #include "fk_phases.cuh"
+#if GEM_FAST
+#include "fk_group.cuh"
+#endif
 
 namespace GEM_NS {
 namespace {
@@ -70,6 +73,18 @@ int bps_sched(int sched) {
   return with_block(sched, [&](auto b) { return bps<PH, b.value>(); });
 }
 
+#if GEM_FAST
+template <int PH>
+cudaError_t launch_grp(const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st) {
+  static_assert(group_smem<PH>() + sizeof(Tab) + sizeof(GroupTab) + 1024 <= 227 * 1024, "one block per SM");
+  cudaError_t e = cudaFuncSetAttribute(fk_group_kernel<PH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)group_smem<PH>());
+  if (e != cudaSuccess) return e;
+  fk_group_kernel<PH><<<grid, GP_WARPS * 32, group_smem<PH>(), st>>>(P, L);
+  return cudaGetLastError();
+}
+#endif
+
 }  // namespace
 
 // one translation unit per phase (GEM_PHASE): they compile side by side
@@ -78,11 +93,21 @@ cudaError_t launch_fk_tor(int sched, const FKStatic& P, const FKLaunch& L, int g
   return launch_sched<PH_TOR>(sched, P, L, grid, st);
 }
 int bps_fk_tor(int sched) { return bps_sched<PH_TOR>(sched); }
+#if GEM_FAST
+cudaError_t launch_grp_tor(const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st) {
+  return launch_grp<PH_TOR>(P, L, grid, st);
+}
+#endif
 #elif GEM_PHASE == 1
 cudaError_t launch_fk_sph(int sched, const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st) {
   return launch_sched<PH_SPH>(sched, P, L, grid, st);
 }
 int bps_fk_sph(int sched) { return bps_sched<PH_SPH>(sched); }
+#if GEM_FAST
+cudaError_t launch_grp_sph(const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st) {
+  return launch_grp<PH_SPH>(P, L, grid, st);
+}
+#endif
 #else
 cudaError_t launch_fk_tor(int sched, const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st);
 cudaError_t launch_fk_sph(int sched, const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st);
@@ -114,6 +139,18 @@ int fk_phase_blocks_per_sm(int phase, int sched) {
 }
 
 int fk_lane_slot_per_node() { return LaneLayout::PER_NODE; }
+
+#if GEM_FAST
+cudaError_t launch_grp_tor(const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st);
+cudaError_t launch_grp_sph(const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st);
+cudaError_t launch_fk_group(int phase, const FKStatic& P, const FKLaunch& L, int grid, cudaStream_t st) {
+  switch (phase) {
+    case PH_TOR: return launch_grp_tor(P, L, grid, st);
+    case PH_SPH: return launch_grp_sph(P, L, grid, st);
+    default: return launch_grp<PH_ADJ>(P, L, grid, st);
+  }
+}
+#endif
 #endif
 
 }  // namespace GEM_NS

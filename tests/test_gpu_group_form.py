@@ -1,0 +1,71 @@
+"""The group form of the fast solver's phases (small slabs) against the thread
+form, which a run takes when its instruments are on: both make the same
+arithmetic in the same order, so the spectra, statuses and step counts must be
+equal bit for bit.  Slabs from a few solves to more than the groups in flight,
+every system (toroidal, minors, fluid, degree 0, adjoint), isotropic or not,
+sources, stresses, DSV output, accuracies that need the seventh attempt and
+rejected steps, and one that fails every solve."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from gemini_unified_b200 import configs, model as M
+
+pytestmark = pytest.mark.gpu
+G = configs.GLOBAL_SMALL
+R = configs.REGIONAL_SMALL
+COUNTS = ("steps_ok", "steps_rej", "attempts", "sysmats", "matvecs", "flops")
+
+CASES = {
+    "lowest_frequency": (G, True, dict(), 2, 2),
+    "one_frequency": (G, True, dict(), 30, 30),
+    "several": (G, True, dict(), 40, 46),
+    "anisotropic_stress": (G, False, dict(source_type="FORCE", stressflag=True), 20, 21),
+    "tight_accuracy": (G, True, dict(eps=1.0e-8), 12, 12),
+    "loose_accuracy": (G, True, dict(eps=1.0e-2), 25, 26),
+    "failing": (G, True, dict(eps=1.0e-30), 4, 4),
+    "regional": (R, True, dict(), 20, 24),
+    "regional_stress": (R, True, dict(stressflag=True), 60, 60),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_group_form_equals_thread_form(gpu, name):
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, GeminiFK
+    w, iso, kw, lo, hi = CASES[name]
+    m = w.model() if iso else configs.prem(isotropic=False)
+    ex = w.nodes(m)
+    jre = ex.node_index(w.rec_radius)
+    p = dataclasses.replace(w.params, **kw)
+    fk = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST)
+    got = fk.run(p, jre, lo, hi, raise_on_failure=False)
+    cg = fk.stats()
+    fk.instrument(True)
+    ref = fk.run(p, jre, lo, hi, raise_on_failure=False)
+    cr = fk.stats()
+    fk.instrument(False)
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
+    assert [cg[k] for k in COUNTS] == [cr[k] for k in COUNTS]
+    assert (name == "failing") == bool(np.any(got[3] != 0))
+
+
+@pytest.mark.parametrize("source", ["MOMENT", "FORCE"])
+def test_group_form_of_dsv_and_set_runs(gpu, source):
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, GeminiFK
+    w = dataclasses.replace(G, nnod_blocks=[4], dr_blocks=[10000.0])
+    m = w.model()
+    ex = w.nodes(m)
+    jre = ex.node_index(w.rec_radius)
+    p = dataclasses.replace(w.params, source_type=source)
+    fk = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST)
+    one = fk.run_dsv(p, 2, 15, 16)
+    many = fk.aski_spectra(p, [1, 3, jre], jre, 15, 16)
+    fk.instrument(True)
+    for a, b in zip(one, fk.run_dsv(p, 2, 15, 16)):
+        np.testing.assert_array_equal(a, b)
+    for x, y in zip(many, fk.aski_spectra(p, [1, 3, jre], jre, 15, 16)):
+        for a, b in zip(x, y):
+            np.testing.assert_array_equal(a, b)
+    fk.instrument(False)
