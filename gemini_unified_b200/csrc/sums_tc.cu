@@ -18,11 +18,18 @@
 // five orders of magnitude (near-antipodal stations), which FP16 operands with
 // FP32 accumulation cannot.
 //
-// GEMM kernel: one CTA per 128 x BN output tile (BN 80 with 6 slices, 64 with 7).  Per k-block of 64 degrees,
-// warp 0 issues TMA loads (64-byte swizzle) of the S slices of A and of T into
-// a 2-stage shared-memory ring; warp 1 issues the S(S+1)/2 slice products (2 MMAs
-// of K 32 each) into S TMEM accumulators of BN columns, one per weight w = i + j;
-// warps 2-5 combine the accumulators in FP64 and write C.  All mbarrier waits
+// GEMM kernel: one CTA per 128 x BN output tile.  Up to 80 (7 slices: 64) columns
+// one launch forms all weights w = i + j on tiles of that width; beyond, two launches
+// form the weights from 3 up and then 0..2 on tiles of 160 (128) columns and pass
+// the partial sums in FP64, in the same order of additions, so both forms give the
+// same bits.  Per k-block of 64 degrees, warp 0 issues TMA loads (64-byte swizzle)
+// of the launch's slices of A and of T into a shared-memory ring; warp 1 issues the
+// slice products (2 MMAs of K 32 each) into one TMEM accumulator of BN columns per
+// weight; warps 2-5 combine the accumulators in FP64 and write C.
+// Bound: the tensor pipe's INT8 rate, 160 cycles for 128 x 160 x 32.  4000 stations
+// (batched band): 2.24 ms in one launch of 80-column tiles, 1.01 + 0.63 ms in two of
+// 160; coupling, 1000 points: 2.51 -> 1.10 + 0.51 ms.  Slower: all products of one A
+// slice in a row (2.7 ms), and with the slice kept in the collector buffer (5.3 ms).  All mbarrier waits
 // of the pipeline are bounded by a timer (1 s unless the context sets another
 // limit): a wait that runs out records an error flag, the CTA stops issuing
 // work, waits (bounded by 1 s, whatever the limit) for its own copies and
@@ -50,6 +57,7 @@ constexpr int TC_BM = 128, TC_BN = 80, TC_BK = 64;      // tile; BK int8 = one s
 // the products' error: with 6 slices their spectra reach 5e-8 of a spectrum's peak against the oracle,
 // with 7 (49 bits; 7 accumulators of 64 columns) the FP64 level.
 constexpr int TC_S_FINE = 7, TC_BN_FINE = 64;
+constexpr int TC_BN2 = 160, TC_BN_FINE2 = 128;   // tiles of the two-launch form
 static_assert(TC_BK == 64 || TC_BK == 32, "swizzle spans of 64 or 32 bytes");
 // Two stages: measured on the same step, 3 stages at N = 64 (8.51 ms) and 5 stages of BK = 32
 // at N = 80 (8.74 ms) both lose to 2 stages of BK = 64 at N = 80 (7.63 ms): the operand bytes
@@ -58,13 +66,21 @@ constexpr int TC_STAGES = 2;
 constexpr int TC_A_BYTES = TC_BM * TC_BK;               // 8 KiB per slice
 constexpr int TC_THREADS = 192;
 constexpr int TC_TMEM_COLS = 512;                       // NS accumulators of BN columns (power-of-two allocation)
-// shape of one product: NS slices per operand, BN stations (columns) per tile
-template <int NS, int BN> struct TcShape {
-  static constexpr int B_BYTES = BN * TC_BK;                        // 5 KiB per slice at BN = 80
-  static constexpr int STAGE_BYTES = NS * (TC_A_BYTES + B_BYTES);   // 78 KiB at (6, 80), 84 KiB at (7, 64)
-  static constexpr int SMEM = TC_STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
-  static_assert(NS * BN <= TC_TMEM_COLS, "the accumulators must fit the tensor memory");
+// One launch of the products: the weights WLO <= w < WHI on tiles of BN columns
+// (stations), WHI - WLO accumulators of BN columns.  A product of K 32 reads its
+// 4 KiB of A and 32 BN bytes of B from shared memory; at BN = 80 (all six weights
+// at once) the products kept the tensor pipe 36 % busy and took 78 cycles instead
+// of the 40 of their arithmetic.  Two launches of three weights at BN = 160 (the
+// fine shape: four and three weights at BN = 128) read half of A per column.
+template <int BN_, int WLO_, int WHI_> struct TcShape {
+  static constexpr int BN = BN_, WLO = WLO_, WHI = WHI_, NACC = WHI - WLO;
+  static constexpr int B_BYTES = BN * TC_BK;                         // per slice
+  static constexpr int STAGE_BYTES = WHI * (TC_A_BYTES + B_BYTES);   // slices 0..WHI-1 of A and T
+  static constexpr int STAGES = WHI <= 3 ? 4 : TC_STAGES;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+  static_assert(NACC * BN <= TC_TMEM_COLS, "the accumulators must fit the tensor memory");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "MMA N of kind::i8 with M = 128");
+  static_assert(B_BYTES % 1024 == 0, "swizzled slices start on 1024 bytes");
   static_assert(SMEM <= 227 * 1024, "stages must fit the shared memory of a CTA");
 };
 constexpr unsigned long long TC_WAIT_NS = 1000000000ull;   // default pipeline wait limit and the drain limit
@@ -298,18 +314,35 @@ __host__ __device__ constexpr uint32_t tc_idesc() {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
 
-// The 16 columns [taddr + w stride, + 16) of the NS accumulators w = 0..NS-1,
-// loaded by one asm statement that ends with the wait for all of them: the NS
+// The 16 columns [taddr + k stride, + 16) of the NA accumulators k = 0..NA-1,
+// loaded by one asm statement that ends with the wait for all of them: the NA
 // loads are in flight together, and the compiler sees the registers defined
 // only after the wait.
 #define GEM_TM16(a, k)                                                                                        \
   "=r"(a[k][0]), "=r"(a[k][1]), "=r"(a[k][2]), "=r"(a[k][3]), "=r"(a[k][4]), "=r"(a[k][5]), "=r"(a[k][6]),    \
       "=r"(a[k][7]), "=r"(a[k][8]), "=r"(a[k][9]), "=r"(a[k][10]), "=r"(a[k][11]), "=r"(a[k][12]),             \
       "=r"(a[k][13]), "=r"(a[k][14]), "=r"(a[k][15])
-template <int NS>
-__device__ __forceinline__ void tmem_ld_acc16(uint32_t taddr, uint32_t stride, uint32_t (&v)[NS][16]) {
-  static_assert(NS == 6 || NS == 7, "six or seven accumulators");
-  if constexpr (NS == 6) {
+template <int NA>
+__device__ __forceinline__ void tmem_ld_acc16(uint32_t taddr, uint32_t stride, uint32_t (&v)[NA][16]) {
+  static_assert(NA == 3 || NA == 4 || NA == 6 || NA == 7, "accumulators of a launch");
+  if constexpr (NA == 3) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%48];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%49];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%50];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2)
+        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride));
+  } else if constexpr (NA == 4) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%65];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%66];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%67];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2), GEM_TM16(v, 3)
+        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride), "r"(taddr + 3u * stride));
+  } else if constexpr (NA == 6) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%96];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%97];\n\t"
@@ -318,11 +351,9 @@ __device__ __forceinline__ void tmem_ld_acc16(uint32_t taddr, uint32_t stride, u
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%64,%65,%66,%67,%68,%69,%70,%71,%72,%73,%74,%75,%76,%77,%78,%79}, [%100];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95}, [%101];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
-        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2), GEM_TM16(v, 3),
-          GEM_TM16(v, 4), GEM_TM16(v, 5)
-        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride), "r"(taddr + 3u * stride),
-          "r"(taddr + 4u * stride), "r"(taddr + 5u * stride));
-  } else {
+        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2), GEM_TM16(v, 3), GEM_TM16(v, 4), GEM_TM16(v, 5)
+        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride), "r"(taddr + 3u * stride), "r"(taddr + 4u * stride), "r"(taddr + 5u * stride));
+  } else if constexpr (NA == 7) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%112];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%113];\n\t"
@@ -332,27 +363,30 @@ __device__ __forceinline__ void tmem_ld_acc16(uint32_t taddr, uint32_t stride, u
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95}, [%117];\n\t"
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%96,%97,%98,%99,%100,%101,%102,%103,%104,%105,%106,%107,%108,%109,%110,%111}, [%118];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
-        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2), GEM_TM16(v, 3),
-          GEM_TM16(v, 4), GEM_TM16(v, 5), GEM_TM16(v, 6)
-        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride), "r"(taddr + 3u * stride),
-          "r"(taddr + 4u * stride), "r"(taddr + 5u * stride), "r"(taddr + 6u * stride));
+        : GEM_TM16(v, 0), GEM_TM16(v, 1), GEM_TM16(v, 2), GEM_TM16(v, 3), GEM_TM16(v, 4), GEM_TM16(v, 5), GEM_TM16(v, 6)
+        : "r"(taddr + 0u * stride), "r"(taddr + 1u * stride), "r"(taddr + 2u * stride), "r"(taddr + 3u * stride), "r"(taddr + 4u * stride), "r"(taddr + 5u * stride), "r"(taddr + 6u * stride));
   }
 }
 #undef GEM_TM16
 
-template <int NS, int BN>
+// ADD: part holds the unscaled sums of the weights from WHI on; FINAL: the sums
+// are complete, scaled and written to C, otherwise left unscaled in part.  part is
+// laid out as the epilogue's threads hold it, [tile][column][row of the tile], so
+// its accesses are whole lines and a chunk's loads are in flight together, a chunk
+// ahead (read from C row by row they took 1.3 of the 1.9 ms of the second launch).
+template <class Sh, bool ADD, bool FINAL>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     sums_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                    const int4* __restrict__ tiles, const int* __restrict__ kind_rows,
                    const long long* __restrict__ kind_rowoff, const long long* __restrict__ coff, int nkind, int nsta,
                    long long mtot, const double* __restrict__ rscale, const double* __restrict__ cscale,
-                   double* C, int* err, unsigned long long wait_ns) {
-  using Sh = TcShape<NS, BN>;
+                   double* C, double* part, int* err, unsigned long long wait_ns) {
+  constexpr int BN = Sh::BN, WLO = Sh::WLO, WHI = Sh::WHI, STAGES = Sh::STAGES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + TC_STAGES * Sh::STAGE_BYTES);
-  uint64_t* empty = full + TC_STAGES;
-  uint64_t* acc_full = empty + TC_STAGES;
+  uint64_t* full = (uint64_t*)(smem + STAGES * Sh::STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
@@ -367,7 +401,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const long long rowB = (long long)kind * nsta + n0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -383,39 +417,39 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
-    // ---- producer: the S slices of A and of T per k-block
+    // ---- producer: the slices of A and of T per k-block
     int issued = 0;
     for (int kb = 0; kb < nkb; ++kb) {
-      const int s = kb % TC_STAGES;
-      if (kb >= TC_STAGES && !mbar_wait(&empty[s], ((kb / TC_STAGES) - 1) & 1, abort_flag, wait_ns)) break;
+      const int s = kb % STAGES;
+      if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1, abort_flag, wait_ns)) break;
       unsigned char* st = smem + s * Sh::STAGE_BYTES;
       mbar_expect_tx(&full[s], Sh::STAGE_BYTES);
 #pragma unroll 1
-      for (int i = 0; i < NS; ++i)
+      for (int i = 0; i < WHI; ++i)
         tma_load_2d(st + i * TC_A_BYTES, &mapA, &full[s], kb * TC_BK, (int)(i * mtot + rowA));
 #pragma unroll 1
-      for (int j = 0; j < NS; ++j)
-        tma_load_2d(st + NS * TC_A_BYTES + j * Sh::B_BYTES, &mapB, &full[s], kb * TC_BK,
+      for (int j = 0; j < WHI; ++j)
+        tma_load_2d(st + WHI * TC_A_BYTES + j * Sh::B_BYTES, &mapB, &full[s], kb * TC_BK,
                     (int)(j * (long long)nkind * nsta + rowB));
       ++issued;
     }
-    for (int kb = (issued > TC_STAGES ? issued - TC_STAGES : 0); kb < issued; ++kb)
-      mbar_drain(&full[kb % TC_STAGES], (kb / TC_STAGES) & 1);
+    for (int kb = (issued > STAGES ? issued - STAGES : 0); kb < issued; ++kb)
+      mbar_drain(&full[kb % STAGES], (kb / STAGES) & 1);
   } else if (warp == 1 && lane == 0) {
-    // ---- MMA issuer: accumulator w = i + j at TMEM columns BN w
+    // ---- MMA issuer: accumulator w = i + j at TMEM columns BN (w - WLO)
     bool ok = true;
     for (int kb = 0; kb < nkb; ++kb) {
-      const int s = kb % TC_STAGES;
-      if (!mbar_wait(&full[s], (kb / TC_STAGES) & 1, abort_flag, wait_ns)) { ok = false; break; }
+      const int s = kb % STAGES;
+      if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, wait_ns)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
       const unsigned char* st = smem + s * Sh::STAGE_BYTES;
 #pragma unroll 1
-      for (int i = 0; i < NS; ++i) {
+      for (int i = 0; i < WHI; ++i) {
         const uint64_t da = smem_desc_kmajor(st + i * TC_A_BYTES);
 #pragma unroll 1
-        for (int j = 0; j + i < NS; ++j) {
-          const uint64_t db = smem_desc_kmajor(st + NS * TC_A_BYTES + j * Sh::B_BYTES);
-          const uint32_t dtm = tmem + (uint32_t)((i + j) * BN);
+        for (int j = i < WLO ? WLO - i : 0; j + i < WHI; ++j) {
+          const uint64_t db = smem_desc_kmajor(st + WHI * TC_A_BYTES + j * Sh::B_BYTES);
+          const uint32_t dtm = tmem + (uint32_t)((i + j - WLO) * BN);
 #pragma unroll
           for (int kk = 0; kk < TC_BK / 32; ++kk) {
             const uint64_t adv = (uint64_t)((kk * 32) >> 4);   // 32 int8 = 32 bytes along K
@@ -456,22 +490,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     double* ck = C + coff[kind];
     const double* cs = cscale + (long long)kind * nsta;
     double* stg = reinterpret_cast<double*>(smem) + q * (32 * 17);   // 17: one pad double per row
-    // columns in chunks of 16 (BN is a multiple of 16); the NS accumulators of a
+    double* pt = part + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * (TC_BM * BN) + q * 32 + lane;
+    double nxt[16];
+    if (ADD) {
+#pragma unroll
+      for (int jj = 0; jj < 16; ++jj) nxt[jj] = pt[jj * TC_BM];
+    }
+    // columns in chunks of 16 (BN is a multiple of 16); the accumulators of a
     // chunk are loaded together, then combined smallest weights first
 #pragma unroll 1
     for (int c = 0; c < BN / 16; ++c) {
-      uint32_t v[NS][16];
-      tmem_ld_acc16<NS>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), (uint32_t)BN, v);
       double sum[16];
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) sum[jj] = 0.0;
+      for (int jj = 0; jj < 16; ++jj) sum[jj] = ADD ? nxt[jj] : 0.0;
+      if (ADD && c + 1 < BN / 16) {
 #pragma unroll
-      for (int w = NS - 1; w >= 0; --w) {
+        for (int jj = 0; jj < 16; ++jj) nxt[jj] = pt[((c + 1) * 16 + jj) * TC_BM];
+      }
+      uint32_t v[Sh::NACC][16];
+      tmem_ld_acc16<Sh::NACC>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), (uint32_t)BN, v);
+#pragma unroll
+      for (int w = WHI - 1; w >= WLO; --w) {
         const double wgt = ldexp(1.0, -7 * (w + 2));
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) sum[jj] += (double)(int)v[w][jj] * wgt;
+        for (int jj = 0; jj < 16; ++jj) sum[jj] += (double)(int)v[w - WLO][jj] * wgt;
       }
-      if (store) {
+      if (store && !FINAL) {
+#pragma unroll
+        for (int jj = 0; jj < 16; ++jj) pt[(c * 16 + jj) * TC_BM] = sum[jj];
+      } else if (store) {
 #pragma unroll
         for (int jj = 0; jj < 16; ++jj) stg[lane * 17 + jj] = sum[jj] * rs;
         __syncwarp();
@@ -535,7 +582,7 @@ bool make_map(CUtensorMap* map, const signed char* base, long long rows, long lo
 
 struct TcLayout {
   int Kp;
-  size_t off[10], total;
+  size_t off[11], total;
 };
 
 int tc_slices(const TcProblem& P) { return P.nslice == TC_S_FINE ? TC_S_FINE : TC_S; }
@@ -544,7 +591,9 @@ TcLayout tc_layout(const TcProblem& P, long long mtot) {
   TcLayout L{};
   const int K = P.lmax + 1, nk = P.nkind, ns = tc_slices(P);
   L.Kp = (K + 63) / 64 * 64;   // the slicing kernels work on 64-degree tiles
-  const size_t sz[10] = {(size_t)ns * nk * P.ncol * L.Kp,             // T8
+  const int bn = ns == TC_S_FINE ? TC_BN_FINE2 : TC_BN2;
+  const bool two = P.ncol > (ns == TC_S_FINE ? TC_BN_FINE : TC_BN);   // launches of the products
+  const size_t sz[11] = {(size_t)ns * nk * P.ncol * L.Kp,             // T8
                         (size_t)ns * mtot * L.Kp,                     // A8
                         (size_t)nk * L.Kp * sizeof(double),           // lscale
                         (size_t)nk * P.ncol * sizeof(double),         // cscale
@@ -553,9 +602,10 @@ TcLayout tc_layout(const TcProblem& P, long long mtot) {
                         (size_t)(mtot / TC_BM + nk + 1) * sizeof(int4),   // tiles
                         (size_t)3 * TC_MAX_KIND * sizeof(long long),  // per-kind tables
                         (size_t)(TC_MAX_KIND + 8) * sizeof(int),      // kind rows + error flag
-                        (size_t)nk * P.ncol * sizeof(unsigned long long)};   // column maxima
+                        (size_t)nk * P.ncol * sizeof(unsigned long long),     // column maxima
+                        two ? (size_t)(mtot / TC_BM + nk + 1) * ((P.ncol + bn - 1) / bn) * TC_BM * bn * sizeof(double) : 0};   // part
   size_t b = 0;
-  for (int i = 0; i < 10; ++i) {
+  for (int i = 0; i < 11; ++i) {
     L.off[i] = b;
     b += (sz[i] + 1023) / 1024 * 1024;
   }
@@ -580,32 +630,72 @@ size_t sums_tc_workspace(const TcProblem& P, long long mtot, int* Kp_out) {
   return L.total;
 }
 
-// operand slices of NS digits and the products on BN-column tiles (blocking)
-template <int NS, int BN>
+struct TcOperands {
+  const TcProblem* P;
+  long long mtot;
+  int Kp;
+  const signed char *T8, *A8;
+  const double *cscale, *rscale;
+  const int4* tiles;
+  size_t ntiles;
+  const int* ints;
+  const long long* tabs;
+  int nslice;
+  double* part;
+};
+
+template <class Sh, bool ADD, bool FINAL>
+const char* tc_products(const TcOperands& O, double* C, int* err, unsigned long long wait_ns, cudaStream_t st) {
+  const int nk = O.P->nkind, ncol = O.P->ncol;
+  // tensor maps over A8 [nslice mtot][Kp] and T8 [nslice * nkind * ncol][Kp]
+  CUtensorMap mA, mB;
+  if (!make_map(&mA, O.A8, O.nslice * O.mtot, O.Kp, TC_BM) ||
+      !make_map(&mB, O.T8, O.nslice * (long long)nk * ncol, O.Kp, Sh::BN))
+    return "sums_tc: cuTensorMapEncodeTiled failed";
+  if (cudaFuncSetAttribute(sums_tc_kernel<Sh, ADD, FINAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::SMEM) !=
+      cudaSuccess)
+    return "sums_tc: shared-memory attribute";
+  dim3 grid((ncol + Sh::BN - 1) / Sh::BN, (unsigned)O.ntiles);
+  sums_tc_kernel<Sh, ADD, FINAL><<<grid, TC_THREADS, Sh::SMEM, st>>>(
+      mA, mB, O.tiles, O.ints, O.tabs + TC_MAX_KIND, O.tabs + 2 * TC_MAX_KIND, nk, ncol, O.mtot, O.rscale, O.cscale, C,
+      O.part, err, wait_ns ? wait_ns : TC_WAIT_NS);
+  return cudaGetLastError() == cudaSuccess ? nullptr : "sums_tc: launch failed";
+}
+
+// operand slices of NS digits and the products (blocking)
+template <int NS>
 const char* tc_slice_and_multiply(const TcProblem& P, long long mtot, int K, int Kp, const double* tab, const double* A,
                                   const double* lscale, const double* cscale, const int* row_kind, signed char* T8,
                                   signed char* A8, double* rscale, const int4* tiles, size_t ntiles, int* ints,
-                                  const long long* tabs, double* C, unsigned long long wait_ns, cudaStream_t st) {
-  using Sh = TcShape<NS, BN>;
+                                  const long long* tabs, double* part, double* C, unsigned long long wait_ns, cudaStream_t st) {
   const int nk = P.nkind, ncol = P.ncol;
   tab_slice_kernel<NS><<<dim3(Kp / 64, (ncol + 63) / 64, nk), 256, 0, st>>>(nk, ncol, P.lcap, K, Kp, tab, lscale,
                                                                             cscale, T8);
   coef_slice_kernel<NS><<<(unsigned)mtot, 256, 0, st>>>(P.lcap, mtot, K, Kp, A, lscale, row_kind, A8, rscale);
-  // tensor maps over A8 [NS mtot][Kp] and T8 [NS * nkind * ncol][Kp]
-  CUtensorMap mA, mB;
-  if (!make_map(&mA, A8, NS * mtot, Kp, TC_BM) || !make_map(&mB, T8, NS * (long long)nk * ncol, Kp, BN))
-    return "sums_tc: cuTensorMapEncodeTiled failed";
-  if (cudaFuncSetAttribute(sums_tc_kernel<NS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::SMEM) !=
-      cudaSuccess)
-    return "sums_tc: shared-memory attribute";
   if (cudaMemsetAsync(ints + TC_MAX_KIND, 0, sizeof(int), st) != cudaSuccess) return "sums_tc: upload failed";
-  dim3 grid((ncol + BN - 1) / BN, (unsigned)ntiles);
-  sums_tc_kernel<NS, BN><<<grid, TC_THREADS, Sh::SMEM, st>>>(mA, mB, tiles, ints, tabs + TC_MAX_KIND,
-                                                             tabs + 2 * TC_MAX_KIND, nk, ncol, mtot, rscale, cscale,
-                                                             C, ints + TC_MAX_KIND, wait_ns ? wait_ns : TC_WAIT_NS);
-  if (cudaGetLastError() != cudaSuccess) return "sums_tc: launch failed";
+  const TcOperands O{&P, mtot, Kp, T8, A8, cscale, rscale, tiles, ntiles, ints, tabs, NS, part};
+  int* err = ints + TC_MAX_KIND;
+  const char* why;
+  // Two launches on wide tiles, unless the columns fit one narrow tile: the wide
+  // tiles' columns beyond ncol are work for nothing.
+  if constexpr (NS == TC_S) {
+    if (ncol <= TC_BN) {
+      why = tc_products<TcShape<TC_BN, 0, TC_S>, false, true>(O, C, err, wait_ns, st);
+    } else {
+      why = tc_products<TcShape<TC_BN2, 3, TC_S>, false, false>(O, C, err, wait_ns, st);
+      if (!why) why = tc_products<TcShape<TC_BN2, 0, 3>, true, true>(O, C, err, wait_ns, st);
+    }
+  } else {
+    if (ncol <= TC_BN_FINE) {
+      why = tc_products<TcShape<TC_BN_FINE, 0, TC_S_FINE>, false, true>(O, C, err, wait_ns, st);
+    } else {
+      why = tc_products<TcShape<TC_BN_FINE2, 3, TC_S_FINE>, false, false>(O, C, err, wait_ns, st);
+      if (!why) why = tc_products<TcShape<TC_BN_FINE2, 0, 3>, true, true>(O, C, err, wait_ns, st);
+    }
+  }
+  if (why) return why;
   int herr = 0;
-  if (cudaMemcpyAsync(&herr, ints + TC_MAX_KIND, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+  if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return "sums_tc: execution failed";
   if (herr) return "sums_tc: a pipeline wait timed out";
@@ -639,6 +729,7 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
   long long* tabs = (long long*)(base + L.off[7]);
   int* ints = (int*)(base + L.off[8]);   // [0..15] rows per kind, [16] error flag
   unsigned long long* colmax = (unsigned long long*)(base + L.off[9]);
+  double* part = (double*)(base + L.off[10]);
   int krows[TC_MAX_KIND + 8] = {0};
   long long htabs[3 * TC_MAX_KIND] = {0};
   std::vector<int4> htiles;
@@ -677,10 +768,10 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
                                                                                 colmax);
   tab_colscale_kernel<<<(nk * ncol + 255) / 256, 256, 0, st>>>(nk * ncol, colmax, cscale);
   if (tc_slices(P) == TC_S_FINE)
-    return tc_slice_and_multiply<TC_S_FINE, TC_BN_FINE>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8,
-                                                      rscale, tiles, htiles.size(), ints, tabs, C, wait_ns, st);
-  return tc_slice_and_multiply<TC_S, TC_BN>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8, rscale, tiles,
-                                            htiles.size(), ints, tabs, C, wait_ns, st);
+    return tc_slice_and_multiply<TC_S_FINE>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8,
+                                                      rscale, tiles, htiles.size(), ints, tabs, part, C, wait_ns, st);
+  return tc_slice_and_multiply<TC_S>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8, rscale, tiles,
+                                            htiles.size(), ints, tabs, part, C, wait_ns, st);
 }
 
 }  // namespace gem
