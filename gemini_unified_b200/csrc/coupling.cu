@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "synth.h"
+#include "tc_slices.cuh"
 
 namespace gem {
 namespace {
@@ -209,6 +210,27 @@ __global__ void __launch_bounds__(CPL_LF_THREADS) cpl_legendre_fast_kernel(int n
   }
 }
 
+// term of degree l < nwn in sum k without the table value and the spectrum
+__device__ __forceinline__ double cpl_weight(const CplSum& cs, int nwn, int l) {
+  if (l < cs.l0) return 0.0;
+  const int lmax = nwn - 1;
+  // cos^2 taper of this frequency (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
+  const double tapfrac = 0.2;
+  int jt = (int)floor((double)lmax * (1.0 - tapfrac) + 0.5);
+  jt = jt < lmax ? jt : lmax;
+  jt = jt > 1 ? jt : 1;
+  double tap = 1.0;
+  if (l >= jt) {
+    const double c1 = (double)lmax * tapfrac * 2.0 / PI_F;
+    const double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
+    const double c = cos((double)(float)l / c1 - c2);
+    tap = c * c;
+  }
+  double c = (2.0 * (double)l + 1.0) / (4.0 * PI_F) * tap;
+  if (cs.fac != 0.0) c = c * (cs.fac / (double)(float)(l * (l + 1)));
+  return c;
+}
+
 // A[aoff[kind] + row * lcap + l], row = 2 (slot nsk[kind] + rank) + re/im: the
 // terms of sum k of frequency nf1 + slot without the table value, zero outside
 // the sum's degrees; one thread per (slot, sum, degree)
@@ -220,23 +242,10 @@ __global__ void cpl_coef_kernel(CplDev S, const float* __restrict__ gr, const fl
   const int k = (int)((idx / S.lcap) % S.nsum);
   const int slot = (int)(idx / ((long long)S.lcap * S.nsum));
   const CplSum cs = S.istyp == 1 ? c_cpl[k] : c_cplf[k];
-  const int jf = S.nf1 + slot, nwn = S.nwn[jf - 1], lmax = nwn - 1;
+  const int nwn = S.nwn[S.nf1 + slot - 1];
   double vr = 0.0, vi = 0.0;
-  if (l >= cs.l0 && l <= lmax) {
-    // cos^2 taper of this frequency (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
-    const double tapfrac = 0.2;
-    int jt = (int)floor((double)lmax * (1.0 - tapfrac) + 0.5);
-    jt = jt < lmax ? jt : lmax;
-    jt = jt > 1 ? jt : 1;
-    double tap = 1.0;
-    if (l >= jt) {
-      const double c1 = (double)lmax * tapfrac * 2.0 / PI_F;
-      const double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
-      const double c = cos((double)(float)l / c1 - c2);
-      tap = c * c;
-    }
-    double c = (2.0 * (double)l + 1.0) / (4.0 * PI_F) * tap;
-    if (cs.fac != 0.0) c = c * (cs.fac / (double)(float)(l * (l + 1)));
+  if (l >= cs.l0 && l < nwn) {
+    const double c = cpl_weight(cs, nwn, l);
     const long long o = (long long)cs.col * S.nkf + S.koff[slot] + l;
     vr = c * (double)gr[o];
     vi = c * (double)gi[o];
@@ -246,6 +255,20 @@ __global__ void cpl_coef_kernel(CplDev S, const float* __restrict__ gr, const fl
   Ar[l] = vr;
   Ar[S.lcap + l] = vi;
 }
+
+// the same rows for the tensor-core products (tc_slices.cuh)
+struct CplRows {
+  CplDev S;
+  __device__ const CplSum& sum(int k) const { return S.istyp == 1 ? c_cpl[k] : c_cplf[k]; }
+  __device__ int nf() const { return S.nf2 - S.nf1 + 1; }
+  __device__ int nsum() const { return S.nsum; }
+  __device__ int nwn(int slot) const { return S.nwn[S.nf1 + slot - 1]; }
+  __device__ int kind(int k) const { return sum(k).kind; }
+  __device__ int rank(int k) const { return S.rank[k]; }
+  __device__ int nsk(int kind) const { return S.nsk[kind]; }
+  __device__ long long index(int slot, int k) const { return (long long)sum(k).col * S.nkf + S.koff[slot]; }
+  __device__ double weight(int slot, int k, int l) const { return cpl_weight(sum(k), nwn(slot), l); }
+};
 
 // FP64 tiled product C[kind][row][pt] = sum_l A[kind][row][l] * T[kind][l][pt]:
 // 128 x 128 output tile per block of 256 threads, 8 x 8 per thread (rows ty + 16 i,
@@ -546,7 +569,8 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   }
   // workspace: tables, coefficient rows, sums, spectra, small inputs
   const size_t b_tab = align256((size_t)npts * CPL_NKIND * lcap * sizeof(double));
-  const size_t b_a = align256((size_t)ao * sizeof(double));
+  const bool fast = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST;   // the tensor-core sums store no coefficient rows
+  const size_t b_a = fast ? 0 : align256((size_t)ao * sizeof(double));
   const size_t b_hd = align256((size_t)co * sizeof(double));
   const size_t b_x = align256((size_t)npts * 6 * p->nf2 * sizeof(double2));
   const size_t b_in = align256((size_t)nf * sizeof(int)) + align256((size_t)p->nf2 * sizeof(int)) +
@@ -592,7 +616,7 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
     cpl_legendre_kernel<<<(npts * 3 + 127) / 128, 128, 0, st>>>(npts, p->nwnmax - 1, lcap, d_delta, tab);
   }
   const long long ncoef = (long long)nf * nsum * lcap;
-  cpl_coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, A);
+  if (!fast) cpl_coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, A);
   int maxnsk = 0;
   for (int kd = 0; kd < CPL_NKIND; ++kd) maxnsk = std::max(maxnsk, S.nsk[kd]);
   const dim3 ggrid((unsigned)((npts + CT_N - 1) / CT_N), (unsigned)((2 * nf * maxnsk + CT_M - 1) / CT_M), CPL_NKIND);
@@ -610,7 +634,10 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
     const size_t wsb = sums_tc_workspace(TP, mtot, nullptr);
     void* tws = gem_ctx_aux(ctx, 14, wsb);
     if (!tws) return GEM_ERROR;
-    if (const char* why = sums_tc_run(TP, nwn, mtot, tab, A, C, tws, wsb, gem_ctx_tc_wait_ns(ctx), st))
+    const TcCoefs rows = [&](const TcCoefSink& K, cudaStream_t s) {
+      return coef_rows_launch(CplRows{S}, nf * nsum, d_gr, d_gi, K, s);
+    };
+    if (const char* why = sums_tc_run(TP, nwn, mtot, tab, rows, C, tws, wsb, gem_ctx_tc_wait_ns(ctx), st))
       return gem_set_error(ctx, why);
   } else {
     cpl_gemm_kernel<<<ggrid, 256, 0, st>>>(S, A, tab, C);

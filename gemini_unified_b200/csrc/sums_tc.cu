@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "synth.h"
+#include "tc_slices.cuh"
 
 namespace gem {
 
@@ -88,48 +89,6 @@ constexpr unsigned long long TC_WAIT_NS = 1000000000ull;   // default pipeline w
 // ---------------------------------------------------------------------------
 //  Operand preparation (FP64 in, INT8 slices out)
 // ---------------------------------------------------------------------------
-
-// smallest power of two strictly above |x| (1 for 0 or non-finite)
-__device__ __forceinline__ double pow2_above(double x) {
-  if (!(x > 0.0) || !isfinite(x)) return 1.0;
-  int e;
-  frexp(x, &e);   // x = f 2^e, f in [0.5, 1)
-  return ldexp(1.0, e);
-}
-
-// the 7-bit slices of x, |x| < 1: x = sum_i q_i 128^-(i+1) + O(128^-S).  The
-// slices are the base-128 digits of u = trunc(|x| 128^S) with the sign of x
-// (x 128^S is exact and the conversion truncates), the same digits as S
-// rounds of x *= 128, q = trunc(x), x -= q, all of which are exact.
-template <int NS>
-__device__ __forceinline__ void slices_of(double x, signed char q[NS]) {
-  static_assert(NS <= 8, "the digits must fit a 64-bit integer");
-  const long long y = (long long)(x * (double)(1ull << (7 * NS)));
-  const unsigned long long u = y < 0 ? (unsigned long long)(-y) : (unsigned long long)y;
-#pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    const int d = (int)((u >> (7 * (NS - 1 - i))) & 127u);
-    q[i] = (signed char)(y < 0 ? -d : d);
-  }
-}
-
-// 1/s for a power of two s whose reciprocal is a normal double (then x * (1/s)
-// equals x / s exactly), else 0: the callers then divide
-__device__ __forceinline__ double inv_pow2(double s) { return s >= 0x1p-1021 && s <= 0x1p1021 ? 1.0 / s : 0.0; }
-__device__ __forceinline__ double div_pow2(double x, double s, double inv) { return inv != 0.0 ? x * inv : x / s; }
-
-__device__ __forceinline__ double block_max(double m) {
-  __shared__ double red[256];
-  red[threadIdx.x] = m;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
-}
 
 // s[kind][l] = power of two above max over stations of |T[kind][l][sta]| (one block per (l, kind))
 __global__ void tab_scale_kernel(int nsta, int lcap, int K, const double* __restrict__ tab, double* lscale, int Kp) {
@@ -194,10 +153,10 @@ __global__ void tab_slice_kernel(int nkind, int nsta, int lcap, int K, int Kp, c
     const int l = l0 + r;
     double v = 0.0;
     if (l < K && sta < nsta) v = div_pow2(div_pow2(tab[((long long)kind * lcap + l) * nsta + sta], sl[r], il[r]), cs, ic);
-    signed char q[NS];
+    int q[NS];
     slices_of<NS>(v, q);
 #pragma unroll
-    for (int j = 0; j < NS; ++j) dig[j][tx][r] = q[j];
+    for (int j = 0; j < NS; ++j) dig[j][tx][r] = (signed char)q[j];
   }
   __syncthreads();
   const long long plane = (long long)nkind * nsta * Kp;
@@ -208,28 +167,6 @@ __global__ void tab_slice_kernel(int nkind, int nsta, int lcap, int K, int Kp, c
 #pragma unroll
     for (int j = 0; j < NS; ++j)
       *reinterpret_cast<uint32_t*>(T8 + j * plane + o) = *reinterpret_cast<const uint32_t*>(&dig[j][r][4 * w]);
-  }
-}
-
-// A8[i][row][l] = slice i of A[row][l] s_l / r_row; one block per row of every kind
-template <int NS>
-__global__ void coef_slice_kernel(int lcap, long long mtot, int K, int Kp, const double* __restrict__ A,
-                                  const double* __restrict__ lscale, const int* __restrict__ row_kind,
-                                  signed char* A8, double* rscale) {
-  const long long row = blockIdx.x;
-  const int kind = row_kind[row];
-  const double* a = A + row * lcap;
-  const double* sl = lscale + (long long)kind * Kp;
-  double m = 0.0;
-  for (int l = threadIdx.x; l < K; l += blockDim.x) m = fmax(m, fabs(a[l] * sl[l]));
-  const double r = pow2_above(block_max(m)), ir = inv_pow2(r);
-  if (threadIdx.x == 0) rscale[row] = r;
-  const long long plane = mtot * Kp;
-  for (int l = threadIdx.x; l < Kp; l += blockDim.x) {
-    signed char q[NS];
-    slices_of<NS>(l < K ? div_pow2(a[l] * sl[l], r, ir) : 0.0, q);
-#pragma unroll
-    for (int i = 0; i < NS; ++i) A8[i * plane + row * Kp + l] = q[i];
   }
 }
 
@@ -598,7 +535,7 @@ TcLayout tc_layout(const TcProblem& P, long long mtot) {
                         (size_t)nk * L.Kp * sizeof(double),           // lscale
                         (size_t)nk * P.ncol * sizeof(double),         // cscale
                         (size_t)mtot * sizeof(double),                // rscale
-                        (size_t)mtot * sizeof(int),                   // row kind
+                        0,
                         (size_t)(mtot / TC_BM + nk + 1) * sizeof(int4),   // tiles
                         (size_t)3 * TC_MAX_KIND * sizeof(long long),  // per-kind tables
                         (size_t)(TC_MAX_KIND + 8) * sizeof(int),      // kind rows + error flag
@@ -664,14 +601,15 @@ const char* tc_products(const TcOperands& O, double* C, int* err, unsigned long 
 
 // operand slices of NS digits and the products (blocking)
 template <int NS>
-const char* tc_slice_and_multiply(const TcProblem& P, long long mtot, int K, int Kp, const double* tab, const double* A,
-                                  const double* lscale, const double* cscale, const int* row_kind, signed char* T8,
+const char* tc_slice_and_multiply(const TcProblem& P, long long mtot, int K, int Kp, const double* tab,
+                                  const TcCoefs& coefs, const double* lscale, const double* cscale, signed char* T8,
                                   signed char* A8, double* rscale, const int4* tiles, size_t ntiles, int* ints,
                                   const long long* tabs, double* part, double* C, unsigned long long wait_ns, cudaStream_t st) {
   const int nk = P.nkind, ncol = P.ncol;
   tab_slice_kernel<NS><<<dim3(Kp / 64, (ncol + 63) / 64, nk), 256, 0, st>>>(nk, ncol, P.lcap, K, Kp, tab, lscale,
                                                                             cscale, T8);
-  coef_slice_kernel<NS><<<(unsigned)mtot, 256, 0, st>>>(P.lcap, mtot, K, Kp, A, lscale, row_kind, A8, rscale);
+  const TcCoefSink sink{K, Kp, NS, TC_BM, TC_BK, mtot, lscale, tabs + TC_MAX_KIND, A8, rscale};
+  if (coefs(sink, st) != cudaSuccess) return "sums_tc: launch of the coefficient rows failed";
   if (cudaMemsetAsync(ints + TC_MAX_KIND, 0, sizeof(int), st) != cudaSuccess) return "sums_tc: upload failed";
   const TcOperands O{&P, mtot, Kp, T8, A8, cscale, rscale, tiles, ntiles, ints, tabs, NS, part};
   int* err = ints + TC_MAX_KIND;
@@ -702,11 +640,11 @@ const char* tc_slice_and_multiply(const TcProblem& P, long long mtot, int K, int
   return nullptr;
 }
 
-// Sliced-integer sums: from the FP64 tables tab[kind][l][col] and coefficients
-// A[kind rows][lcap], write C[kind][row][col] in FP64.  ws: device workspace of
+// Sliced-integer sums: from the FP64 tables tab[kind][l][col] and the coefficient
+// rows that coefs launches, write C[kind][row][col] in FP64.  ws: device workspace of
 // sums_tc_workspace bytes; wait_ns: limit of each pipeline wait (0: 1 s).
 // Blocking (synchronises the stream).
-const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const double* A,
+const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const TcCoefs& coefs,
                         double* C, void* ws, size_t ws_bytes, unsigned long long wait_ns, cudaStream_t st) {
   if (P.nkind < 1 || P.nkind > TC_MAX_KIND) return "sums_tc: table kinds outside 1..16";
   TcLayout L = tc_layout(P, mtot);
@@ -724,7 +662,6 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
   double* lscale = (double*)(base + L.off[2]);
   double* cscale = (double*)(base + L.off[3]);
   double* rscale = (double*)(base + L.off[4]);
-  int* row_kind = (int*)(base + L.off[5]);
   int4* tiles = (int4*)(base + L.off[6]);
   long long* tabs = (long long*)(base + L.off[7]);
   int* ints = (int*)(base + L.off[8]);   // [0..15] rows per kind, [16] error flag
@@ -733,7 +670,6 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
   int krows[TC_MAX_KIND + 8] = {0};
   long long htabs[3 * TC_MAX_KIND] = {0};
   std::vector<int4> htiles;
-  std::vector<int> hrk((size_t)mtot);
   long long ro = 0;
   for (int k = 0; k < nk; ++k) {
     krows[k] = 2 * nf * P.nsk[k];
@@ -748,7 +684,6 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
       ext = std::min(ext, K);
       htiles.push_back(make_int4(k, m, std::max(1, (ext + TC_BK - 1) / TC_BK), 0));
     }
-    for (int m = 0; m < krows[k]; ++m) hrk[(size_t)(ro + m)] = k;
     ro += krows[k];
   }
   if (ro != mtot) return "sums_tc: row count mismatch";
@@ -756,7 +691,6 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
   // longest k-loops first: the short tiles fill the last wave
   std::stable_sort(htiles.begin(), htiles.end(), [](const int4& a, const int4& b) { return a.z > b.z; });
   if (cudaMemcpyAsync(tiles, htiles.data(), htiles.size() * sizeof(int4), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(row_kind, hrk.data(), hrk.size() * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(tabs, htabs, sizeof htabs, cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(ints, krows, sizeof krows, cudaMemcpyHostToDevice, st) != cudaSuccess)
     return "sums_tc: upload failed";
@@ -768,9 +702,9 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
                                                                                 colmax);
   tab_colscale_kernel<<<(nk * ncol + 255) / 256, 256, 0, st>>>(nk * ncol, colmax, cscale);
   if (tc_slices(P) == TC_S_FINE)
-    return tc_slice_and_multiply<TC_S_FINE>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8,
+    return tc_slice_and_multiply<TC_S_FINE>(P, mtot, K, Kp, tab, coefs, lscale, cscale, T8, A8,
                                                       rscale, tiles, htiles.size(), ints, tabs, part, C, wait_ns, st);
-  return tc_slice_and_multiply<TC_S>(P, mtot, K, Kp, tab, A, lscale, cscale, row_kind, T8, A8, rscale, tiles,
+  return tc_slice_and_multiply<TC_S>(P, mtot, K, Kp, tab, coefs, lscale, cscale, T8, A8, rscale, tiles,
                                             htiles.size(), ints, tabs, part, C, wait_ns, st);
 }
 

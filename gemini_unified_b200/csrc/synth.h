@@ -1,5 +1,6 @@
 // Launch-level structure of the synthetics kernels (device pointers only).
 #pragma once
+#include <functional>
 #include <vector>
 #include "../../include/gemini_fk.h"
 #include "gem_device.cuh"
@@ -7,7 +8,7 @@
 namespace gem {
 
 struct SynthDev {
-  int nf1, nf2, nsta, nmt, lmax, lcap, ns, nslog, nsamp, ndec, velocity;
+  int nf1, nf2, nsta, nmt, lmax, lcap, ns, nslog, nsamp, ndec, velocity, global_;
   long long nkf;
   long long ldx;            // complex elements between consecutive spectra of the FFT input
   double df, sigma, tred;
@@ -70,7 +71,7 @@ void event_filter_host(const gem_synth_params* p, std::vector<double2>& h);
 // sliced-integer tensor-core degree sums (sums_tc.cu).  One product per table
 // kind: C[coff[kind] + row * ncol + col] = sum_l A[row][l] T[kind][l][col] for the
 // 2 * nf * nsk[kind] rows of the kind (frequency slot slowest, then sum rank, then
-// re/im; the rows of all kinds contiguous in A with leading dimension lcap), and
+// re/im; the rows of all kinds contiguous), and
 // T[kind][l][col] = tab[(kind * lcap + l) * ncol + col].
 constexpr int TC_MAX_KIND = 16;
 struct TcProblem {
@@ -79,11 +80,25 @@ struct TcProblem {
   int nsk[TC_MAX_KIND];
   long long coff[TC_MAX_KIND];
 };
+// Where the coefficient rows of the products go: slices of nslice digits A8[i][row][Kp]
+// with the row scales rscale; K degrees, products in tiles of tile_rows rows whose
+// k-loops take tile_k degrees a time, lscale[kind][Kp] the degree scales, rowoff
+// [kind] the first row of each kind (device).  TcCoefs launches the kernel that
+// writes them (tc_slices.cuh).
+struct TcCoefSink {
+  int K, Kp, nslice, tile_rows, tile_k;
+  long long mtot;
+  const double* lscale;
+  const long long* rowoff;
+  signed char* A8;
+  double* rscale;
+};
+using TcCoefs = std::function<cudaError_t(const TcCoefSink&, cudaStream_t)>;
 TcProblem tc_problem_of(const SynthDev& S);   // the synthetics' 8 Legendre / Bessel kinds
 // workspace size and run; nwn: host copy of the wavenumber counts per frequency
 // (1-based frequency index); wait_ns: limit of each pipeline wait (0: 1 s)
 size_t sums_tc_workspace(const TcProblem& P, long long mtot, int* Kp_out);
-const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const double* A,
+const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const TcCoefs& coefs,
                         double* C, void* ws, size_t ws_bytes, unsigned long long wait_ns, cudaStream_t st);
 
 }  // namespace gem
