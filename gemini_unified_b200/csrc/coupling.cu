@@ -23,6 +23,7 @@
 #include <cmath>
 #include <vector>
 
+#include "legendre_chain.cuh"
 #include "synth.h"
 #include "tc_slices.cuh"
 
@@ -142,93 +143,79 @@ __global__ void cpl_legendre_kernel(int npts, int lmax, int lcap, const double* 
   cpl_legendre_series(pt, m, npts, lmax, lcap, cos(delta[pt]), sin(delta[pt]), tab);
 }
 
-// Fast form (fast backend): the same tables with the upward recurrence written as
-// p_l = alpha_l p_{l-1} + beta_l p_{l-2} and 1/(l - m) from a shared-memory
-// table, so one FMA per degree sits on the dependent chain (the plain form's
-// software division leaves the 3 npts threads of this kernel waiting on it); the
-// derivative tables follow in FMA form.  Rounding differs from the plain form's
-// only (relative 1e-13 at l = 3200).  Poles keep the plain form's special values.
-constexpr int CPL_LF_THREADS = 64;
-__global__ void __launch_bounds__(CPL_LF_THREADS) cpl_legendre_fast_kernel(int npts, int lmax, int lcap,
-                                                                           const double* __restrict__ delta,
-                                                                           double* tab) {
-  extern __shared__ double rcp[];   // rcp[n] = 1/n, n = 1..lmax
-  for (int n = threadIdx.x + 1; n <= lmax; n += blockDim.x) rcp[n] = 1.0 / (double)n;
-  __syncthreads();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= npts * 3) return;
-  const int pt = idx % npts, m = idx / npts;
-  const double ct = cos(delta[pt]), st = sin(delta[pt]);
-  if (!(st > 0.0)) {
-    cpl_legendre_series(pt, m, npts, lmax, lcap, ct, st, tab);
-    return;
-  }
-  auto row = [&](int kind) { return tab + (long long)kind * lcap * npts + pt; };
-  double* Tp = row(m);
-  double* Td = row(3 + m);
-  double* Ts = m >= 1 ? row(5 + m) : nullptr;
-  double* T2 = row(8 + m);
-  double* Tt = m >= 1 ? row(10 + m) : nullptr;
-  const long long stride = npts;
-  double pmm = 1.0, fact = 1.0;
-  for (int j = 1; j <= m; ++j) { pmm = pmm * fact * st; fact = fact + 2.0; }
-  const double rst = 1.0 / st, ctr = ct * rst, m2r2 = (double)(m * m) * (rst * rst);
+// Fast form (fast backend): the same tables and their exponents from the chains of
+// legendre_chain.cuh, block (32 points, m); the derivative tables follow in FMA
+// form.  Rounding differs from the plain form's only (relative 1e-13 at l = 3200).
+// Poles keep the plain form's special values.  1000 points, 13 tables: 0.15 ms.
+__global__ void __launch_bounds__(LC_THREADS) cpl_legendre_fast_kernel(int npts, int lmax, int lcap,
+                                                                       const double* __restrict__ delta,
+                                                                       double* __restrict__ tab,
+                                                                       short* __restrict__ texp) {
+  const int m = blockIdx.y, pt = blockIdx.x * 32 + (threadIdx.x & 31);
+  const double d = delta[min(pt, npts - 1)];
+  const double ct = cos(d), st = sin(d);
+  const bool pole = !(st > 0.0);
+  const double rst = 1.0 / st, ctr = ct * rst, m2r2 = (double)(m * m) * (rst * rst), md = (double)m;
+  const double isct = ct >= 0.0 ? 1.0 : -1.0;
+  const long long plane = (long long)lcap * npts;
   // d2P/dtheta2 = -(cos/sin) dP/dtheta + (m^2/sin^2 - l(l+1)) P,  d/dtheta (P/sin) = (dP/dtheta - (cos/sin) P)/sin
-  auto put = [&](long long o, double p, double dp, double ll1) {
-    Tp[o] = p;
-    Td[o] = dp;
-    T2[o] = fma(-ctr, dp, (m2r2 - ll1) * p);
-    if (Ts) Ts[o] = p * rst;
-    if (Tt) Tt[o] = rst * fma(-ctr, p, dp);
-  };
-  long long o = 0;
-  for (int l = 0; l < m && l <= lmax; ++l, o += stride) {
-    Tp[o] = 0.0; Td[o] = 0.0; T2[o] = 0.0;
-    if (Ts) Ts[o] = 0.0;
-    if (Tt) Tt[o] = 0.0;
-  }
-  if (m > lmax) return;
-  put(o, pmm, (double)m * ct * pmm * rst, (double)m * (double)(m + 1));   // l = m
-  if (m + 1 > lmax) return;
-  o += stride;
-  const double p1 = ct * (double)(2 * m + 1) * pmm;   // l = m + 1
-  double dl = (double)(m + 1);
-  put(o, p1, fma(dl * ct, p1, -(dl + (double)m) * pmm) * rst, dl * (dl + 1.0));
-  o += stride;
-  double pl2 = pmm, pl1 = p1;
-  const double mm1 = (double)(m - 1), md = (double)m;
-#pragma unroll 2
-  for (int l = m + 2; l <= lmax; ++l, o += stride) {
-    dl += 1.0;
-    const double r = rcp[l - m];
-    const double alpha = ct * fma(2.0, dl, -1.0) * r;
-    const double bp = -(dl + mm1) * r * pl2;   // off the chain: pl2 is known a degree early
-    const double p = fma(alpha, pl1, bp);
-    put(o, p, fma(dl * ct, p, -(dl + md) * pl1) * rst, dl * (dl + 1.0));
-    pl2 = pl1;
-    pl1 = p;
-  }
+  legendre_chain(m, lmax, ct, st, [&](int l, double p, double pl1) {
+    if (pt >= npts) return;
+    const double dl = (double)l, ll1 = dl * (dl + 1.0);
+    double dp = 0.0, ps = 0.0, d2 = 0.0, dts = 0.0;
+    if (!pole) {
+      if (l >= m) {
+        dp = fma(dl * ct, p, -(dl + md) * pl1) * rst;
+        d2 = fma(-ctr, dp, (m2r2 - ll1) * p);
+        ps = p * rst;
+        dts = rst * fma(-ctr, p, dp);
+      }
+    } else {
+      const double sl = (l % 2 == 0) ? 1.0 : isct;          // isct^l
+      const double sl1 = (l % 2 == 0) ? isct : 1.0;         // isct^(l+1)
+      const double q = (double)(l + 2) * (double)(l + 1) * (double)l * (double)(l - 1);
+      if (m == 1) dp = 0.5 * ll1 * sl;
+      if (m == 1 && l >= 1) ps = 0.5 * ll1 * sl1;
+      if (m == 0) d2 = 0.5 * ll1 * sl;
+      if (m == 2) d2 = 0.25 * q * sl;
+      if (m == 2 && l >= 1) dts = 0.125 * q * sl1;
+    }
+    auto put = [&](int kind, double v) {
+      const long long o = kind * plane + (long long)l * npts + pt;
+      tab[o] = v;
+      texp[o] = tc_exponent(v);
+    };
+    put(m, p);
+    put(3 + m, dp);
+    put(8 + m, d2);
+    if (m >= 1) {
+      put(5 + m, ps);
+      put(10 + m, dts);
+    }
+  });
 }
 
-// term of degree l < nwn in sum k without the table value and the spectrum
-__device__ __forceinline__ double cpl_weight(const CplSum& cs, int nwn, int l) {
-  if (l < cs.l0) return 0.0;
-  const int lmax = nwn - 1;
-  // cos^2 taper of this frequency (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
+// cos^2 taper of the degree l of a frequency with degrees 0..lmax
+// (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
+__device__ __forceinline__ double cpl_taper(int lmax, int l) {
   const double tapfrac = 0.2;
   int jt = (int)floor((double)lmax * (1.0 - tapfrac) + 0.5);
   jt = jt < lmax ? jt : lmax;
   jt = jt > 1 ? jt : 1;
-  double tap = 1.0;
-  if (l >= jt) {
-    const double c1 = (double)lmax * tapfrac * 2.0 / PI_F;
-    const double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
-    const double c = cos((double)(float)l / c1 - c2);
-    tap = c * c;
-  }
-  double c = (2.0 * (double)l + 1.0) / (4.0 * PI_F) * tap;
-  if (cs.fac != 0.0) c = c * (cs.fac / (double)(float)(l * (l + 1)));
-  return c;
+  if (l < jt) return 1.0;
+  const double c1 = (double)lmax * tapfrac * 2.0 / PI_F;
+  const double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
+  const double c = cos((double)(float)l / c1 - c2);
+  return c * c;
+}
+
+// w[l] = (2l+1)/4pi and w[lcap + l] = 2/(l(l+1)): a sum's factor is 0, +-2 or
+// +-4 (the second times +-1 or +-2, which is exact)
+__global__ void cpl_degree_table_kernel(int lcap, double* w) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= lcap) return;
+  w[l] = (2.0 * (double)l + 1.0) / (4.0 * PI_F);
+  w[lcap + l] = l > 0 ? 2.0 / (double)(float)(l * (l + 1)) : 0.0;
 }
 
 // A[aoff[kind] + row * lcap + l], row = 2 (slot nsk[kind] + rank) + re/im: the
@@ -245,7 +232,8 @@ __global__ void cpl_coef_kernel(CplDev S, const float* __restrict__ gr, const fl
   const int nwn = S.nwn[S.nf1 + slot - 1];
   double vr = 0.0, vi = 0.0;
   if (l >= cs.l0 && l < nwn) {
-    const double c = cpl_weight(cs, nwn, l);
+    double c = (2.0 * (double)l + 1.0) / (4.0 * PI_F) * cpl_taper(nwn - 1, l);
+    if (cs.fac != 0.0) c = c * (cs.fac / (double)(float)(l * (l + 1)));
     const long long o = (long long)cs.col * S.nkf + S.koff[slot] + l;
     vr = c * (double)gr[o];
     vi = c * (double)gi[o];
@@ -259,6 +247,7 @@ __global__ void cpl_coef_kernel(CplDev S, const float* __restrict__ gr, const fl
 // the same rows for the tensor-core products (tc_slices.cuh)
 struct CplRows {
   CplDev S;
+  const double* wtab;   // cpl_degree_table_kernel's
   __device__ const CplSum& sum(int k) const { return S.istyp == 1 ? c_cpl[k] : c_cplf[k]; }
   __device__ int nf() const { return S.nf2 - S.nf1 + 1; }
   __device__ int nsum() const { return S.nsum; }
@@ -267,7 +256,12 @@ struct CplRows {
   __device__ int rank(int k) const { return S.rank[k]; }
   __device__ int nsk(int kind) const { return S.nsk[kind]; }
   __device__ long long index(int slot, int k) const { return (long long)sum(k).col * S.nkf + S.koff[slot]; }
-  __device__ double weight(int slot, int k, int l) const { return cpl_weight(sum(k), nwn(slot), l); }
+  __device__ double weight(int slot, int k, int l) const {
+    const CplSum& cs = sum(k);
+    if (l < cs.l0) return 0.0;
+    const double c = wtab[l] * cpl_taper(nwn(slot) - 1, l);
+    return cs.fac == 0.0 ? c : c * (0.5 * cs.fac * wtab[S.lcap + l]);
+  }
 };
 
 // FP64 tiled product C[kind][row][pt] = sum_l A[kind][row][l] * T[kind][l][pt]:
@@ -575,7 +569,10 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   const size_t b_x = align256((size_t)npts * 6 * p->nf2 * sizeof(double2));
   const size_t b_in = align256((size_t)nf * sizeof(int)) + align256((size_t)p->nf2 * sizeof(int)) +
                       3 * align256((size_t)npts * 3 * sizeof(double)) + align256(evf.size() * sizeof(double2)) +
-                      align256((size_t)p->nf2 * 7 * sizeof(double2));
+                      align256((size_t)p->nf2 * 7 * sizeof(double2)) +
+                      (fast ? align256((size_t)2 * lcap * sizeof(double)) +
+                                  align256((size_t)npts * CPL_NKIND * lcap * sizeof(short))
+                            : 0);
   char* ws = (char*)gem_ctx_aux(ctx, 12, b_tab + b_a + b_hd + b_x + b_in);
   if (!ws) return GEM_ERROR;
   double* tab = (double*)ws;
@@ -591,6 +588,8 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   double* d_nrm = (double*)take((size_t)npts * 3 * sizeof(double));
   double2* d_evf = (double2*)take(evf.size() * sizeof(double2));
   double2* d_zel = (double2*)take((size_t)p->nf2 * 7 * sizeof(double2));
+  double* wtab = fast ? (double*)take((size_t)2 * lcap * sizeof(double)) : nullptr;
+  short* texp = fast ? (short*)take((size_t)npts * CPL_NKIND * lcap * sizeof(short)) : nullptr;
   if (cudaMemcpyAsync(d_koff, koff.data(), (size_t)nf * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_nwn, nwn, (size_t)p->nf2 * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_delta, delta, (size_t)npts * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -607,14 +606,16 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   S.istyp = p->istyp; S.nsum = nsum;
   for (int i = 0; i < (p->istyp == 1 ? 6 : 3); ++i) S.mt[i] = mt[i];
   S.nwn = d_nwn; S.koff = d_koff; S.delta = d_delta; S.xi = d_xi; S.nrm = d_nrm; S.evf = d_evf; S.zel = d_zel;
-  const size_t rcp_bytes = (size_t)p->nwnmax * sizeof(double);
-  if (gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST && rcp_bytes <= 200 * 1024) {
+  if (fast && legendre_chain_supported(p->nwnmax - 1)) {
+    const size_t rcp_bytes = legendre_chain_bytes(p->nwnmax - 1);
     cudaFuncSetAttribute(cpl_legendre_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rcp_bytes);
-    cpl_legendre_fast_kernel<<<(npts * 3 + CPL_LF_THREADS - 1) / CPL_LF_THREADS, CPL_LF_THREADS, rcp_bytes, st>>>(
-        npts, p->nwnmax - 1, lcap, d_delta, tab);
+    cpl_legendre_fast_kernel<<<dim3((npts + 31) / 32, 3), LC_THREADS, rcp_bytes, st>>>(npts, p->nwnmax - 1, lcap,
+                                                                                       d_delta, tab, texp);
   } else {
     cpl_legendre_kernel<<<(npts * 3 + 127) / 128, 128, 0, st>>>(npts, p->nwnmax - 1, lcap, d_delta, tab);
+    if (fast) tc_exponents_launch(tab, (long long)npts * CPL_NKIND * lcap, texp, st);
   }
+  if (fast) cpl_degree_table_kernel<<<(lcap + 255) / 256, 256, 0, st>>>(lcap, wtab);
   const long long ncoef = (long long)nf * nsum * lcap;
   if (!fast) cpl_coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, A);
   int maxnsk = 0;
@@ -635,9 +636,9 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
     void* tws = gem_ctx_aux(ctx, 14, wsb);
     if (!tws) return GEM_ERROR;
     const TcCoefs rows = [&](const TcCoefSink& K, cudaStream_t s) {
-      return coef_rows_launch(CplRows{S}, nf * nsum, d_gr, d_gi, K, s);
+      return coef_rows_launch(CplRows{S, wtab}, nf * nsum, d_gr, d_gi, K, s);
     };
-    if (const char* why = sums_tc_run(TP, nwn, mtot, tab, rows, C, tws, wsb, gem_ctx_tc_wait_ns(ctx), st))
+    if (const char* why = sums_tc_run(TP, nwn, mtot, tab, texp, rows, C, tws, wsb, gem_ctx_tc_wait_ns(ctx), st))
       return gem_set_error(ctx, why);
   } else {
     cpl_gemm_kernel<<<ggrid, 256, 0, st>>>(S, A, tab, C);

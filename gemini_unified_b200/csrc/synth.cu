@@ -97,26 +97,27 @@ __global__ void legendre_kernel(int nsta, int lmax, int lcap, const double* __re
 //  runs over the sums of that kind (harmonicDegreeSums.f90:238-351,356-369).
 //  A layout: A[kind][row][lcap]; rowoff[kind], nsk[kind] describe the rows.
 // ---------------------------------------------------------------------------
-// coefficient of degree l < nwn in sum k without the spectrum
-__device__ __forceinline__ double degree_weight(int t, int k, int nwn, int l) {
-  if (l < c_sum_l0[t][k]) return 0.0;
-  const int lmaxf = nwn - 1;
-  // cos^2 taper of this frequency (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
+// cos^2 taper of the degree l of a frequency with degrees 0..lmaxf
+// (harmonicDegreeSums.f90:356-369), TAPFRAC = 0.2
+__device__ __forceinline__ double degree_taper(int lmaxf, int l) {
   const double tapfrac = 0.2;
   int jt = (int)floor((double)lmaxf * (1.0 - tapfrac) + 0.5);
   jt = jt < lmaxf ? jt : lmaxf;
   jt = jt > 1 ? jt : 1;
-  double tap = 1.0;
-  if (l >= jt) {
-    double c1 = (double)lmaxf * tapfrac * 2.0 / PI_F;
-    double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
-    double c = cos((double)(float)l / c1 - c2);
-    tap = c * c;
-  }
-  double w = 1.0;
-  double fac = c_sum_fac[t][k];
-  if (fac != 0.0) w = fac / (double)(float)(l * (l + 1));
-  return w * (2.0 * (double)l + 1.0) / (4.0 * PI_F) * tap;
+  if (l < jt) return 1.0;
+  double c1 = (double)lmaxf * tapfrac * 2.0 / PI_F;
+  double c2 = (1.0 - tapfrac) / tapfrac * 0.5 * PI_F;
+  double c = cos((double)(float)l / c1 - c2);
+  return c * c;
+}
+
+// w[l] = (2l+1)/4pi and w[lcap + l] = 2/(l(l+1)) (2l+1)/4pi: a sum's factor is 0
+// (the first) or +-2 or 4 (the second times +-1 or 2, which is exact)
+__global__ void degree_table_kernel(int lcap, double* w) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= lcap) return;
+  w[l] = (2.0 * (double)l + 1.0) / (4.0 * PI_F);
+  w[lcap + l] = l > 0 ? 2.0 / (double)(float)(l * (l + 1)) * (2.0 * (double)l + 1.0) / (4.0 * PI_F) : 0.0;
 }
 
 __global__ void coef_kernel(SynthDev S, const float* __restrict__ gr, const float* __restrict__ gi, double* A) {
@@ -135,7 +136,10 @@ __global__ void coef_kernel(SynthDev S, const float* __restrict__ gr, const floa
   double vr = 0.0, vi = 0.0;
   if (l < nwn && l >= c_sum_l0[t][k]) {
     const long long o = (long long)S.col_off[c_sum_col[t][k]] * S.nkf + S.koff[slot] + l;
-    const double sc = degree_weight(t, k, nwn, l);
+    double w = 1.0;
+    double fac = c_sum_fac[t][k];
+    if (fac != 0.0) w = fac / (double)(float)(l * (l + 1));
+    const double sc = w * (2.0 * (double)l + 1.0) / (4.0 * PI_F) * degree_taper(nwn - 1, l);
     vr = sc * (double)gr[o];
     vi = sc * (double)gi[o];
   }
@@ -184,7 +188,7 @@ __device__ __forceinline__ WnGeom wn_geom(double xx, double dwn) {
   return g;
 }
 // tab[(kind * lcap + j-1) * nsta + sta], j = 1..lcap (1-based wavenumber index)
-__global__ void bessel_tab_kernel(SynthDev S, const double* __restrict__ theta, double* tab) {
+__global__ void bessel_tab_kernel(SynthDev S, const double* __restrict__ theta, double* tab, short* texp) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)S.lcap * S.nsta) return;
   const int sta = (int)(idx % S.nsta);
@@ -200,7 +204,9 @@ __global__ void bessel_tab_kernel(SynthDev S, const double* __restrict__ theta, 
   if (w != 0.0) { const double a = wn * g.x; b0 = j0(a); b1 = j1(a); b2 = -b0 + 2.0 / a * b1; }
   for (int kind = 0; kind < 8; ++kind) {
     const double v = w != 0.0 ? wn_kernel(kind, wn, b0, b1, b2, S.rearth, g.x) * w * scale : 0.0;
-    tab[((long long)kind * S.lcap + (j - 1)) * S.nsta + sta] = v;
+    const long long o = ((long long)kind * S.lcap + (j - 1)) * S.nsta + sta;
+    tab[o] = v;
+    if (texp) texp[o] = tc_exponent(v);
   }
 }
 
@@ -244,6 +250,7 @@ __global__ void bessel_coef_kernel(SynthDev S, const float* __restrict__ gr, con
 // coefficient rows of the tensor-core products (tc_slices.cuh): degree sums and wavenumber integrals
 struct SynthRows {
   SynthDev S;
+  const double* wtab;   // degree_table_kernel's
   __device__ int nf() const { return S.nf2 - S.nf1 + 1; }
   __device__ int nsum() const { return S.nsum; }
   __device__ int nwn(int slot) const { return S.nwn[S.nf1 + slot - 1]; }
@@ -254,7 +261,11 @@ struct SynthRows {
     return (long long)S.col_off[c_sum_col[S.istyp][k]] * S.nkf + S.koff[slot];
   }
   __device__ double weight(int slot, int k, int l) const {
-    if (S.global_) return degree_weight(S.istyp, k, nwn(slot), l);
+    if (S.global_) {
+      if (l < c_sum_l0[S.istyp][k]) return 0.0;
+      const double fac = c_sum_fac[S.istyp][k];
+      return (fac == 0.0 ? wtab[l] : 0.5 * fac * wtab[S.lcap + l]) * degree_taper(nwn(slot) - 1, l);
+    }
     return wn_taper(nwn(slot), S.dwn, l + 1) * c_wn_sign[S.istyp][k];
   }
 };
@@ -738,20 +749,22 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   const bool fast_fft = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST && ifft_fast_supported(ns);
   const bool o_tred = o && o->tred, o_ns = o && o->nsamp_true, o_sf = o && o->stafilter;
   const bool fast = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST;   // the tensor-core sums store no coefficient rows
-  const size_t sizes[18] = {(size_t)8 * S.lcap * nsta * sizeof(double), fast ? 0 : (size_t)ao * sizeof(double),
+  const size_t sizes[20] = {(size_t)8 * S.lcap * nsta * sizeof(double), fast ? 0 : (size_t)ao * sizeof(double),
                             (size_t)co * sizeof(double), (size_t)ntr * S.ldx * sizeof(double2),
                             evf.size() * sizeof(double2), tw.size() * sizeof(double2), fac.size() * sizeof(double),
                             (size_t)p->nf2 * sizeof(int), (size_t)nf * sizeof(int), nsta * sizeof(double),
                             nsta * sizeof(double), nsta * sizeof(double), (size_t)nmt * nfo * sizeof(double),
                             fast_fft ? ifft_fast_twiddle_bytes(ns) : 0,
                             o_tred ? nsta * sizeof(double) : 0, o_ns ? nsta * sizeof(int) : 0,
-                            o_sf ? (size_t)nsta * 3 * p->nf2 * sizeof(double2) : 0, (size_t)nstf * sizeof(float)};
+                            o_sf ? (size_t)nsta * 3 * p->nf2 * sizeof(double2) : 0, (size_t)nstf * sizeof(float),
+                            fast ? (size_t)8 * S.lcap * nsta * sizeof(short) : 0,
+                            fast ? (size_t)2 * S.lcap * sizeof(double) : 0};
   size_t total = 0;
   for (size_t z : sizes) total += (z + 255) / 256 * 256;
   char* pool = (char*)gem_ctx_aux(ctx, 4, total);
   if (!pool) return GEM_ERROR;
-  void* parts[18];
-  for (int i = 0; i < 18; ++i) { parts[i] = sizes[i] ? pool : nullptr; pool += (sizes[i] + 255) / 256 * 256; }
+  void* parts[20];
+  for (int i = 0; i < 20; ++i) { parts[i] = sizes[i] ? pool : nullptr; pool += (sizes[i] + 255) / 256 * 256; }
   b.tab = (double*)parts[0]; b.A = (double*)parts[1]; b.C = (double*)parts[2]; b.X = (double2*)parts[3];
   b.evf = (double2*)parts[4]; b.tw = (double2*)parts[5]; b.fac = (double*)parts[6]; b.nwn = (int*)parts[7];
   b.koff = (int*)parts[8]; b.theta = (double*)parts[9]; b.phi = (double*)parts[10]; b.propdir = (double*)parts[11];
@@ -765,6 +778,8 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   cudaMemcpyAsync(b.phi, phi, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.propdir, propdir, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.mt, mt, (size_t)nmt * nfo * sizeof(double), cudaMemcpyHostToDevice, st);
+  short* texp = (short*)parts[18];
+  double* wtab = (double*)parts[19];
   S.nwn = b.nwn; S.koff = b.koff;
   S.tred_sta = o_tred ? (const double*)parts[14] : nullptr;
   S.stafil = o_sf ? (const double2*)parts[16] : nullptr;
@@ -780,14 +795,17 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   nvtxRangePushA("gem_synth: sums, spectra, inverse FFT");   // profiler range (no cost without a tool)
   long long ncoef = (long long)nf * S.nsum * S.lcap;
   if (p->global_ == 1) {
-    if (gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST && legendre_fast_supported(S.lmax))
-      legendre_fast_launch(nsta, S.lmax, S.lcap, b.theta, b.tab, st);
-    else
+    if (fast && legendre_fast_supported(S.lmax)) {
+      legendre_fast_launch(nsta, S.lmax, S.lcap, b.theta, b.tab, texp, st);
+    } else {
       legendre_kernel<<<(nsta * 3 + 127) / 128, 128, 0, st>>>(nsta, S.lmax, S.lcap, b.theta, b.tab);
+      if (fast) tc_exponents_launch(b.tab, (long long)8 * S.lcap * nsta, texp, st);
+    }
+    if (fast) degree_table_kernel<<<(S.lcap + 255) / 256, 256, 0, st>>>(S.lcap, wtab);
     if (!fast) coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, b.A);
   } else {
     const long long ntab = (long long)S.lcap * nsta;
-    bessel_tab_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, st>>>(S, b.theta, b.tab);
+    bessel_tab_kernel<<<(unsigned)((ntab + 255) / 256), 256, 0, st>>>(S, b.theta, b.tab, fast ? texp : nullptr);
     if (!fast) bessel_coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, b.A);
   }
   if (gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST) {
@@ -797,9 +815,9 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
     const size_t wsb = sums_tc_workspace(TP, mtot, nullptr);
     void* ws = gem_ctx_aux(ctx, 3, wsb);
     const TcCoefs rows = [&](const TcCoefSink& K, cudaStream_t s) {
-      return coef_rows_launch(SynthRows{S}, nf * S.nsum, d_gr, d_gi, K, s);
+      return coef_rows_launch(SynthRows{S, wtab}, nf * S.nsum, d_gr, d_gi, K, s);
     };
-    const char* why = ws ? sums_tc_run(TP, nwn, mtot, b.tab, rows, b.C, ws, wsb, gem_ctx_tc_wait_ns(ctx), st) : "";
+    const char* why = ws ? sums_tc_run(TP, nwn, mtot, b.tab, texp, rows, b.C, ws, wsb, gem_ctx_tc_wait_ns(ctx), st) : "";
     if (why) {
       nvtxRangePop();
       cudaEventDestroy(e0); cudaEventDestroy(e1);

@@ -63,7 +63,8 @@ inline bool ifft_fast_supported(int ns) { return ns >= 512 && ns <= IFFT_MAX_NS;
 // fast-form Legendre tables (legendre_fast.cu): the tables of legendre_kernel with
 // the recurrence's division replaced by a reciprocal table; lmax up to 25,599
 bool legendre_fast_supported(int lmax);
-cudaError_t legendre_fast_launch(int nsta, int lmax, int lcap, const double* theta, double* tab, cudaStream_t st);
+cudaError_t legendre_fast_launch(int nsta, int lmax, int lcap, const double* theta, double* tab, short* texp,
+                                 cudaStream_t st);
 
 // event filter of the synthetics (Butterworth band-pass at f - i sigma/2pi), h[jf] for jf = nf1..nf2
 void event_filter_host(const gem_synth_params* p, std::vector<double2>& h);
@@ -94,11 +95,17 @@ struct TcCoefSink {
   double* rscale;
 };
 using TcCoefs = std::function<cudaError_t(const TcCoefSink&, cudaStream_t)>;
+// texp[(kind * lcap + l) * ncol + col]: binary exponents of the table's entries,
+// which the kernels that fill a table write beside it (the field of the double:
+// |T| < 2^(e - 1022); 0 for zero and subnormal entries, 2047 for inf and NaN)
+__device__ __forceinline__ short tc_exponent(double x) { return (short)((__double2hiint(x) >> 20) & 0x7ff); }
+cudaError_t tc_exponents_launch(const double* tab, long long n, short* texp, cudaStream_t st);   // of a table without them
 TcProblem tc_problem_of(const SynthDev& S);   // the synthetics' 8 Legendre / Bessel kinds
 // workspace size and run; nwn: host copy of the wavenumber counts per frequency
 // (1-based frequency index); wait_ns: limit of each pipeline wait (0: 1 s)
 size_t sums_tc_workspace(const TcProblem& P, long long mtot, int* Kp_out);
-const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const TcCoefs& coefs,
+const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const short* texp,
+                        const TcCoefs& coefs,
                         double* C, void* ws, size_t ws_bytes, unsigned long long wait_ns, cudaStream_t st);
 
 }  // namespace gem
