@@ -10,12 +10,28 @@
 // Real output from a half-length complex transform: with H = N/2,
 //   Z_k = (X_k + conj X_{H-k}) + i w^k (X_k - conj X_{H-k}),  w = e^{2 pi i/N},
 //   z_n = sum_k Z_k e^{2 pi i kn/H},  x_{2n} = Re z_n,  x_{2n+1} = Im z_n,
-// where X_{H-k} stands for X_{k+H} of the Hermitian spectrum.  The H-point
-// transform is a Stockham autosort of radix-16 passes (one of radix 2, 4 or 8
-// when log2 H is not a multiple of 4): each of the H/16 threads keeps 16
-// points in registers per pass and the passes exchange through shared memory.
-// One CTA per trace.
+// where X_{H-k} stands for X_{k+H} of the Hermitian spectrum.  One CTA of T =
+// H/16 threads per trace; each thread keeps 16 points in registers per pass and
+// the passes exchange through shared memory.  With k = T d2 + RB d1 + d0 and n =
+// o2 + 16 o1 + 256 o0 (RB = H/256),
+//   z_n = sum_d0 e^{2 pi i d0 (o2 + 16 o1)/H} e^{2 pi i d0 o0/RB}
+//         sum_d1 e^{2 pi i d1 o2/256} e^{2 pi i d1 o1/16} sum_d2 e^{2 pi i d2 o2/16} Z_k:
+// radix 16, 16 and RB, each pass writing where it read, so that one barrier
+// separates two passes (an autosorting transform needs two) and the last one
+// leaves consecutive threads consecutive samples.
+//
+// Bound: the FP64 pipe (580 instructions per thread and trace of 4096 points, 2 clocks each) and
+// the L1 pipe (340 wavefronts per warp), each busy half of the time with the 16 warps per SM that
+// the points' registers leave.  So the butterflies are those of radix 2 in FMA form, p = a + w b
+// and 2 a - p, 6 instructions with the twiddle factor included; a radix-16 pass with its 15
+// twiddles needs 208 that way and 4 loads (268 and 3 in a 4 x 4 split).  12,001 traces of 8192
+// samples from 410 bins: 0.254 -> 0.212 ms (three CTAs per SM of 80 registers spill: 0.240; one
+// trace per CTA, nothing fetched ahead: 0.221); 72,000: 1.42 -> 1.20 ms (2.4 GB written).  9009 traces
+// of 2048 samples, band above 1/16, one trace per CTA, 128 registers and loads without a branch
+// around them: 0.129 -> 0.079 ms (many traces per CTA: 0.177).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "synth.h"
 
@@ -26,136 +42,126 @@ namespace {
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 times_i(double2 a) { return make_double2(-a.y, a.x); }
 
-// shared-memory position of point p: one pad element per 16 keeps the strided
-// accesses of the passes off a single bank group
-__device__ __forceinline__ int pad(int p) { return p + (p >> 4); }
+constexpr double C16 = 0.92387953251128675613, S16 = 0.38268343236508977173, R8 = 0.70710678118654752440;
 
-// 4-point inverse DFT in place: out_k = sum_n a_n i^{nk}
-__device__ __forceinline__ void dft4(double2& a0, double2& a1, double2& a2, double2& a3) {
-  const double2 p = cadd(a0, a2), m = csub(a0, a2), q = cadd(a1, a3), d = times_i(csub(a1, a3));
-  a0 = cadd(p, q);
-  a2 = csub(p, q);
-  a1 = cadd(m, d);
-  a3 = csub(m, d);
+// (a, b) <- (a + w b, a - w b)
+__device__ __forceinline__ void bf(double2& a, double2& b, double2 w) {
+  const double2 p = make_double2(fma(-w.y, b.y, fma(w.x, b.x, a.x)), fma(w.y, b.x, fma(w.x, b.y, a.y)));
+  b = make_double2(fma(2.0, a.x, -p.x), fma(2.0, a.y, -p.y));
+  a = p;
 }
-
-// e^{2 pi i n/16}, n = 0..9 (the exponents r0*k0 of the 4 x 4 split)
-__device__ __forceinline__ double2 w16(int n) {
-  constexpr double C1 = 0.92387953251128675613, S1 = 0.38268343236508977173, H2 = 0.70710678118654752440;
-  switch (n) {
-    case 0: return make_double2(1.0, 0.0);
-    case 1: return make_double2(C1, S1);
-    case 2: return make_double2(H2, H2);
-    case 3: return make_double2(S1, C1);
-    case 4: return make_double2(0.0, 1.0);
-    case 6: return make_double2(-H2, H2);
-    default: return make_double2(-C1, -S1);   // n = 9
-  }
+__device__ __forceinline__ void bf_i(double2& a, double2& b, double2 w) {   // i w for w
+  b = times_i(b);
+  bf(a, b, w);
 }
-
-// 16-point inverse DFT in place (4 x 4: rows r = 4 r1 + r0, outputs k = k0 + 4 k1)
-__device__ __forceinline__ void dft16(double2* v) {
-#pragma unroll
-  for (int r0 = 0; r0 < 4; ++r0) dft4(v[r0], v[4 + r0], v[8 + r0], v[12 + r0]);
-  // v[r0 + 4 k0] now holds Y[r0][k0]; twiddle by w16^(r0 k0)
-#pragma unroll
-  for (int r0 = 1; r0 < 4; ++r0)
-#pragma unroll
-    for (int k0 = 1; k0 < 4; ++k0) v[r0 + 4 * k0] = cmul(v[r0 + 4 * k0], w16(r0 * k0));
-  double2 o[16];
-#pragma unroll
-  for (int k0 = 0; k0 < 4; ++k0) {
-    double2 a0 = v[0 + 4 * k0], a1 = v[1 + 4 * k0], a2 = v[2 + 4 * k0], a3 = v[3 + 4 * k0];
-    dft4(a0, a1, a2, a3);
-    o[k0] = a0; o[k0 + 4] = a1; o[k0 + 8] = a2; o[k0 + 12] = a3;
-  }
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = o[k];
+__device__ __forceinline__ void bf(double2& a, double2& b) {   // w = 1
+  const double2 p = make_double2(a.x + b.x, a.y + b.y);
+  b = make_double2(a.x - b.x, a.y - b.y);
+  a = p;
 }
-
-__device__ __forceinline__ void dft2(double2* v) {
-  const double2 a = v[0], b = v[1];
-  v[0] = cadd(a, b);
-  v[1] = csub(a, b);
+__device__ __forceinline__ void bf_i(double2& a, double2& b) {   // w = i
+  b = times_i(b);
+  bf(a, b);
 }
+__device__ __forceinline__ double2 times_w8(double2 w) { return make_double2((w.x - w.y) * R8, (w.x + w.y) * R8); }
+__device__ __forceinline__ double2 times_w16(double2 w) { return cmul(w, make_double2(C16, S16)); }
 
-__device__ __forceinline__ void dft8(double2* v) {
-  // even/odd split: X_k = E_k + w8^k O_k, X_{k+4} = E_k - w8^k O_k
-  double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-  dft4(e0, e1, e2, e3);
-  dft4(o0, o1, o2, o3);
-  constexpr double H2 = 0.70710678118654752440;
-  o1 = cmul(o1, make_double2(H2, H2));
-  o2 = times_i(o2);
-  o3 = cmul(o3, make_double2(-H2, H2));
-  v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
-  v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
-  v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
-  v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
-}
-
+// out_o = sum_{r < R} w^r v_r e^{2 pi i r o/R}, left in v[rev<R>(o)].  The pairs (r, r +
+// R/2) meet with w^{R/2}; the sums go on with w for the even o, the differences with w
+// e^{2 pi i/R} for the odd.  w1, w2, w4, w8: powers of w.
 template <int R>
-__device__ __forceinline__ void dftR(double2* v) {
-  if constexpr (R == 16) dft16(v);
-  else if constexpr (R == 8) dft8(v);
-  else if constexpr (R == 4) dft4(v[0], v[1], v[2], v[3]);
-  else dft2(v);
+__device__ __forceinline__ constexpr int rev(int o) {
+  int q = 0;
+  for (int b = 1; b < R; b <<= 1) q = 2 * q + ((o & b) != 0);
+  return q;
 }
+__device__ __forceinline__ void dft_tw(double2 (&v)[16], double2 w1, double2 w2, double2 w4, double2 w8) {
+#pragma unroll
+  for (int r = 0; r < 8; ++r) bf(v[r], v[r + 8], w8);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    bf(v[r], v[r + 4], w4);
+    bf_i(v[r + 8], v[r + 12], w4);
+  }
+  const double2 w2b = times_w8(w2);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    bf(v[r], v[r + 2], w2);
+    bf_i(v[r + 4], v[r + 6], w2);
+    bf(v[r + 8], v[r + 10], w2b);
+    bf_i(v[r + 12], v[r + 14], w2b);
+  }
+  const double2 wb = times_w8(w1), wc = times_w16(w1), wd = times_w16(wb);
+  bf(v[0], v[1], w1);
+  bf_i(v[2], v[3], w1);
+  bf(v[4], v[5], wb);
+  bf_i(v[6], v[7], wb);
+  bf(v[8], v[9], wc);
+  bf_i(v[10], v[11], wc);
+  bf(v[12], v[13], wd);
+  bf_i(v[14], v[15], wd);
+}
+__device__ __forceinline__ void dft_tw(double2 (&v)[8], double2 w1, double2 w2, double2 w4, double2) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) bf(v[r], v[r + 4], w4);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    bf(v[r], v[r + 2], w2);
+    bf_i(v[r + 4], v[r + 6], w2);
+  }
+  const double2 wb = times_w8(w1);
+  bf(v[0], v[1], w1);
+  bf_i(v[2], v[3], w1);
+  bf(v[4], v[5], wb);
+  bf_i(v[6], v[7], wb);
+}
+__device__ __forceinline__ void dft_tw(double2 (&v)[4], double2 w1, double2 w2, double2, double2) {
+  bf(v[0], v[2], w2);
+  bf(v[1], v[3], w2);
+  bf(v[0], v[1], w1);
+  bf_i(v[2], v[3], w1);
+}
+__device__ __forceinline__ void dft_tw(double2 (&v)[2], double2 w1, double2, double2, double2) { bf(v[0], v[1], w1); }
 
-// One Stockham pass of radix R over the H points in shared memory (NS: length of
-// the sub-transforms already done).  Each of the H/16 threads runs 16/R
-// butterflies.  The last pass hands its 16 results (point indices idx) back.
-// twp: the pass's twiddles twp[(r - 1) NS + k] = e^{2 pi i r k / (NS R)}, laid out
-// so that the threads of a warp (consecutive k) read consecutive entries.
-template <int H, int R, int NS, bool LAST>
-__device__ __forceinline__ void stockham_pass(double2* buf, double2* v, int* idx, const double2* __restrict__ twp) {
-  constexpr int T = H / 16, NB = 16 / R;
-  const int tid = threadIdx.x;
+// the first pass, w = 1.  BAND: only v0, v1, v14 and v15 are not zero, whose first
+// two levels are copies
+template <bool BAND>
+__device__ __forceinline__ void dft16(double2 (&v)[16]) {
+  if constexpr (BAND) {
+    auto minus = [](double2 a) { return make_double2(-a.x, -a.y); };
+    const double2 a = v[14], b = v[15];
+    v[2] = a; v[3] = b;
+    v[4] = v[0]; v[5] = v[1]; v[6] = minus(a); v[7] = minus(b);
+    v[12] = v[8] = v[0]; v[13] = v[9] = v[1];
+    v[14] = times_i(a); v[15] = times_i(b);
+    v[10] = minus(v[14]); v[11] = minus(v[15]);
+  } else {
 #pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    const int j = tid + b * T;
+    for (int r = 0; r < 8; ++r) bf(v[r], v[r + 8]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[b * R + r] = buf[pad(j + r * (H / R))];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    const int j = tid + b * T;
-    const int k = j % NS;
-    if (NS > 1) {
-      // w^r, r = 1..R-1, of w = e^{2 pi i k/(NS R)}: R = 16 loads w, w^4 and w^8 and forms the
-      // others by products (a few ulps; 3 loads in place of 15, the L1 pipe bounds this kernel)
-      if constexpr (R == 16) {
-        const double2 w1 = twp[k], w4 = twp[3 * NS + k], w8 = twp[7 * NS + k];
-        const double2 w2 = cmul(w1, w1), w3 = cmul(w2, w1);
-        double2* u = v + b * R;
-        u[1] = cmul(u[1], w1); u[2] = cmul(u[2], w2); u[3] = cmul(u[3], w3);
-#pragma unroll
-        for (int q = 1; q < 4; ++q) {   // rows 4q .. 4q + 3 with base w^{4q}
-          const double2 wb = q == 1 ? w4 : (q == 2 ? w8 : cmul(w8, w4));
-          u[4 * q] = cmul(u[4 * q], wb);
-          u[4 * q + 1] = cmul(u[4 * q + 1], cmul(wb, w1));
-          u[4 * q + 2] = cmul(u[4 * q + 2], cmul(wb, w2));
-          u[4 * q + 3] = cmul(u[4 * q + 3], cmul(wb, w3));
-        }
-      } else {
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[b * R + r] = cmul(v[b * R + r], twp[(r - 1) * NS + k]);
-      }
-    }
-    dftR<R>(v + b * R);
-    const int d = (j / NS) * NS * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (LAST) idx[b * R + r] = d + r * NS;
-      else buf[pad(d + r * NS)] = v[b * R + r];
+    for (int r = 0; r < 4; ++r) {
+      bf(v[r], v[r + 4]);
+      bf_i(v[r + 8], v[r + 12]);
     }
   }
-  if (!LAST) __syncthreads();
+  const double2 w8 = make_double2(R8, R8), w16 = make_double2(C16, S16), w163 = make_double2(S16, C16);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    bf(v[r], v[r + 2]);
+    bf_i(v[r + 4], v[r + 6]);
+    bf(v[r + 8], v[r + 10], w8);
+    bf_i(v[r + 12], v[r + 14], w8);
+  }
+  bf(v[0], v[1]);
+  bf_i(v[2], v[3]);
+  bf(v[4], v[5], w8);
+  bf_i(v[6], v[7], w8);
+  bf(v[8], v[9], w16);
+  bf_i(v[10], v[11], w16);
+  bf(v[12], v[13], w163);
+  bf_i(v[14], v[15], w163);
 }
 
 }  // namespace
@@ -164,7 +170,10 @@ __device__ __forceinline__ void stockham_pass(double2* buf, double2* v, int* idx
 // pass (NS 16, R 16) and tw + N + IFFT_TWB for the last pass (NS 256, R H/256),
 // entry (r - 1) NS + k = e^{2 pi i r k / (NS R)}.  Both angles are the same double
 // as the m = r k N / (NS R) of the full table, so the entries equal tw[m].
-__global__ void ifft_fast_twiddles(int N, double2* tw) {
+// fac[i] = e^{arg i}, arg = sigma times the sampling interval: the reference's running product
+// (frequencyTime.f90:105-110) is one dependent chain of nsamp multiplications, 46 us of one thread
+// for 8192 samples, and departs from the exponential by the rounding of its base times i.
+__global__ void ifft_fast_twiddles(int N, double2* tw, int nsamp, double arg, double* fac) {
   const int H = N / 2, RB = H / 256;
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < N + IFFT_TW_EXTRA; m += blockDim.x * gridDim.x) {
     long long num = 0, den = 1;
@@ -181,98 +190,168 @@ __global__ void ifft_fast_twiddles(int N, double2* tw) {
     sincospi(2.0 * (double)num / (double)den, &s, &c);
     tw[m] = make_double2(c, s);
   }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nsamp; i += blockDim.x * gridDim.x) fac[i] = exp(arg * (double)i);
 }
 
-template <int H>
-__global__ void __launch_bounds__(H / 16, H == 4096 ? 3 : 1) ifft_fast_kernel(SynthDev S, const double2* __restrict__ X,
+// keeps what follows from a loop-invariant value inside the loop: hoisted twiddle products
+// would take the registers of the 16 points
+__device__ __forceinline__ void in_loop(double2& a) { asm volatile("" : "+d"(a.x), "+d"(a.y)); }
+__device__ __forceinline__ double2 load_in_loop(const double2* p) {
+  double2 a;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(a.x), "=d"(a.y) : "l"(p));
+  return a;
+}
+
+// BAND: the band's bins lie below H/8, so that Z_k is not zero for k < 2 T and k > H - 2 T only.
+// H = 4096: a CTA runs over the traces blockIdx.x, + gridDim.x, ..., and with BAND loads the next
+// trace's bins while the current one is transformed; else one trace per CTA.  128 registers.
+template <int H, bool BAND>
+__global__ void __launch_bounds__(H / 16, H == 256 ? 16 : 8192 / H) ifft_fast_kernel(SynthDev S, long long ntr,
+                                                          const double2* __restrict__ X,
                                                           const double2* __restrict__ tw,
                                                           const double* __restrict__ fac, float* traces) {
-  extern __shared__ double2 buf[];
-  constexpr int T = H / 16;
+  constexpr bool MANY = H == 4096;   // more than one trace per CTA
+  extern __shared__ double2 buf[];   // point p = T d2 + RB d1 + d0 at p + d2: the last pass reads along d2
+  constexpr int T = H / 16, RB = H / 256;
   const int N = 2 * H;
   const int tid = threadIdx.x;
-  const long long tr = blockIdx.x;
-  const double2* x = X + tr * S.ldx;
   const int lo = S.nf1 - 1, hi = S.nf2 - 1;   // 0-based bins of the spectrum
-  double2 v[16];
-  int idx[16];
-  // ---- pass 0 (radix 16, NS = 1): Z_k formed on the fly, k = tid + r T.  Z_k is
-  // zero unless k or H - k is a bin of the band, so a block of T consecutive k
-  // outside both ranges skips its loads (a branch uniform over the CTA)
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 in[4];
+  auto fetch = [&](long long tr) {   // bins k and H - k of the blocks r = 0, 1 and 14, 15
+    const double2* x = X + tr * S.ldx;
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
-    const int k = tid + r * T;
-    const int ka = r * T, kb = r * T + T - 1;
-    if (!((ka <= hi && kb >= lo) || (H - kb <= hi && H - ka >= lo))) {
-      v[r] = make_double2(0.0, 0.0);
-      continue;
+    for (int r = 0; r < 2; ++r) {
+      const int k = tid + r * T, kk = (2 - r) * T - tid;
+      in[r] = (k >= lo && k <= hi) ? x[k] : zero;
+      in[r + 2] = (kk >= lo && kk <= hi) ? x[kk] : zero;
     }
-    const double2 a = (k >= lo && k <= hi) ? x[k] : make_double2(0.0, 0.0);
-    const int kk = H - k;
-    double2 b = make_double2(0.0, 0.0);
-    if (k > 0 && kk >= lo && kk <= hi) { b = x[kk]; b.y = -b.y; }
-    const double2 s = cadd(a, b), d = csub(a, b), w = tw[k];
-    // Z = s + i w d
-    v[r] = make_double2(s.x - w.y * d.x - w.x * d.y, s.y + w.x * d.x - w.y * d.y);
-  }
-  dft16(v);
+  };
+  if (BAND && MANY) fetch(blockIdx.x);
+  double2 w0 = tw[tid];
+  double2 wb1 = RB == 16 ? tw[N + IFFT_TWB + tid] : zero;
+  // H = 4096, ndec = 1: the last pass leaves thread tid the samples 2 tid + 512 q (+1), whose factors are
+  // df fac(2 tid) fac(512)^q (+1), formed by products instead of 32 table loads (a few ulps of a double)
+  const bool ratios = H == 4096 && S.ndec == 1 && S.nsamp > 512;
+  const bool pairs = (S.nsamp & 1) == 0 && (reinterpret_cast<size_t>(traces) & 7) == 0;   // 8-byte stores
+  for (long long tr = blockIdx.x; tr < ntr; tr += gridDim.x) {
+    double2 v[16];
+    in_loop(w0);
+    in_loop(wb1);
+    // ---- pass over d2: Z_k formed on the fly, k = tid + r T
+    if constexpr (BAND) {
+      if (!MANY) fetch(tr);
 #pragma unroll
-  for (int r = 0; r < 16; ++r) buf[pad(tid * 16 + r)] = v[r];
-  __syncthreads();
-  // ---- remaining passes
-  if constexpr (H == 256) {
-    stockham_pass<H, 16, 16, true>(buf, v, idx, tw + N + IFFT_TWA);
-  } else if constexpr (H == 512) {
-    stockham_pass<H, 16, 16, false>(buf, v, idx, tw + N + IFFT_TWA);
-    stockham_pass<H, 2, 256, true>(buf, v, idx, tw + N + IFFT_TWB);
-  } else if constexpr (H == 1024) {
-    stockham_pass<H, 16, 16, false>(buf, v, idx, tw + N + IFFT_TWA);
-    stockham_pass<H, 4, 256, true>(buf, v, idx, tw + N + IFFT_TWB);
-  } else if constexpr (H == 2048) {
-    stockham_pass<H, 16, 16, false>(buf, v, idx, tw + N + IFFT_TWA);
-    stockham_pass<H, 8, 256, true>(buf, v, idx, tw + N + IFFT_TWB);
-  } else {
-    static_assert(H == 4096, "supported half lengths: 256..4096");
-    stockham_pass<H, 16, 16, false>(buf, v, idx, tw + N + IFFT_TWA);
-    stockham_pass<H, 16, 256, true>(buf, v, idx, tw + N + IFFT_TWB);
-  }
-  // ---- x_{2n} = Re z_n, x_{2n+1} = Im z_n; ts(i) = x(ndec i) df fac(i)
-  float* out = traces + tr * S.nsamp;
-  const int ndec = S.ndec;
-  if constexpr (H == 4096) {
-    // the last pass leaves thread tid the points n = tid + 256 q: samples 2 tid + 512 q (+1), whose factors are
-    // df fac(2 tid) expo^(512 q) (+1), formed by products with fac(512) = expo^512 instead of 32 table loads
-    // (the table is the running product expo^i; the products differ from it by a few ulps of a double)
-    if (ndec == 1 && S.nsamp > 512) {
-      const double2 f01 = *reinterpret_cast<const double2*>(fac + 2 * tid);
-      const double ratio = fac[512];
+      for (int r = 0; r < 2; ++r) {   // e^{2 pi i k/N} = w0 e^{2 pi i r/32}
+        constexpr double C1 = 0.98078528040323044913, S1 = 0.19509032201612826785;
+        const double2 w = r ? cmul(w0, make_double2(C1, S1)) : w0;
+        const double2 u = cmul(w0, r ? make_double2(-C1, S1) : make_double2(-C16, S16));
+        const double2 a = in[r], b = make_double2(in[r + 2].x, -in[r + 2].y);
+        v[r] = make_double2(a.x - w.y * a.x - w.x * a.y, a.y + w.x * a.x - w.y * a.y);
+        v[r + 14] = make_double2(b.x + u.y * b.x + u.x * b.y, b.y - u.x * b.x + u.y * b.y);
+      }
+      if (MANY && tr + gridDim.x < ntr) fetch(tr + gridDim.x);
+    } else {
+      // Z = s + i w d of the bins k and H - k; the loads carry no branch, so that they are in flight together
+      const double2* x = X + tr * S.ldx;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int k = tid + r * T, kk = H - k;
+        const double2 a = (k >= lo && k <= hi) ? x[k] : zero;
+        double2 b = (k > 0 && kk >= lo && kk <= hi) ? x[kk] : zero;
+        b.y = -b.y;
+        const double2 s = make_double2(a.x + b.x, a.y + b.y), d = make_double2(a.x - b.x, a.y - b.y), w = tw[k];
+        v[r] = make_double2(s.x - w.y * d.x - w.x * d.y, s.y + w.x * d.x - w.y * d.y);
+      }
+    }
+    dft16<BAND>(v);
+#pragma unroll
+    for (int o = 0; o < 16; ++o) buf[o * (T + 1) + tid] = v[rev<16>(o)];
+    __syncthreads();
+    // ---- pass over d1 of (o2, d0)
+    {
+      const int o2 = tid / RB;
+      double2* p = buf + o2 * (T + 1) + tid % RB;
+      const double2* t = tw + N + IFFT_TWA + o2;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = p[r * RB];
+      dft_tw(v, load_in_loop(t), load_in_loop(t + 16), load_in_loop(t + 3 * 16), load_in_loop(t + 7 * 16));
+      if constexpr (RB > 1) {
+#pragma unroll
+        for (int o = 0; o < 16; ++o) p[o * RB] = v[rev<16>(o)];
+      }
+      __syncthreads();
+    }
+    // ---- pass over d0 of j = o2 + 16 o1: out_of(q) is then the point n = tid + q T
+    if constexpr (RB > 1) {
+#pragma unroll
+      for (int b = 0; b < 16 / RB; ++b) {
+        const int j = tid + b * T;
+        const double2* p = buf + (j % 16) * (T + 1) + j / 16 * RB;
+        double2 u[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) u[r] = p[r];
+        if constexpr (RB == 16) {
+          { const double2 w4 = load_in_loop(tw + N + IFFT_TWB + 3 * 256 + tid); dft_tw(u, wb1, cmul(wb1, wb1), w4, cmul(w4, w4)); }
+        } else {
+          const double2* t = tw + N + IFFT_TWB + j;
+          const double2 w1 = load_in_loop(t);
+          dft_tw(u, w1, RB > 2 ? load_in_loop(t + 256) : w1, RB > 4 ? load_in_loop(t + 3 * 256) : w1, w1);
+        }
+#pragma unroll
+        for (int o = 0; o < RB; ++o) v[b + o * (16 / RB)] = u[rev<RB>(o)];
+      }
+      if (MANY) __syncthreads();   // the next trace writes the buffer
+    }
+    auto out_of = [&](int q) -> double2 { return RB > 1 ? v[q] : v[rev<16>(q)]; };
+    // ---- x_{2n} = Re z_n, x_{2n+1} = Im z_n; ts(i) = x(ndec i) df fac(i)
+    float* out = traces + tr * S.nsamp;
+    const int ndec = S.ndec;
+    if (ratios) {
+      const double2 f01 = load_in_loop(reinterpret_cast<const double2*>(fac + 2 * tid));
+      double ratio;
+      asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(ratio) : "l"(fac + 512));
       double g0 = S.df * f01.x, g1 = S.df * f01.y;
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
+        const double2 z = out_of(q);
         const int t0 = 2 * tid + 512 * q, t1 = t0 + 1;
-        if (t1 < S.nsamp) *reinterpret_cast<float2*>(out + t0) = make_float2((float)(v[q].x * g0), (float)(v[q].y * g1));
-        else if (t0 < S.nsamp) out[t0] = (float)(v[q].x * g0);
+        const float y0 = (float)(z.x * g0), y1 = (float)(z.y * g1);
+        if (pairs) {
+          if (t1 < S.nsamp) *reinterpret_cast<float2*>(out + t0) = make_float2(y0, y1);
+        } else {
+          if (t0 < S.nsamp) out[t0] = y0;
+          if (t1 < S.nsamp) out[t1] = y1;
+        }
         g0 *= ratio;
         g1 *= ratio;
       }
-      return;
+      continue;
     }
-  }
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int n = idx[q];
-    const int t0 = 2 * n, t1 = 2 * n + 1;
-    if (ndec == 1) {
-      if (t1 < S.nsamp) {
-        const double2 f = *reinterpret_cast<const double2*>(fac + t0);   // t0 even: 16-byte aligned
-        *reinterpret_cast<float2*>(out + t0) = make_float2((float)(v[q].x * S.df * f.x), (float)(v[q].y * S.df * f.y));
-      } else if (t0 < S.nsamp) {
-        out[t0] = (float)(v[q].x * S.df * fac[t0]);
+    for (int q = 0; q < 16; ++q) {
+      const double2 z = out_of(q);
+      const int n = tid + q * T;
+      const int t0 = 2 * n, t1 = 2 * n + 1;
+      if (ndec == 1) {
+        if (t1 < S.nsamp) {
+          const double2 f = *reinterpret_cast<const double2*>(fac + t0);   // t0 even: 16-byte aligned
+          const float y0 = (float)(z.x * S.df * f.x), y1 = (float)(z.y * S.df * f.y);
+          if (pairs) {
+            *reinterpret_cast<float2*>(out + t0) = make_float2(y0, y1);
+          } else {
+            out[t0] = y0;
+            out[t1] = y1;
+          }
+        } else if (t0 < S.nsamp) {
+          out[t0] = (float)(z.x * S.df * fac[t0]);
+        }
+      } else {
+        if (t0 % ndec == 0 && t0 / ndec < S.nsamp) out[t0 / ndec] = (float)(z.x * S.df * fac[t0 / ndec]);
+        if (t1 % ndec == 0 && t1 / ndec < S.nsamp) out[t1 / ndec] = (float)(z.y * S.df * fac[t1 / ndec]);
       }
-    } else {
-      if (t0 % ndec == 0 && t0 / ndec < S.nsamp) out[t0 / ndec] = (float)(v[q].x * S.df * fac[t0 / ndec]);
-      if (t1 % ndec == 0 && t1 / ndec < S.nsamp) out[t1 / ndec] = (float)(v[q].y * S.df * fac[t1 / ndec]);
     }
+    if (!MANY) return;
   }
 }
 
@@ -280,27 +359,34 @@ __global__ void __launch_bounds__(H / 16, H == 4096 ? 3 : 1) ifft_fast_kernel(Sy
 cudaError_t ifft_fast_launch(const SynthDev& S, long long ntr, const double2* X, const double2* tw, const double* fac,
                              float* traces, cudaStream_t st) {
   const int H = S.ns / 2;
-  const size_t smem = (size_t)(H + H / 16) * sizeof(double2);
+  const size_t smem = (size_t)(H + 16) * sizeof(double2);
+  const bool band = S.nf2 - 1 < H / 8;   // the first pass has 4 blocks of 16 that are not zero: 84 of 148 instructions, no partner bins
   auto go = [&](auto kern, int threads) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)   // all of the unified L1 as shared memory: more CTAs of the longest transforms per SM
       e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)ntr, threads, smem, st>>>(S, X, tw, fac, traces);
+    int dev = 0, sms = 0, per = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem)) != cudaSuccess)
+      return e;
+    const long long grid = H == 4096 ? std::min<long long>(ntr, (long long)sms * std::max(per, 1)) : ntr;
+    kern<<<(unsigned)grid, threads, smem, st>>>(S, ntr, X, tw, fac, traces);
     return cudaGetLastError();
   };
   switch (H) {
-    case 256: return go(ifft_fast_kernel<256>, 16);
-    case 512: return go(ifft_fast_kernel<512>, 32);
-    case 1024: return go(ifft_fast_kernel<1024>, 64);
-    case 2048: return go(ifft_fast_kernel<2048>, 128);
-    case 4096: return go(ifft_fast_kernel<4096>, 256);
+    case 256: return band ? go(ifft_fast_kernel<256, true>, 16) : go(ifft_fast_kernel<256, false>, 16);
+    case 512: return band ? go(ifft_fast_kernel<512, true>, 32) : go(ifft_fast_kernel<512, false>, 32);
+    case 1024: return band ? go(ifft_fast_kernel<1024, true>, 64) : go(ifft_fast_kernel<1024, false>, 64);
+    case 2048: return band ? go(ifft_fast_kernel<2048, true>, 128) : go(ifft_fast_kernel<2048, false>, 128);
+    case 4096: return band ? go(ifft_fast_kernel<4096, true>, 256) : go(ifft_fast_kernel<4096, false>, 256);
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t ifft_fast_twiddles_launch(int N, double2* tw, cudaStream_t st) {
-  ifft_fast_twiddles<<<(N + IFFT_TW_EXTRA + 255) / 256, 256, 0, st>>>(N, tw);
+cudaError_t ifft_fast_twiddles_launch(int N, double2* tw, int nsamp, double arg, double* fac, cudaStream_t st) {
+  ifft_fast_twiddles<<<(N + IFFT_TW_EXTRA + 255) / 256, 256, 0, st>>>(N, tw, nsamp, arg, fac);
   return cudaGetLastError();
 }
 

@@ -771,7 +771,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   b.mt = (double*)parts[12]; b.twx = (double2*)parts[13];
   cudaMemcpyAsync(b.evf, evf.data(), evf.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.fac, fac.data(), fac.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+  if (!fast_fft) cudaMemcpyAsync(b.fac, fac.data(), fac.size() * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.nwn, nwn, (size_t)p->nf2 * sizeof(int), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.koff, koff.data(), nf * sizeof(int), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(b.theta, theta, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
@@ -835,7 +835,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   spectra_kernel<<<dim3((unsigned)((nsta + SP_STA - 1) / SP_STA), (unsigned)((nf + SP_SLOT - 1) / SP_SLOT)), SP_THREADS, 0,
                    st>>>(S, b.C, b.evf, b.phi, b.propdir, b.mt, b.X);
   if (fast_fft) {
-    ifft_fast_twiddles_launch(ns, b.twx, st);
+    ifft_fast_twiddles_launch(ns, b.twx, p->nsamp, p->sigma * dts, b.fac, st);
     ifft_fast_launch(S, ntr, b.X, b.twx, b.fac, d_traces, st);
   } else {
     size_t smem = (size_t)ns * sizeof(double2);
@@ -977,13 +977,12 @@ extern "C" int gem_ifft_run_device(gem_ctx* ctx, int nf1, int nf2, double df, do
   SynthDev S{};
   S.nf1 = nf1; S.nf2 = nf2; S.ns = g.ns; S.nslog = g.nslog; S.nsamp = nsamp; S.ndec = g.ndec; S.df = df;
   S.sigma = sigma; S.ldx = ldsp;
-  const double expo = std::exp(sigma * g.dts);
-  ifft_tables_kernel<<<8, 256, 0, st>>>(g.ns, g.nslog, nsamp, expo, tw, fac);
   if (fast) {
     double2* twx = (double2*)(tab + (tbytes + 15) / 16 * 16);
-    ifft_fast_twiddles_launch(g.ns, twx, st);
+    ifft_fast_twiddles_launch(g.ns, twx, nsamp, sigma * g.dts, fac, st);
     ifft_fast_launch(S, ntr, (const double2*)d_sp, twx, fac, d_ts, st);
   } else {
+    ifft_tables_kernel<<<8, 256, 0, st>>>(g.ns, g.nslog, nsamp, std::exp(sigma * g.dts), tw, fac);
     const size_t smem = (size_t)g.ns * sizeof(double2);
     cudaFuncSetAttribute(ifft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     ifft_kernel<<<(unsigned)ntr, IFFT_THREADS, smem, st>>>(S, (const double2*)d_sp, tw, fac, d_ts);

@@ -57,7 +57,7 @@ constexpr int IFFT_TWA = 0, IFFT_TWB = 256, IFFT_TW_EXTRA = 4096;
 inline size_t ifft_fast_twiddle_bytes(int ns) { return ((size_t)ns + IFFT_TW_EXTRA) * sizeof(double2); }
 cudaError_t ifft_fast_launch(const SynthDev& S, long long ntr, const double2* X, const double2* tw, const double* fac,
                              float* traces, cudaStream_t st);
-cudaError_t ifft_fast_twiddles_launch(int N, double2* tw, cudaStream_t st);
+cudaError_t ifft_fast_twiddles_launch(int N, double2* tw, int nsamp, double arg, double* fac, cudaStream_t st);   // fac[i] = e^{arg i}
 inline bool ifft_fast_supported(int ns) { return ns >= 512 && ns <= IFFT_MAX_NS; }
 
 // fast-form Legendre tables (legendre_fast.cu): the tables of legendre_kernel with
