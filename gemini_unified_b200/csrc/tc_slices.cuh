@@ -21,27 +21,51 @@ __device__ __forceinline__ double pow2_above(double x) {
 // the 7-bit slices of x, |x| < 1: x = sum_i q_i 128^-(i+1) + O(128^-S).  The
 // slices are the base-128 digits of u = trunc(|x| 128^S) with the sign of x
 // (x 128^S is exact and the conversion truncates), the same digits as S
-// rounds of x *= 128, q = trunc(x), x -= q, all of which are exact.  u is taken
-// in two parts of 32 bits, the upper three digits and the others.
+// rounds of x *= 128, q = trunc(x), x -= q, all of which are exact.
+// Of four numbers y = x 128^S: w[i] holds the four bytes of slice i.  The upper
+// three digits and the others are spread to bytes and signed four at a time, then
+// transposed (about 25 instructions per number for 6 slices; one digit at a time, 80).
 template <int NS>
-__device__ __forceinline__ void slices_of(double x, int q[NS]) {
+__device__ __forceinline__ void slice_words(const double (&y)[4], unsigned (&w)[NS]) {
   static_assert(NS == 6 || NS == 7, "three digits above 21 or 28 bits");
   constexpr int LOW = 7 * (NS - 3);
-  const long long y = (long long)(x * (double)(1ull << (7 * NS)));
-  const unsigned long long u = y < 0 ? (unsigned long long)(-y) : (unsigned long long)y;
-  const unsigned hi = (unsigned)(u >> LOW), lo = (unsigned)u & ((1u << LOW) - 1u);
-  const int s = y < 0 ? -1 : 0;
+  unsigned h[4], g[4];
 #pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    const unsigned d = i < 3 ? (hi >> (7 * (2 - i))) & 127u : (lo >> (7 * (NS - 1 - i))) & 127u;
-    q[i] = ((int)d ^ s) - s;
+  for (int b = 0; b < 4; ++b) {
+    const unsigned long long u = __double2ull_rz(fabs(y[b]));
+    const unsigned hi = (unsigned)(u >> LOW), lo = (unsigned)u;
+    h[b] = (hi & 0x7fu) | ((hi << 1) & 0x7f00u) | ((hi << 2) & 0x7f0000u);
+    g[b] = (lo & 0x7fu) | ((lo << 1) & 0x7f00u) | ((lo << 2) & 0x7f0000u) | (NS == 7 ? (lo << 3) & 0x7f000000u : 0u);
+    if (__double2hiint(y[b]) < 0) {   // 128 - d in every byte, then its top bit flipped: -d
+      h[b] = (0x80808080u - h[b]) ^ 0x80808080u;
+      g[b] = (0x80808080u - g[b]) ^ 0x80808080u;
+    }
   }
+  auto transpose = [](const unsigned (&a)[4], unsigned& o0, unsigned& o1, unsigned& o2, unsigned& o3) {
+    const unsigned p = __byte_perm(a[0], a[1], 0x5140), q = __byte_perm(a[2], a[3], 0x5140);
+    const unsigned r = __byte_perm(a[0], a[1], 0x7362), s = __byte_perm(a[2], a[3], 0x7362);
+    o0 = __byte_perm(p, q, 0x5410);
+    o1 = __byte_perm(p, q, 0x7632);
+    o2 = __byte_perm(r, s, 0x5410);
+    o3 = __byte_perm(r, s, 0x7632);
+  };
+  unsigned none;
+  transpose(h, w[2], w[1], w[0], none);
+  transpose(g, w[NS - 1], w[NS - 2], w[NS - 3], NS == 7 ? w[3] : none);
 }
 
-// 1/s for a power of two s whose reciprocal is a normal double (then x * (1/s)
-// equals x / s exactly), else 0: the callers then divide
-__device__ __forceinline__ double inv_pow2(double s) { return s >= 0x1p-1021 && s <= 0x1p1021 ? 1.0 / s : 0.0; }
-__device__ __forceinline__ double div_pow2(double x, double s, double inv) { return inv != 0.0 ? x * inv : x / s; }
+// x 128^S / s of a power of two s, by one product where its factor is exact
+struct SliceScale {
+  double s, f;
+};
+template <int NS>
+__device__ __forceinline__ SliceScale slice_scale(double s) {
+  return {s, s >= 0x1p-900 && s <= 0x1p900 ? (double)(1ull << (7 * NS)) / s : 0.0};
+}
+template <int NS>
+__device__ __forceinline__ double slice_scaled(double x, SliceScale k) {
+  return k.f != 0.0 ? x * k.f : x / k.s * (double)(1ull << (7 * NS));
+}
 
 __device__ __forceinline__ double block_max(double m) {
   __shared__ double red[32];
@@ -88,25 +112,23 @@ __global__ void __launch_bounds__(256) coef_rows_kernel(F f, const float* __rest
     mi = fmax(mi, fabs(w * (double)gi[o + l] * sl[l]));
   }
   const double rr = pow2_above(block_max(mr)), ri = pow2_above(block_max(mi));   // the barriers publish wgt and kext
-  const double ir = inv_pow2(rr), ii = inv_pow2(ri);
+  const SliceScale kr = slice_scale<NS>(rr), ki = slice_scale<NS>(ri);
   const long long r0 = K.rowoff[kind] + row, plane = K.mtot * K.Kp;
   if (threadIdx.x == 0) { K.rscale[r0] = rr; K.rscale[r0 + 1] = ri; }
   const int end = (kext + K.tile_k - 1) / K.tile_k * K.tile_k;   // <= Kp
   for (int l0 = 4 * threadIdx.x; l0 < end; l0 += 4 * blockDim.x) {
-    unsigned qr[NS] = {}, qi[NS] = {};
+    double yr[4] = {}, yi[4] = {};
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int l = l0 + b;
       if (l < nwn) {
-        int d[NS];
-        slices_of<NS>(div_pow2(wgt[l] * (double)gr[o + l] * sl[l], rr, ir), d);
-#pragma unroll
-        for (int i = 0; i < NS; ++i) qr[i] |= ((unsigned)d[i] & 255u) << (8 * b);
-        slices_of<NS>(div_pow2(wgt[l] * (double)gi[o + l] * sl[l], ri, ii), d);
-#pragma unroll
-        for (int i = 0; i < NS; ++i) qi[i] |= ((unsigned)d[i] & 255u) << (8 * b);
+        yr[b] = slice_scaled<NS>(wgt[l] * (double)gr[o + l] * sl[l], kr);
+        yi[b] = slice_scaled<NS>(wgt[l] * (double)gi[o + l] * sl[l], ki);
       }
     }
+    unsigned qr[NS], qi[NS];
+    slice_words<NS>(yr, qr);
+    slice_words<NS>(yi, qi);
     signed char* a = K.A8 + r0 * K.Kp + l0;
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
