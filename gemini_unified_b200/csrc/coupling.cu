@@ -211,6 +211,14 @@ __device__ __forceinline__ double cpl_taper(int lmax, int l) {
   return c * c;
 }
 
+// taper of every degree of every frequency, at the position of its spectrum: the sums
+// of a frequency share it.  One block per frequency.
+__global__ void __launch_bounds__(256) cpl_taper_kernel(CplDev S, double* tap) {
+  const int nwn = S.nwn[S.nf1 + blockIdx.x - 1];
+  double* t = tap + S.koff[blockIdx.x];
+  for (int l = threadIdx.x; l < nwn; l += blockDim.x) t[l] = cpl_taper(nwn - 1, l);
+}
+
 // w[l] = (2l+1)/4pi and w[lcap + l] = 2/(l(l+1)): a sum's factor is 0, +-2 or
 // +-4 (the second times +-1 or +-2, which is exact)
 __global__ void cpl_degree_table_kernel(int lcap, double* w) {
@@ -250,19 +258,26 @@ __global__ void cpl_coef_kernel(CplDev S, const float* __restrict__ gr, const fl
 struct CplRows {
   CplDev S;
   const double* wtab;   // cpl_degree_table_kernel's
+  const double* tap;    // cpl_taper_kernel's
   __device__ const CplSum& sum(int k) const { return S.istyp == 1 ? c_cpl[k] : c_cplf[k]; }
   __device__ int nf() const { return S.nf2 - S.nf1 + 1; }
-  __device__ int nsum() const { return S.nsum; }
   __device__ int nwn(int slot) const { return S.nwn[S.nf1 + slot - 1]; }
   __device__ int kind(int k) const { return sum(k).kind; }
   __device__ int rank(int k) const { return S.rank[k]; }
   __device__ int nsk(int kind) const { return S.nsk[kind]; }
   __device__ long long index(int slot, int k) const { return (long long)sum(k).col * S.nkf + S.koff[slot]; }
-  __device__ double weight(int slot, int k, int l) const {
+  struct Row {
+    const double *w, *tap, *w2;   // w2 null: no factor
+    double m;
+    int l0;
+    __device__ double operator()(int l) const {
+      const double c = w[l] * tap[l];
+      return w2 ? c * (m * w2[l]) : c;
+    }
+  };
+  __device__ Row row(int slot, int k) const {
     const CplSum& cs = sum(k);
-    if (l < cs.l0) return 0.0;
-    const double c = wtab[l] * cpl_taper(nwn(slot) - 1, l);
-    return cs.fac == 0.0 ? c : c * (0.5 * cs.fac * wtab[S.lcap + l]);
+    return {wtab, tap + S.koff[slot], cs.fac == 0.0 ? nullptr : wtab + S.lcap, 0.5 * cs.fac, cs.l0};
   }
 };
 
@@ -615,7 +630,7 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   const size_t b_in = align256((size_t)nf * sizeof(int)) + align256((size_t)p->nf2 * sizeof(int)) +
                       3 * align256((size_t)npts * 3 * sizeof(double)) + align256(evf.size() * sizeof(double2)) +
                       align256((size_t)p->nf2 * 7 * sizeof(double2)) +
-                      (fast ? align256((size_t)2 * lcap * sizeof(double)) +
+                      (fast ? align256(((size_t)2 * lcap + k) * sizeof(double)) +
                                   align256((size_t)npts * CPL_NKIND * lcap * sizeof(short))
                             : 0);
   char* ws = (char*)gem_ctx_aux(ctx, 12, b_tab + b_a + b_hd + b_x + b_in);
@@ -633,7 +648,7 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   double* d_nrm = (double*)take((size_t)npts * 3 * sizeof(double));
   double2* d_evf = (double2*)take(evf.size() * sizeof(double2));
   double2* d_zel = (double2*)take((size_t)p->nf2 * 7 * sizeof(double2));
-  double* wtab = fast ? (double*)take((size_t)2 * lcap * sizeof(double)) : nullptr;
+  double* wtab = fast ? (double*)take(((size_t)2 * lcap + k) * sizeof(double)) : nullptr;
   short* texp = fast ? (short*)take((size_t)npts * CPL_NKIND * lcap * sizeof(short)) : nullptr;
   if (cudaMemcpyAsync(d_koff, koff.data(), (size_t)nf * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_nwn, nwn, (size_t)p->nf2 * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -660,7 +675,10 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
     cpl_legendre_kernel<<<(npts * 3 + 127) / 128, 128, 0, st>>>(npts, p->nwnmax - 1, lcap, d_delta, tab);
     if (fast) tc_exponents_launch(tab, (long long)npts * CPL_NKIND * lcap, texp, st);
   }
-  if (fast) cpl_degree_table_kernel<<<(lcap + 255) / 256, 256, 0, st>>>(lcap, wtab);
+  if (fast) {
+    cpl_degree_table_kernel<<<(lcap + 255) / 256, 256, 0, st>>>(lcap, wtab);
+    cpl_taper_kernel<<<nf, 256, 0, st>>>(S, wtab + 2 * (size_t)lcap);
+  }
   const long long ncoef = (long long)nf * nsum * lcap;
   if (!fast) cpl_coef_kernel<<<(unsigned)((ncoef + 255) / 256), 256, 0, st>>>(S, d_gr, d_gi, A);
   int maxnsk = 0;
@@ -681,7 +699,7 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
     void* tws = gem_ctx_aux(ctx, 14, wsb);
     if (!tws) return GEM_ERROR;
     const TcCoefs rows = [&](const TcCoefSink& K, cudaStream_t s) {
-      return coef_rows_launch(CplRows{S, wtab}, nf * nsum, d_gr, d_gi, K, s);
+      return coef_rows_launch(CplRows{S, wtab, wtab + 2 * (size_t)lcap}, nsum, nf, d_gr, d_gi, K, s);
     };
     if (const char* why = sums_tc_run(TP, nwn, mtot, tab, texp, rows, C, tws, wsb, gem_ctx_tc_wait_ns(ctx), st))
       return gem_set_error(ctx, why);

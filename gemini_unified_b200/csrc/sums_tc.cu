@@ -88,8 +88,6 @@ template <int BN_, int WLO_, int WHI_> struct TcShape {
 constexpr unsigned long long TC_WAIT_NS = 1000000000ull;   // default pipeline wait limit and the drain limit
 
 constexpr int TC_COLMAX_NONE = (int)0x80808080u;   // a column of zeros (every byte 0x80)
-// finite non-zero exponent, else 0
-__device__ __forceinline__ int tc_finite(short e) { return e == 2047 ? 0 : e; }
 
 // ---------------------------------------------------------------------------
 //  Operand preparation (FP64 in, INT8 slices out)

@@ -249,26 +249,40 @@ __global__ void bessel_coef_kernel(SynthDev S, const float* __restrict__ gr, con
   Ar[S.lcap + jj] = vi;
 }
 
+// taper of every degree (wavenumber) of every frequency, at the position of its spectrum: the
+// sums of a frequency share it, and its cosines in the taper's 20 % of the degrees cost more than
+// the rest of a coefficient row.  One block per frequency.
+__global__ void __launch_bounds__(256) taper_kernel(SynthDev S, double* tap) {
+  const int nwn = S.nwn[S.nf1 + blockIdx.x - 1];
+  double* t = tap + S.koff[blockIdx.x];
+  for (int l = threadIdx.x; l < nwn; l += blockDim.x)
+    t[l] = S.global_ ? degree_taper(nwn - 1, l) : wn_taper(nwn, S.dwn, l + 1);
+}
+
 // coefficient rows of the tensor-core products (tc_slices.cuh): degree sums and wavenumber integrals
 struct SynthRows {
   SynthDev S;
   const double* wtab;   // degree_table_kernel's
+  const double* tap;    // taper_kernel's
   __device__ int nf() const { return S.nf2 - S.nf1 + 1; }
-  __device__ int nsum() const { return S.nsum; }
   __device__ int nwn(int slot) const { return S.nwn[S.nf1 + slot - 1]; }
   __device__ int kind(int k) const { return c_sum_kind[S.istyp][k]; }
-  __device__ int rank(int k) const { return sum_rank(S.istyp, k); }
+  __device__ int rank(int k) const { return S.rank[k]; }
   __device__ int nsk(int kind) const { return S.nsk[kind]; }
   __device__ long long index(int slot, int k) const {
     return (long long)S.col_off[c_sum_col[S.istyp][k]] * S.nkf + S.koff[slot];
   }
-  __device__ double weight(int slot, int k, int l) const {
-    if (S.global_) {
-      if (l < c_sum_l0[S.istyp][k]) return 0.0;
-      const double fac = c_sum_fac[S.istyp][k];
-      return (fac == 0.0 ? wtab[l] : 0.5 * fac * wtab[S.lcap + l]) * degree_taper(nwn(slot) - 1, l);
-    }
-    return wn_taper(nwn(slot), S.dwn, l + 1) * c_wn_sign[S.istyp][k];
+  struct Row {
+    const double *w, *tap;   // w null: regional
+    double m;
+    int l0;
+    __device__ double operator()(int l) const { return (w ? m * w[l] : m) * tap[l]; }
+  };
+  __device__ Row row(int slot, int k) const {
+    const double* tp = tap + S.koff[slot];
+    if (!S.global_) return {nullptr, tp, c_wn_sign[S.istyp][k], 0};
+    const double fac = c_sum_fac[S.istyp][k];
+    return {fac == 0.0 ? wtab : wtab + S.lcap, tp, fac == 0.0 ? 1.0 : 0.5 * fac, c_sum_l0[S.istyp][k]};
   }
 };
 
@@ -740,7 +754,8 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   int rank[8] = {};
   for (int k = 0; k < S.nsum; ++k) {
     const int kind = SUM_KIND[p->istyp][k];
-    S.c0[k] = S.coff[kind] + 2LL * rank[kind]++ * nsta;
+    S.rank[k] = rank[kind]++;
+    S.c0[k] = S.coff[kind] + 2LL * S.rank[k] * nsta;
     S.cstep[k] = 2LL * nsk_h[kind] * nsta;
   }
   for (int c = 0; c < 10; ++c) S.col_off[c] = c;
@@ -783,7 +798,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
                             o_tred ? nsta * sizeof(double) : 0, o_ns ? nsta * sizeof(int) : 0,
                             o_sf ? (size_t)nsta * 3 * p->nf2 * sizeof(double2) : 0, (size_t)nstf * sizeof(float),
                             fast ? (size_t)8 * S.lcap * nsta * sizeof(short) : 0,
-                            fast ? (size_t)2 * S.lcap * sizeof(double) : 0};
+                            fast ? ((size_t)2 * S.lcap + kk) * sizeof(double) : 0};
   size_t total = 0;
   for (size_t z : sizes) total += (z + 255) / 256 * 256;
   char* pool = (char*)gem_ctx_aux(ctx, 4, total);
@@ -839,8 +854,10 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
     const TcProblem TP = tc_problem_of(S);
     const size_t wsb = sums_tc_workspace(TP, mtot, nullptr);
     void* ws = gem_ctx_aux(ctx, 3, wsb);
+    double* tap = wtab + 2 * (size_t)S.lcap;
+    taper_kernel<<<nf, 256, 0, st>>>(S, tap);
     const TcCoefs rows = [&](const TcCoefSink& K, cudaStream_t s) {
-      return coef_rows_launch(SynthRows{S, wtab}, nf * S.nsum, d_gr, d_gi, K, s);
+      return coef_rows_launch(SynthRows{S, wtab, tap}, S.nsum, nf, d_gr, d_gi, K, s);
     };
     const char* why = ws ? sums_tc_run(TP, nwn, mtot, b.tab, texp, rows, b.C, ws, wsb, gem_ctx_tc_wait_ns(ctx), st) : "";
     if (why) {

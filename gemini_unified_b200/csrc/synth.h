@@ -18,6 +18,7 @@ struct SynthDev {
   const double2* stafil;    // [nsta][3][nf2] station filter per component, or null: unit filter
   int nsk[8];               // sums per Legendre table kind
   long long aoff[8], coff[8];   // offsets of each kind's coefficient and result matrices
+  int rank[14];             // rank of each sum among the sums of its table kind
   long long c0[14], cstep[14];  // per sum: its real row of the first frequency in the results, step to the next frequency
   int col_off[10];          // FK column of each (component, jump) spectrum
   const int* nwn;           // [nf2]

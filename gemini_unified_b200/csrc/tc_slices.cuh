@@ -10,13 +10,8 @@
 
 namespace gem {
 
-// smallest power of two strictly above |x| (1 for 0 or non-finite)
-__device__ __forceinline__ double pow2_above(double x) {
-  if (!(x > 0.0) || !isfinite(x)) return 1.0;
-  int e;
-  frexp(x, &e);   // x = f 2^e, f in [0.5, 1)
-  return ldexp(1.0, e);
-}
+// finite non-zero exponent, else 0
+__device__ __forceinline__ int tc_finite(short e) { return e == 2047 ? 0 : e; }
 
 // the 7-bit slices of x, |x| < 1: x = sum_i q_i 128^-(i+1) + O(128^-S).  The
 // slices are the base-128 digits of u = trunc(|x| 128^S) with the sign of x
@@ -54,100 +49,131 @@ __device__ __forceinline__ void slice_words(const double (&y)[4], unsigned (&w)[
   transpose(g, w[NS - 1], w[NS - 2], w[NS - 3], NS == 7 ? w[3] : none);
 }
 
-// x 128^S / s of a power of two s, by one product where its factor is exact
+// Scale 2^(e - 1022) of a row from its largest finite biased exponent e (no number above
+// the subnormals: 1), and 128^S over it as two factors of half
+// the shift, whose products with the row's numbers are exact
 struct SliceScale {
-  double s, f;
+  double s, f1, f2;
 };
 template <int NS>
-__device__ __forceinline__ SliceScale slice_scale(double s) {
-  return {s, s >= 0x1p-900 && s <= 0x1p900 ? (double)(1ull << (7 * NS)) / s : 0.0};
-}
-template <int NS>
-__device__ __forceinline__ double slice_scaled(double x, SliceScale k) {
-  return k.f != 0.0 ? x * k.f : x / k.s * (double)(1ull << (7 * NS));
-}
-
-__device__ __forceinline__ double block_max(double m) {
-  __shared__ double red[32];
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  m = red[0];
-  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-  __syncthreads();
-  return m;
+__device__ __forceinline__ SliceScale slice_scale(int e) {
+  if (e == 0) e = 1022;
+  const int shift = 7 * NS - (e - 1022), a = shift / 2;
+  auto pow2 = [](int n) { return __hiloint2double((1023 + n) << 20, 0); };
+  return {pow2(e - 1022), pow2(a), pow2(shift - a)};
 }
 
 // A8[i][row][l] = slice i of A[row][l] s_l / r_row for the row pair (re, im) of
 // sum k of frequency slot, r_row the power of two above the row's largest
-// |A s_l|.  One block per (slot, sum).  The coefficients A = F::weight times the
-// spectrum are never stored: the row's weights stay in shared memory between the
-// pass for the largest value and the slicing.  Slices are written up to the end
+// |A s_l|.  One block per (sum, slot).  The coefficients A = F's weight times the
+// spectrum are never stored: the products stay in registers between the pass for
+// the largest value and the slicing.  Slices are written up to the end
 // of the k-loop of the row's 128-row tile, which is all the products read.
-// F: nwn(slot), kind(sum), rank(sum), nsk(kind), nf(), nsum(), weight(slot, sum,
-// l) for l < nwn, and index(slot, sum): position of degree 0 in gr and gi.
+// F: nwn(slot), kind(sum), rank(sum), nsk(kind), nf(), row(slot,
+// sum): the weights w(l), w.l0 <= l < nwn, and index(slot, sum): position of degree 0 in gr and gi.
 // Bound: the slices' bytes.  Coefficients to FP64 rows, then slices, took 0.40 +
 // 0.52 ms for the coupling at 1000 points (34,440 rows, 883 MB of FP64 written
 // once and read twice), 0.22 + 0.30 ms for the regional integrals of 1001
-// stations, 0.17 + 0.17 ms for the network; in one kernel 0.41, 0.20 and 0.15 ms.
-template <int NS, class F>
-__global__ void __launch_bounds__(256) coef_rows_kernel(F f, const float* __restrict__ gr, const float* __restrict__ gi,
-                                                        TcCoefSink K) {
-  extern __shared__ double wgt[];   // [K.K]
-  __shared__ int kext;
-  const int k = blockIdx.x % f.nsum(), slot = blockIdx.x / f.nsum();
+// stations, 0.17 + 0.17 ms for the network; in one kernel that passed twice over
+// the spectrum, weights in shared memory, 0.40, 0.20 and 0.14 ms, bound by its
+// instructions (taper cosines per sum, divisions per block, scales by maxima of
+// doubles).  Each thread now keeps the products of 4 R degrees between the passes,
+// the scales come from the largest exponents behind one barrier, and the tapers from
+// a table that the sums of a frequency share: 0.31, 0.14 and 0.10 ms.
+template <int NS, int R, class F>
+__global__ void __launch_bounds__(512, 2) coef_rows_kernel(F f, const float* __restrict__ gr, const float* __restrict__ gi,
+                                                           TcCoefSink K) {
+  __shared__ int red[2][16], tile_ext;
+  const int k = blockIdx.x, slot = blockIdx.y;
   const int kind = f.kind(k), nsk = f.nsk(kind), nwn = min(f.nwn(slot), K.K);
   const int row = 2 * (slot * nsk + f.rank(k));
-  const int m0 = row / K.tile_rows * K.tile_rows, s0 = m0 / (2 * nsk), s1 = min(f.nf() - 1, (m0 + K.tile_rows - 1) / (2 * nsk));
-  if (threadIdx.x == 0) kext = 1;
-  __syncthreads();
-  for (int s = s0 + threadIdx.x; s <= s1; s += blockDim.x) atomicMax(&kext, min(f.nwn(s), K.K));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const double* sl = K.lscale + (long long)kind * K.Kp;
   const long long o = f.index(slot, k);
-  double mr = 0.0, mi = 0.0;
-  for (int l = threadIdx.x; l < nwn; l += blockDim.x) {
-    const double w = f.weight(slot, k, l);
-    wgt[l] = w;
-    mr = fmax(mr, fabs(w * (double)gr[o + l] * sl[l]));
-    mi = fmax(mi, fabs(w * (double)gi[o + l] * sl[l]));
+  const float *pr = gr + o, *pi = gi + o;
+  const auto weight = f.row(slot, k);
+  if (warp == nwarp - 1) {   // largest count of the rows' tile
+    const int m0 = row / K.tile_rows * K.tile_rows, s0 = m0 / (2 * nsk), s1 = min(f.nf() - 1, (m0 + K.tile_rows - 1) / (2 * nsk));
+    int kext = 1;
+    for (int s = s0 + lane; s <= s1; s += 32) kext = max(kext, min(f.nwn(s), K.K));
+    kext = __reduce_max_sync(0xffffffffu, kext);
+    if (lane == 0) tile_ext = kext;
   }
-  const double rr = pow2_above(block_max(mr)), ri = pow2_above(block_max(mi));   // the barriers publish wgt and kext
-  const SliceScale kr = slice_scale<NS>(rr), ki = slice_scale<NS>(ri);
-  const long long r0 = K.rowoff[kind] + row, plane = K.mtot * K.Kp;
-  if (threadIdx.x == 0) { K.rscale[r0] = rr; K.rscale[r0 + 1] = ri; }
-  const int end = (kext + K.tile_k - 1) / K.tile_k * K.tile_k;   // <= Kp
-  for (int l0 = 4 * threadIdx.x; l0 < end; l0 += 4 * blockDim.x) {
-    double yr[4] = {}, yi[4] = {};
+  int er = 0, ei = 0;   // upper words of the rows' largest finite absolute values
+  double vr[R][4], vi[R][4];
+  auto load = [&](int base) {
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int l = l0 + b;
-      if (l < nwn) {
-        yr[b] = slice_scaled<NS>(wgt[l] * (double)gr[o + l] * sl[l], kr);
-        yi[b] = slice_scaled<NS>(wgt[l] * (double)gi[o + l] * sl[l], ki);
+    for (int c = 0; c < R; ++c) {
+      const int l0 = base + 4 * (threadIdx.x + c * blockDim.x);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) vr[c][b] = vi[c][b] = 0.0;
+      if (l0 >= nwn) continue;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int l = l0 + b;
+        if (l < nwn && l >= weight.l0) {   // a spectrum need not be defined below a sum's first degree
+          const double w = weight(l), s = sl[l];
+          vr[c][b] = w * (double)pr[l] * s;
+          vi[c][b] = w * (double)pi[l] * s;
+        }
       }
     }
-    unsigned qr[NS], qi[NS];
-    slice_words<NS>(yr, qr);
-    slice_words<NS>(yi, qi);
-    signed char* a = K.A8 + r0 * K.Kp + l0;
+  };
+  const int part = 4 * R * blockDim.x;
+  for (int base = 0; base < nwn; base += part) {
+    load(base);
 #pragma unroll
-    for (int i = 0; i < NS; ++i) {
-      *reinterpret_cast<unsigned*>(a + i * plane) = qr[i];
-      *reinterpret_cast<unsigned*>(a + i * plane + K.Kp) = qi[i];
+    for (int c = 0; c < R; ++c)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int hr = __double2hiint(vr[c][b]) & 0x7fffffff, hi = __double2hiint(vi[c][b]) & 0x7fffffff;
+        er = max(er, hr < 0x7ff00000 ? hr : 0);
+        ei = max(ei, hi < 0x7ff00000 ? hi : 0);
+      }
+  }
+  er = __reduce_max_sync(0xffffffffu, er);
+  ei = __reduce_max_sync(0xffffffffu, ei);
+  if (lane == 0) { red[0][warp] = er; red[1][warp] = ei; }
+  __syncthreads();
+  const int q = min(lane, nwarp - 1);
+  er = __reduce_max_sync(0xffffffffu, red[0][q]) >> 20;
+  ei = __reduce_max_sync(0xffffffffu, red[1][q]) >> 20;
+  const SliceScale kr = slice_scale<NS>(er), ki = slice_scale<NS>(ei);
+  const long long r0 = K.rowoff[kind] + row, plane = K.mtot * K.Kp;
+  if (threadIdx.x == 0) { K.rscale[r0] = kr.s; K.rscale[r0 + 1] = ki.s; }
+  const int end = (tile_ext + K.tile_k - 1) / K.tile_k * K.tile_k;   // <= Kp
+  for (int base = 0; base < end; base += part) {
+    if (base > 0 || nwn > part) load(base);   // a row that does not fit the registers is formed again
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int l0 = base + 4 * (threadIdx.x + c * blockDim.x);
+      if (l0 >= end) break;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        vr[c][b] = vr[c][b] * kr.f1 * kr.f2;
+        vi[c][b] = vi[c][b] * ki.f1 * ki.f2;
+      }
+      unsigned qr[NS], qi[NS];
+      slice_words<NS>(vr[c], qr);
+      slice_words<NS>(vi[c], qi);
+      signed char* a = K.A8 + r0 * K.Kp + l0;
+#pragma unroll
+      for (int i = 0; i < NS; ++i) {
+        *reinterpret_cast<unsigned*>(a + i * plane) = qr[i];
+        *reinterpret_cast<unsigned*>(a + i * plane + K.Kp) = qi[i];
+      }
     }
   }
 }
 
+// 8 degrees per thread; 512 threads when a row has more than 2048
 template <class F>
-cudaError_t coef_rows_launch(const F& f, int nblocks, const float* gr, const float* gi, const TcCoefSink& K, cudaStream_t st) {
-  const size_t smem = (size_t)K.K * sizeof(double);
-  auto go = [&](auto kern) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<nblocks, 256, smem, st>>>(f, gr, gi, K);
-    return cudaGetLastError();
-  };
-  return K.nslice == 7 ? go(coef_rows_kernel<7, F>) : go(coef_rows_kernel<6, F>);
+cudaError_t coef_rows_launch(const F& f, int nsum, int nf, const float* gr, const float* gi, const TcCoefSink& K, cudaStream_t st) {
+  const int threads = K.K > 2048 ? 512 : 256;
+  const dim3 nblocks(nsum, nf);
+  if (K.nslice == 7) coef_rows_kernel<7, 2, F><<<nblocks, threads, 0, st>>>(f, gr, gi, K);
+  else coef_rows_kernel<6, 2, F><<<nblocks, threads, 0, st>>>(f, gr, gi, K);
+  return cudaGetLastError();
 }
 
 }  // namespace gem
