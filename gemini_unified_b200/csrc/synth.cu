@@ -769,29 +769,33 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   // ---- host tables: event filter, twiddles, exp(sigma t)
   std::vector<double2> evf;
   event_filter(p, evf);
+  const bool fast = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST;   // the tensor-core sums store no coefficient rows
+  const bool fast_fft = fast && ifft_fast_supported(ns);            // its tables are made on the device
   std::vector<double2> tw;
-  const double piz = 2.0 * PI_F;
-  for (int m = 1; m <= nslog; ++m) {
-    int nar = 1 << (m - 1), lar = ns / nar, larh = lar / 2;
-    double alpha = piz / (double)lar;
-    for (int jr = 1; jr <= larh; ++jr) {
-      double beta = alpha * (double)(jr - 1);
-      tw.push_back(make_double2(std::cos(beta), std::sin(beta)));
+  std::vector<double> fac;
+  if (!fast_fft) {
+    const double piz = 2.0 * PI_F;
+    for (int m = 1; m <= nslog; ++m) {
+      int nar = 1 << (m - 1), lar = ns / nar, larh = lar / 2;
+      double alpha = piz / (double)lar;
+      for (int jr = 1; jr <= larh; ++jr) {
+        double beta = alpha * (double)(jr - 1);
+        tw.push_back(make_double2(std::cos(beta), std::sin(beta)));
+      }
     }
+    fac.resize(p->nsamp);
+    double f = 1.0, expo = std::exp(p->sigma * dts);
+    for (int i = 0; i < p->nsamp; ++i) { fac[i] = f; f = f * expo; }
   }
-  std::vector<double> fac(p->nsamp);
-  double f = 1.0, expo = std::exp(p->sigma * dts);
-  for (int i = 0; i < p->nsamp; ++i) { fac[i] = f; f = f * expo; }
   // ---- device buffers
   SynthBuffers b;
   const long long ntr = (long long)nsta * nmt * 3;
   // all buffers of one run in one context-owned allocation, grown on demand
-  const bool fast_fft = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST && ifft_fast_supported(ns);
   const bool o_tred = o && o->tred, o_ns = o && o->nsamp_true, o_sf = o && o->stafilter;
-  const bool fast = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST;   // the tensor-core sums store no coefficient rows
   const size_t sizes[20] = {(size_t)8 * S.lcap * nsta * sizeof(double), fast ? 0 : (size_t)ao * sizeof(double),
                             (size_t)co * sizeof(double), (size_t)ntr * S.ldx * sizeof(double2),
-                            evf.size() * sizeof(double2), tw.size() * sizeof(double2), fac.size() * sizeof(double),
+                            evf.size() * sizeof(double2), tw.size() * sizeof(double2),
+                            (size_t)p->nsamp * sizeof(double),
                             (size_t)p->nf2 * sizeof(int), (size_t)nf * sizeof(int), nsta * sizeof(double),
                             nsta * sizeof(double), nsta * sizeof(double), (size_t)nmt * nfo * sizeof(double),
                             fast_fft ? ifft_fast_twiddle_bytes(ns) : 0,
@@ -799,36 +803,39 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
                             o_sf ? (size_t)nsta * 3 * p->nf2 * sizeof(double2) : 0, (size_t)nstf * sizeof(float),
                             fast ? (size_t)8 * S.lcap * nsta * sizeof(short) : 0,
                             fast ? ((size_t)2 * S.lcap + kk) * sizeof(double) : 0};
-  size_t total = 0;
-  for (size_t z : sizes) total += (z + 255) / 256 * 256;
+  // the small inputs lie together, so that one copy brings them all (sixteen of a few KB each took
+  // about a fifth of a call with 50 stations)
+  const void* src[20] = {};
+  src[4] = evf.data(); src[5] = tw.data(); src[6] = fast_fft ? nullptr : fac.data(); src[7] = nwn; src[8] = koff.data();
+  src[9] = theta; src[10] = phi; src[11] = propdir; src[12] = mt;
+  src[14] = o_tred ? o->tred : nullptr; src[15] = o_ns ? o->nsamp_true : nullptr; src[17] = nstf > 0 ? o->stf : nullptr;
+  auto padded = [](size_t z) { return (z + 255) / 256 * 256; };
+  size_t total = 0, nin = 0;
+  for (int i = 0; i < 20; ++i) total += padded(sizes[i]);
   char* pool = (char*)gem_ctx_aux(ctx, 4, total);
   if (!pool) return GEM_ERROR;
   void* parts[20];
-  for (int i = 0; i < 20; ++i) { parts[i] = sizes[i] ? pool : nullptr; pool += (sizes[i] + 255) / 256 * 256; }
+  for (int i = 0; i < 20; ++i)
+    if (src[i] && sizes[i]) { parts[i] = pool + nin; nin += padded(sizes[i]); }
+  size_t at = nin;
+  for (int i = 0; i < 20; ++i)
+    if (!(src[i] && sizes[i])) { parts[i] = sizes[i] ? pool + at : nullptr; at += padded(sizes[i]); }
+  std::vector<char> in(nin);
+  for (int i = 0; i < 20; ++i)
+    if (src[i] && sizes[i]) std::memcpy(in.data() + ((char*)parts[i] - pool), src[i], sizes[i]);
   b.tab = (double*)parts[0]; b.A = (double*)parts[1]; b.C = (double*)parts[2]; b.X = (double2*)parts[3];
   b.evf = (double2*)parts[4]; b.tw = (double2*)parts[5]; b.fac = (double*)parts[6]; b.nwn = (int*)parts[7];
   b.koff = (int*)parts[8]; b.theta = (double*)parts[9]; b.phi = (double*)parts[10]; b.propdir = (double*)parts[11];
   b.mt = (double*)parts[12]; b.twx = (double2*)parts[13];
-  cudaMemcpyAsync(b.evf, evf.data(), evf.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
-  if (!fast_fft) cudaMemcpyAsync(b.fac, fac.data(), fac.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.nwn, nwn, (size_t)p->nf2 * sizeof(int), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.koff, koff.data(), nf * sizeof(int), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.theta, theta, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.phi, phi, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.propdir, propdir, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(b.mt, mt, (size_t)nmt * nfo * sizeof(double), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(pool, in.data(), nin, cudaMemcpyHostToDevice, st);
   short* texp = (short*)parts[18];
   double* wtab = (double*)parts[19];
   S.nwn = b.nwn; S.koff = b.koff;
   S.tred_sta = o_tred ? (const double*)parts[14] : nullptr;
   S.stafil = o_sf ? (const double2*)parts[16] : nullptr;
   const int* d_nstrue = o_ns ? (const int*)parts[15] : nullptr;
-  if (o_tred) cudaMemcpyAsync(parts[14], o->tred, nsta * sizeof(double), cudaMemcpyHostToDevice, st);
-  if (o_ns) cudaMemcpyAsync(parts[15], o->nsamp_true, nsta * sizeof(int), cudaMemcpyHostToDevice, st);
   if (o_sf)
     cudaMemcpyAsync(parts[16], o->stafilter, (size_t)nsta * 3 * p->nf2 * sizeof(double2), cudaMemcpyHostToDevice, st);
-  if (nstf > 0) cudaMemcpyAsync(parts[17], o->stf, (size_t)nstf * sizeof(float), cudaMemcpyHostToDevice, st);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0); cudaEventCreate(&e1);
   cudaEventRecord(e0, st);
