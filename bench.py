@@ -201,13 +201,13 @@ def run_reference(args, rank, size):
 
 
 def fk_launches_per_run(backend):
-    """Kernels one gem_fk_run_device call launches: knots, splines, (Horner table,) setup, 3 phases."""
-    return 6 + (1 if backend == 2 else 0)
+    """Kernels one gem_fk_run_device call launches: knots, splines, (Horner table,) start table, setup, 3 phases."""
+    return 7 + (1 if backend == 2 else 0)
 
 
-# mixed-precision synthetics: Legendre tables, coefficients, 5 operand-slicing kernels, tensor-core sums,
-# spectra, FFT twiddles, inverse FFT
-SYNTH_LAUNCHES = 11
+# mixed-precision synthetics: Legendre tables, degree factors, tapers, 4 kernels of the table operand,
+# coefficient rows, 2 launches of tensor-core sums, spectra, FFT twiddles, inverse FFT
+SYNTH_LAUNCHES = 13
 
 
 def main():
