@@ -290,16 +290,15 @@ struct SynthRows {
 // The integrals of a frequency and station share the Bessel functions at the ends
 // of the range: one thread per (frequency, integral, station) evaluated six of
 // them for each (7 single-force integrals of 512 frequencies at 1001 stations:
-// 0.30 -> 0.15 ms).
+// 0.30 -> 0.15 ms; with the sums' rows from the parameters instead of counted out
+// per integral 0.112 ms; 2 or 8 frequencies of a station per thread, which share the
+// geometry and the lower end's functions, 0.160 and 0.225 ms: the threads are too few).
 __global__ void __launch_bounds__(128) bessel_corr_kernel(SynthDev S, const float* __restrict__ gr,
                                                           const float* __restrict__ gi,
                                                           const double* __restrict__ theta, double* C) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int nf = S.nf2 - S.nf1 + 1;
   const int t = S.istyp;
-  if (idx >= (long long)nf * S.nsta) return;
-  const int sta = (int)(idx % S.nsta);
-  const int slot = (int)(idx / S.nsta);
+  const int sta = blockIdx.x * blockDim.x + threadIdx.x, slot = blockIdx.y;
+  if (sta >= S.nsta) return;
   const int nwn = S.nwn[S.nf1 + slot - 1];
   if (nwn < 2) return;
   const double re = S.rearth, dwn = S.dwn;
@@ -316,6 +315,7 @@ __global__ void __launch_bounds__(128) bessel_corr_kernel(SynthDev S, const floa
       y3.b0 = y0(a3); y3.b1 = y1(a3); y3.b2 = -y3.b0 + 2.0 / a3 * y3.b1;
     }
   }
+  const double sx = 1.0 - sin(g.xdk) / g.xdk;
   const double tn = wn_taper(nwn, dwn, nwn), t3 = filon ? wn_taper(nwn, dwn, g.j3) : 0.0;
   for (int k = 0; k < S.nsum; ++k) {
     const int kind = c_sum_kind[t][k];
@@ -329,17 +329,16 @@ __global__ void __launch_bounds__(128) bessel_corr_kernel(SynthDev S, const floa
       const double ybn = sg * wn_kernel(kind, wne, ye.b0, ye.b1, ye.b2, re, g.x);
       const double yb3 = sg * wn_kernel(kind, wn3, y3.b0, y3.b1, y3.b2, re, g.x);
       corr = corr - (G(nwn) * kn) * (tn * g.F);
-      corr = corr + ((G(nwn) * ybn) * tn - (G(g.j3) * yb3) * t3) / g.x * (1.0 - sin(g.xdk) / g.xdk);
+      corr = corr + ((G(nwn) * ybn) * tn - (G(g.j3) * yb3) * t3) / g.x * sx;
     } else if (nwn == g.j3) {
       corr = corr - (G(nwn) * kn) * (tn * g.F);   // no Filon part
     } else {
       corr = corr - (G(nwn) * kn) * (tn * 0.5 * dwn);   // trapezoid end
     }
     corr = corr * (re * re / (2.0 * PI_F));
-    const long long row = 2LL * ((long long)slot * S.nsk[kind] + sum_rank(t, k));
-    double* Ck = C + S.coff[kind];
-    Ck[row * S.nsta + sta] += corr.re;
-    Ck[(row + 1) * S.nsta + sta] += corr.im;
+    double* Ck = C + S.c0[k] + slot * S.cstep[k] + sta;
+    Ck[0] += corr.re;
+    Ck[S.nsta] += corr.im;
   }
 }
 
@@ -878,8 +877,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
     sums_gemm_kernel<<<g, 256, 0, st>>>(S, b.A, b.tab, b.C);
   }
   if (p->global_ == 0) {
-    const long long ncorr = (long long)nf * nsta;
-    bessel_corr_kernel<<<(unsigned)((ncorr + 127) / 128), 128, 0, st>>>(S, d_gr, d_gi, b.theta, b.C);
+    bessel_corr_kernel<<<dim3((nsta + 127) / 128, nf), 128, 0, st>>>(S, d_gr, d_gi, b.theta, b.C);
   }
   const dim3 sgrid((unsigned)((nsta + SP_STA - 1) / SP_STA), (unsigned)((nf + SP_SLOT - 1) / SP_SLOT));
   if (S.istyp == 1) spectra_kernel<1><<<sgrid, SP_THREADS, 0, st>>>(S, b.C, b.evf, b.phi, b.propdir, b.mt, b.X);
