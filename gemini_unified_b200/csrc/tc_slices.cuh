@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(512, 2) coef_rows_kernel(F f, const float* __r
     }
   };
   const int part = 4 * R * blockDim.x;
-  for (int base = 0; base < nwn; base += part) {
+  int base = 0;
+  do {   // once for a frequency without degrees too: its products are the zeros that load() sets
     load(base);
 #pragma unroll
     for (int c = 0; c < R; ++c)
@@ -130,7 +131,8 @@ __global__ void __launch_bounds__(512, 2) coef_rows_kernel(F f, const float* __r
         er = max(er, hr < 0x7ff00000 ? hr : 0);
         ei = max(ei, hi < 0x7ff00000 ? hi : 0);
       }
-  }
+    base += part;
+  } while (base < nwn);
   er = __reduce_max_sync(0xffffffffu, er);
   ei = __reduce_max_sync(0xffffffffu, ei);
   if (lane == 0) { red[0][warp] = er; red[1][warp] = ei; }
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(512, 2) coef_rows_kernel(F f, const float* __r
   const long long r0 = K.rowoff[kind] + row, plane = K.mtot * K.Kp;
   if (threadIdx.x == 0) { K.rscale[r0] = kr.s; K.rscale[r0 + 1] = ki.s; }
   const int end = (tile_ext + K.tile_k - 1) / K.tile_k * K.tile_k;   // <= Kp
-  for (int base = 0; base < end; base += part) {
+  for (base = 0; base < end; base += part) {
     if (base > 0 || nwn > part) load(base);   // a row that does not fit the registers is formed again
 #pragma unroll
     for (int c = 0; c < R; ++c) {

@@ -58,3 +58,14 @@ def test_rows(fk, n):
     from gemini_unified_b200.synth_run import fk_coefficients
     g = _grid(fk[0], [n, 5, n - 1])   # rows of very different length share a tile
     _check(*_run(fk, g, n, *fk_coefficients(10, int(g.nkfmax))))
+
+
+@pytest.mark.parametrize("counts", [(300, 0, 299), (3000, 0, 2999), (9000, 0, 2, 0), (300, 1, 299)])
+def test_frequency_without_degrees(fk, counts):
+    """A frequency without degrees (or with degree 0 alone) adds nothing: the other
+    rows of its tile are as long as ever.  The spectra vanish there in the FP64 form."""
+    from gemini_unified_b200.synth_run import fk_coefficients
+    nwn = np.zeros(fk[0].nf1 - 1 + len(counts), np.int32)
+    nwn[fk[0].nf1 - 1:] = counts
+    g = dataclasses.replace(fk[0], nf2=len(nwn), nwn=nwn, nwnmax=max(counts))
+    _check(*_run(fk, g, counts[0], *fk_coefficients(10, int(g.nkfmax))))
