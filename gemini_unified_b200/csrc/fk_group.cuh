@@ -92,6 +92,18 @@ struct GroupTab {   // in shared memory: lanes index them divergently
   double2 ext[4][5];   // extrapolation weights (w, e) of attempt 6, 5, 4 (chains 0, 1, 2) and 3 on attempts 1, 2, 3, 5, 4
   unsigned char grid[GP_PTS + 3], index[52];
 };
+__device__ __forceinline__ void group_tab(GroupTab& T) {
+  int np = 0;
+  for (int g = 0; g <= 48; ++g) {
+    T.index[g] = (unsigned char)np;
+    if (g % 3 == 0 || g % 4 == 0) T.grid[np++] = (unsigned char)g;
+  }
+  for (int q = 0; q < 4; ++q)
+    for (int l = 0; l < 5; ++l) {
+      const int j = 6 - q, i = l < 3 ? l + 1 : (l == 3 ? 5 : 4);
+      T.ext[q][l] = i < j ? make_double2(EXTRAP.w[j][i - 1], EXTRAP.e[j][i - 1]) : make_double2(0.0, 0.0);
+    }
+}
 
 // One step of the groups with act set (all lanes of the warp call); the result
 // (attempts, 0 for a failed step) is returned to every lane of the group and an
@@ -224,6 +236,7 @@ __device__ __noinline__ int group_step(const FKStatic& P, GroupItem<PH>& G, cons
       sys_at<SYS, ISO>(e, zom2, fma((double)(2 * (p + 1)), h48, x), E);
       put_entries<SYS>(E, G.E + p * QS);
     }
+    __syncwarp();   // the rows are other lanes' stores, and a vote orders no memory
     const unsigned onm7 = __ballot_sync(FULL, on7);
     if (on7) {
       const double hf = 2.0 * h48;
@@ -267,18 +280,7 @@ __global__ void __launch_bounds__(GP_WARPS * 32, 1) fk_group_kernel(const __grid
   __shared__ GroupTab T;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & (GL - 1);
-  if (threadIdx.x == 0) {
-    int np = 0;
-    for (int g = 0; g <= 48; ++g) {
-      T.index[g] = (unsigned char)np;
-      if (g % 3 == 0 || g % 4 == 0) T.grid[np++] = (unsigned char)g;
-    }
-    for (int q = 0; q < 4; ++q)
-      for (int l = 0; l < 5; ++l) {
-        const int j = 6 - q, i = l < 3 ? l + 1 : (l == 3 ? 5 : 4);
-        T.ext[q][l] = i < j ? make_double2(EXTRAP.w[j][i - 1], EXTRAP.e[j][i - 1]) : make_double2(0.0, 0.0);
-      }
-  }
+  if (threadIdx.x == 0) group_tab(T);
   load_tab(P, tab);
   load_bounds(P, tab);
   GroupItem<PH>& G = reinterpret_cast<GroupItem<PH>*>(gp_raw)[warp * IPW + lane / GL];

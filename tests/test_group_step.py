@@ -1,0 +1,33 @@
+"""The group form's step (csrc/fk_group.cuh) compiled for the host, one warp on 32
+threads (group_step_host.cpp)."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "gemini_unified_b200", "csrc")
+
+
+def _build(tmp_path, *flags):
+    if not shutil.which("g++"):
+        pytest.skip("no host compiler")
+    open(tmp_path / "cuda_runtime.h", "w").close()   # the harness declares what the headers need
+    exe = str(tmp_path / "warp")
+    cmd = ["g++", "-std=c++17", "-ffp-contract=off", "-w", "-I", str(tmp_path), "-I", CSRC, *flags,
+           os.path.join(HERE, "group_step_host.cpp"), "-o", exe, "-pthread"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if "-ltsan" in r.stderr or "libtsan" in r.stderr:
+        pytest.skip("no thread sanitizer")
+    assert r.returncode == 0, r.stderr[-2000:]
+    return exe
+
+
+def test_shared_memory_is_ordered(tmp_path):
+    """No access to the group's shared memory that only a vote separates from another lane's."""
+    r = subprocess.run([_build(tmp_path, "-O1", "-g", "-fsanitize=thread")], capture_output=True, text=True)
+    if "unexpected memory mapping" in r.stderr:
+        pytest.skip("the sanitizer cannot map its memory here")
+    assert "data race" not in r.stderr, r.stderr[:2000]
+    assert r.returncode == 0, r.stderr[:2000]
