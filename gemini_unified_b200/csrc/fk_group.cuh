@@ -180,17 +180,20 @@ __device__ __noinline__ int group_step(const FKStatic& P, GroupItem<PH>& G, cons
     }
   }
   __syncwarp();
-  // extrapolation to the attempt with result yj (component c) from the results
-  // of the attempts 1, 2, 3, 5, 4 (weight 0 for those not used yet), as in bs_step
-  auto extrapolate = [&](const double2* wt, dz yj, dz& yy, dz& dy) {
+  // extrapolation to the attempt with result yj (component c) from the first NL of the results of
+  // the attempts 1, 2, 3, 5, 4, as in bs_step.  5 and 4 have weight 0 where the thread form has not
+  // made them yet: left out, because they may have overflowed.
+  auto extrapolate = [&](auto NL, const double2* wt, dz yj, dz& yy, dz& dy) {
     yy = yj;
     dy = dz{0.0, 0.0};
 #pragma unroll
-    for (int l = 0; l < 5; ++l) {
+    for (int l = 0; l < decltype(NL)::value; ++l) {
       const double2 q = G.Y[(l < 3 ? l : (l == 3 ? 4 : 3)) * NV + c], k = wt[l];
-      const dz d = dz{q.x, q.y} - yj;
-      cfma(yy, k.x, d);
-      cfma(dy, k.y, d);
+      if (l < 3 || k.x != 0.0) {
+        const dz d = dz{q.x, q.y} - yj;
+        cfma(yy, k.x, d);
+        cfma(dy, k.y, d);
+      }
     }
   };
   auto put_test = [&](int q, dz yy, dz dy) {
@@ -211,11 +214,11 @@ __device__ __noinline__ int group_step(const FKStatic& P, GroupItem<PH>& G, cons
   dz yy{0.0, 0.0}, dy{0.0, 0.0}, y3{0.0, 0.0};
   if (on) {
     const double2 q = G.Y[(5 - ch) * NV + c];
-    extrapolate(T.ext[ch], dz{q.x, q.y}, yy, dy);
+    extrapolate(std::integral_constant<int, 5>(), T.ext[ch], dz{q.x, q.y}, yy, dy);
     put_test(ch, yy, dy);
     if (ch == 2) {
       const double2 r = G.Y[2 * NV + c];
-      extrapolate(T.ext[3], dz{r.x, r.y}, y3, dy);
+      extrapolate(std::integral_constant<int, 2>(), T.ext[3], dz{r.x, r.y}, y3, dy);
       put_test(3, y3, dy);
     }
   }

@@ -3,7 +3,8 @@
 // exchanged by relaxed atomics and orders nothing, as on the GPU.  Built with
 // ThreadSanitizer, a shared-memory access of one lane that nothing orders with
 // another lane's is reported.
-// Every system, with steps that reach the seventh attempt.
+//   group_step_host race      every system, steps that reach the seventh attempt
+//   group_step_host compare   step sizes over many decades: group form = thread form, bit for bit
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -154,12 +155,57 @@ template <int PH, int SYS, bool ISO> void race() {
   }
 }
 
-int main() {
+static int seen[8], beyond;   // steps by their result; accepted ones beside an attempt that overflowed
+
+template <int PH, int SYS, bool ISO> int compare() {
+  constexpr int NG = 32 / GroupShape<PH>::GL, NV = SysNV<SYS>::NV, NVD = PhaseNV<PH>::NV;
+  std::vector<GroupItem<PH>> G(NG);
+  std::vector<double2> D(4 * NVD * 32), scratch(32 * FK_LANE_STEP_SLOTS);
+  int bad = 0;
+  for (double eps : {1e-6, 1e-2, 1e3})
+    for (int k = -6; k <= 64; ++k) {
+      P.eps = eps;
+      const double h = 500.0 * pow(10.0, k < 8 ? k / 4.0 : k - 6.0), y = k < 8 ? 1.0 : 1e-100;
+      std::vector<Lane> L(32);
+      for (int l = 0; l < 32; ++l) lane_state<PH>(L[l], 1010.0, h, y, l % NG);
+      for (int g = 0; g < NG; ++g) G[g].L = L[g];
+      const std::vector<int> rg = groups<PH, SYS, ISO>(G, 0xffu);
+      std::vector<int> rt(32);
+      warp([&](int l) {
+        dz ye[5];
+        Counters cnt{};
+        Lane& q = L[l];
+        bs_step<SYS, NVD, 4, ISO>(P, q.e, l < NG, q.h, q.x, q.y, ye, rt[l], D.data(), l, Slot{&scratch[l * FK_LANE_STEP_SLOTS], 1}, cnt, q.jknot);
+        if (rt[l])
+          for (int v = 0; v < NV; ++v) q.y[v] = ye[v];
+      });
+      for (int g = 0; g < NG; ++g) {
+        bool over = false;
+        for (int i = 0; i < 6 * NV; ++i) over |= !std::isfinite(G[g].Y[i].x);
+        ++seen[rt[g]];
+        beyond += rt[g] && over;
+        if (rg[g] == rt[g] && !memcmp(G[g].L.y, L[g].y, NV * sizeof(dz))) continue;
+        if (++bad < 4) printf("phase %d system %d eps %g h %g: group form %d, thread form %d\n", PH, SYS, eps, h, rg[g], rt[g]);
+      }
+    }
+  return bad;
+}
+
+int main(int argc, char** argv) {
   setup();
-  race<PH_TOR, SYS_TOROIDAL, true>();
-  race<PH_SPH, SYS_MINORS, true>();
-  race<PH_SPH, SYS_MINORS, false>();
-  race<PH_SPH, SYS_FLUID, true>();
-  race<PH_SPH, SYS_RADIAL, false>();
-  race<PH_ADJ, SYS_SOLIDT, true>();
+  if (argc > 1 && !strcmp(argv[1], "race")) {
+    race<PH_TOR, SYS_TOROIDAL, true>();
+    race<PH_SPH, SYS_MINORS, true>();
+    race<PH_SPH, SYS_MINORS, false>();
+    race<PH_SPH, SYS_FLUID, true>();
+    race<PH_SPH, SYS_RADIAL, false>();
+    race<PH_ADJ, SYS_SOLIDT, true>();
+    return 0;
+  }
+  const int bad = compare<PH_TOR, SYS_TOROIDAL, true>() + compare<PH_SPH, SYS_MINORS, false>() +
+                  compare<PH_SPH, SYS_RADIAL, true>() + compare<PH_ADJ, SYS_SOLIDT, true>();
+  printf("steps by attempts:");
+  for (int v : seen) printf(" %d", v);
+  printf("; accepted beside an overflow: %d; different: %d\n", beyond, bad);
+  return bad || !beyond || !seen[3] || !seen[4] || !seen[5] || !seen[6] || !seen[7] || !seen[0];
 }

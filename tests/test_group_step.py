@@ -26,8 +26,15 @@ def _build(tmp_path, *flags):
 
 def test_shared_memory_is_ordered(tmp_path):
     """No access to the group's shared memory that only a vote separates from another lane's."""
-    r = subprocess.run([_build(tmp_path, "-O1", "-g", "-fsanitize=thread")], capture_output=True, text=True)
+    r = subprocess.run([_build(tmp_path, "-O1", "-g", "-fsanitize=thread"), "race"], capture_output=True, text=True)
     if "unexpected memory mapping" in r.stderr:
         pytest.skip("the sanitizer cannot map its memory here")
     assert "data race" not in r.stderr, r.stderr[:2000]
     assert r.returncode == 0, r.stderr[:2000]
+
+
+def test_group_form_equals_thread_form(tmp_path):
+    """Steps of every size, from one whose attempts agree to one whose attempts overflow: the
+    group form makes more attempts than the thread form and may use no more of them."""
+    r = subprocess.run([_build(tmp_path, "-O2"), "compare"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
