@@ -85,6 +85,7 @@ struct gem_ctx {
   // queue granularity of each phase (index into FK_GRAN), per build
   int qgran[2][3] = {{FK_GRAN_DEFAULT, FK_GRAN_DEFAULT, FK_GRAN_DEFAULT},
                      {FK_GRAN_DEFAULT, FK_GRAN_DEFAULT, FK_GRAN_DEFAULT}};
+  bool tuning = false;   // set by gem_fk_autotune for its runs: thread form at every size
   // captured launch sequence of one slab (gem_fk_graph_build)
   cudaGraphExec_t graph_exec = nullptr;
   cudaStream_t graph_stream = nullptr;
@@ -535,10 +536,11 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
   return GEM_OK;
 }
 
-// Whether a phase runs in the group form (fk_group.cuh): few queue positions, and
-// none of the instruments of the thread form.
+// Whether a phase runs in the group form (fk_group.cuh): few queue positions, none of
+// the instruments of the thread form, and not while the autotuner times the thread
+// form's settings, which the group form has no use for.
 bool use_groups(const gem_ctx* ctx, const SlabPlan& S, int ph, const FKLaunch& L) {
-  if (!S.fast || ctx->d_prof || ctx->d_warp_ns || ctx->d_steplog) return false;
+  if (!S.fast || ctx->tuning || ctx->d_prof || ctx->d_warp_ns || ctx->d_steplog) return false;
   return (long long)L.nqueue <= FK_GROUP_MAX[S.P.hascore][ph];
 }
 
@@ -1086,12 +1088,20 @@ int gem_fk_queue_get(const gem_ctx* ctx, int* gran3) {
 
 // Autotuner: runs frequencies jf_first..jf_last once per candidate (all three
 // phases at once, repeats times, the minimum kept) and keeps per phase the
-// fastest.  Stage 1 tries the schedules (block size, matrix caching) under the
-// current deferral and queue granularity, stage 2 the deferrals under the
-// chosen schedules, stage 3 the queue granularities under both.
+// fastest.  Stage 1 tries the schedules (block size) under the current deferral
+// and queue granularity, stage 2 the deferrals under the chosen schedules,
+// stage 3 the queue granularities under both.  Every run takes the thread form,
+// whose settings these are: a slab small enough for the group form would time
+// that form for every candidate and keep one by chance for later large slabs.
 // ms[c*3 + ph]: stage-1 times for c < GEM_FK_NSCHED, then the stage-2 and the
-// stage-3 times; -1 for candidates not run (the plain build has no
-// matrix-caching variants).
+// stage-3 times; -1 for candidates not run (the plain build tries three schedules).
+namespace {
+struct TuneScope {
+  gem_ctx* c;
+  explicit TuneScope(gem_ctx* ctx) : c(ctx) { c->tuning = true; }
+  ~TuneScope() { c->tuning = false; }
+};
+}  // namespace
 int gem_fk_autotune(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, int repeats, float* ms,
                     int* sched3, int* defer3) {
   if (!ctx) return GEM_ERROR;
@@ -1109,6 +1119,7 @@ int gem_fk_autotune(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_l
   float* dim = dre ? (float*)gem_ctx_aux(ctx, 9, nout * sizeof(float)) : nullptr;
   int32_t* dst = dim ? (int32_t*)gem_ctx_aux(ctx, 11, (size_t)nkf * sizeof(int32_t)) : nullptr;
   if (!dst) return GEM_ERROR;
+  TuneScope scope(ctx);
   const int b = ctx->backend == GEM_BACKEND_GPU_FAST ? 1 : 0;
   const int saved_s[3] = {ctx->sched[b][0], ctx->sched[b][1], ctx->sched[b][2]};
   const int saved_d[3] = {ctx->defer[b][0], ctx->defer[b][1], ctx->defer[b][2]};

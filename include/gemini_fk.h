@@ -229,7 +229,9 @@ int gem_fk_graph_launch(gem_ctx* ctx, void* stream);
  * schedules: 256, 384, 512, 320, 448 or 192 threads per block with the fast
  * backend, 384, 512, 256, 384, 512 or 256 with the plain one.
  * Every schedule gives bit-identical spectra.  sched3[ph] is kept per context
- * and backend; the default is {1, 0, 1}. */
+ * and backend; the default is {1, 0, 1}.  A phase of few solves runs in the fast
+ * backend's group form, several lanes per solve, which has no use for schedule,
+ * deferral and granularity (nor do they change its spectra). */
 #define GEM_FK_NSCHED 6
 int gem_fk_schedule_set(gem_ctx* ctx, const int* sched3);
 int gem_fk_schedule_get(const gem_ctx* ctx, int* sched3);
@@ -254,7 +256,8 @@ int gem_fk_queue_get(const gem_ctx* ctx, int* gran3);
 /* Autotuner: runs frequencies jf_first..jf_last once per candidate (repeats
  * times, minimum kept), first the schedules, then the deferrals under the
  * chosen schedules, then the queue granularities under both, and keeps per
- * phase the fastest of each.  ms (may be NULL,
+ * phase the fastest of each.  All runs take one lane per solve, the form that
+ * has these settings, whatever the slab's size.  ms (may be NULL,
  * (GEM_FK_NSCHED + GEM_FK_NDEFER + GEM_FK_NGRAN) * 3 floats) receives the phase
  * times in ms of every candidate, -1 for candidates not run (the plain backend
  * tries schedules 0..2 only); sched3 and defer3 (may be NULL) the choice, and

@@ -69,3 +69,19 @@ def test_group_form_of_dsv_and_set_runs(gpu, source):
         for a, b in zip(x, y):
             np.testing.assert_array_equal(a, b)
     fk.instrument(False)
+
+
+def test_autotuner_times_the_thread_form(gpu):
+    """The settings that the autotuner chooses are the thread form's: on a slab that runs in the
+    group form (96 solves, about three times faster) it times the thread form all the same."""
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, NSCHED, GeminiFK
+    m = G.model()
+    ex = G.nodes(m)
+    jre = ex.node_index(G.rec_radius)
+    fk = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST)
+    ms = fk.autotune(G.params, jre, 8, 8, repeats=3)["ms"]
+    group = []
+    for _ in range(5):
+        fk.run(G.params, jre, 8, 8)
+        group.append(fk.stats()["phase_ms"][1])
+    assert ms[:NSCHED, 1].min() > 1.5 * min(group)
