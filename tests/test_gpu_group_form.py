@@ -85,3 +85,42 @@ def test_autotuner_times_the_thread_form(gpu):
         fk.run(G.params, jre, 8, 8)
         group.append(fk.stats()["phase_ms"][1])
     assert ms[:NSCHED, 1].min() > 1.5 * min(group)
+
+
+def test_settings_of_the_thread_form_give_identical_spectra(gpu):
+    """Every schedule, deferral and granularity of the form of one lane per solve, which a run
+    with instruments takes at every size, against the group form: bit for bit."""
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, NDEFER, NGRAN, NSCHED, GeminiFK
+    m = G.model()
+    ex = G.nodes(m)
+    jre = ex.node_index(G.rec_radius)
+    fk = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST)
+    ref = fk.run(G.params, jre, 40, 52, f32=False)[2]
+    fk.instrument(True)
+    for put, n in ((fk.schedule_set, NSCHED), (fk.defer_set, NDEFER), (fk.queue_set, NGRAN)):
+        for i in range(n):
+            put([i, i, i])
+            got = fk.run(G.params, jre, 40, 52, f32=False)[2]
+            assert int(fk.instrument_read()[0][3]) > 0   # lane attempts, which the thread form counts
+            np.testing.assert_array_equal(got, ref)
+    fk.instrument(False)
+
+
+@pytest.mark.parametrize("srcs", [(-1, 1), (5, 3, -1, 1)])
+def test_granularities_of_a_set_run_in_the_thread_form(gpu, srcs):
+    """Runs of queue positions that cross from one source to the next, with one lane per solve."""
+    from gemini_unified_b200.fk import GEM_BACKEND_GPU_FAST, NGRAN, GeminiFK
+    w = dataclasses.replace(G, nnod_blocks=[4], dr_blocks=[10000.0])
+    m = w.model()
+    ex = w.nodes(m)
+    jre = ex.node_index(w.rec_radius)
+    fk = GeminiFK(m, ex, backend=GEM_BACKEND_GPU_FAST)
+    js = [jre if j < 0 else j for j in srcs]
+    ref = fk.aski_spectra(w.params, js, jre, 3, 6, f32=False)
+    fk.instrument(True)
+    for q in range(NGRAN):
+        fk.queue_set([q, q, q])
+        for a, b in zip(fk.aski_spectra(w.params, js, jre, 3, 6, f32=False), ref):
+            for x, y in zip(a, b):
+                np.testing.assert_array_equal(x, y)
+    fk.instrument(False)
