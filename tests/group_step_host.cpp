@@ -5,6 +5,7 @@
 // another lane's is reported.
 //   group_step_host race      every system, steps that reach the seventh attempt
 //   group_step_host compare   step sizes over many decades: group form = thread form, bit for bit
+//   group_step_host status    statuses of a set of sources after its adjoint phase
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -191,6 +192,32 @@ template <int PH, int SYS, bool ISO> int compare() {
   return bad;
 }
 
+// item k of nkf, sources: two of moments, the force.  Failures: item 0 none, item 1 the toroidal or
+// spheroidal phase, item 2 the second source, item 3 the first and the force, item 4 the force
+static int set_status() {
+  constexpr int NKF = 5, NN = 3, BLK = NKF * 20 * NN, FBLK = NKF * 10 * NN;
+  int status[NKF] = {0, 7, 0, 0, 0}, src[3 * NKF] = {0, 0, 0, 2, 0, 0, 0, 1, 0, 0, 0, 0, 0, 3, 1};
+  const int want[NKF] = {0, 7, 1, 2, 1}, from[NKF] = {3, 3, 2, 1, 3};   // first source whose block is cleared
+  std::vector<double2> g64(2 * BLK + FBLK, double2{1.0, 1.0});
+  std::vector<float> re(g64.size(), 1.0f), im(re);
+  FKLaunch L{};
+  L.nkf = NKF; L.nsrc = 3; L.src_blk = BLK; L.status = status; L.status_src = src;
+  L.gf64 = g64.data(); L.gfre = re.data(); L.gfim = im.data();
+  L.src_type[0] = L.src_type[1] = 1;
+  blockDim.x = 128;
+  for (threadIdx.x = 0; threadIdx.x < 128; ++threadIdx.x) fk_set_status_kernel(L, NN);
+  int bad = memcmp(status, want, sizeof want) != 0;
+  for (int b = 0; b < 3; ++b) {
+    const int nsp = b < 2 ? 20 : 10, nsph = b < 2 ? 16 : 8;   // the toroidal spectra, the last ones of a node, stay
+    for (int o = 0; o < NKF * nsp * NN; ++o) {
+      const int k = o % NKF, q = o / NKF % nsp, at = b * BLK + o;
+      const double v = b >= from[k] && q < nsph ? 0.0 : 1.0;
+      bad += g64[at].x != v || g64[at].y != v || re[at] != v || im[at] != v;
+    }
+  }
+  return bad;
+}
+
 int main(int argc, char** argv) {
   setup();
   if (argc > 1 && !strcmp(argv[1], "race")) {
@@ -202,6 +229,7 @@ int main(int argc, char** argv) {
     race<PH_ADJ, SYS_SOLIDT, true>();
     return 0;
   }
+  if (argc > 1 && !strcmp(argv[1], "status")) return set_status();
   const int bad = compare<PH_TOR, SYS_TOROIDAL, true>() + compare<PH_SPH, SYS_MINORS, false>() +
                   compare<PH_SPH, SYS_RADIAL, true>() + compare<PH_ADJ, SYS_SOLIDT, true>();
   printf("steps by attempts:");

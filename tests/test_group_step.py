@@ -1,5 +1,5 @@
 """The group form's step (csrc/fk_group.cuh) compiled for the host, one warp on 32
-threads (group_step_host.cpp)."""
+threads, and the statuses of a set of sources (group_step_host.cpp)."""
 import os
 import shutil
 import subprocess
@@ -38,3 +38,9 @@ def test_group_form_equals_thread_form(tmp_path):
     group form makes more attempts than the thread form and may use no more of them."""
     r = subprocess.run([_build(tmp_path, "-O2"), "compare"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_status_of_a_set_of_sources(tmp_path):
+    """An item takes the status of its first source that failed; the spheroidal spectra of the
+    sources after it are cleared, the blocks before it and the toroidal spectra stay."""
+    assert subprocess.run([_build(tmp_path, "-O1"), "status"]).returncode == 0
