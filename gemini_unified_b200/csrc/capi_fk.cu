@@ -541,7 +541,7 @@ int fk_prepare(gem_ctx* ctx, const gem_fk_params* p, int jf_first, int jf_last, 
 // form's settings, which the group form has no use for.
 bool use_groups(const gem_ctx* ctx, const SlabPlan& S, int ph, const FKLaunch& L) {
   if (!S.fast || ctx->tuning || ctx->d_prof || ctx->d_warp_ns || ctx->d_steplog) return false;
-  return (long long)L.nqueue <= FK_GROUP_MAX[S.P.hascore][ph];
+  return (long long)L.nqueue <= fk_group_max(S.P.hascore != 0, ph, S.P.nnod);
 }
 
 // The device work of one slab on stream st: zeroing, model preparation, start

@@ -7,29 +7,36 @@
 namespace gem {
 
 // Schedules of a solver phase kernel: threads per block (one block per SM) of
-// the plain and of the fast build.  The autotuner picks one per phase; the
-// defaults are the fastest of the first three at the batched configuration
-// (fast build, toroidal / spheroidal / adjoint phase in ms: 256 threads 65.6 /
-// 203 / 107, 384 threads 56.2 / 210 / 99.8, 512 threads 55.3 / 210 / 108; of
-// small slabs every phase is fastest at 256).  The plain build tries 0..2 only.
+// the plain and of the fast build.  The autotuner picks one per phase.  Batched
+// configuration, fast build, toroidal / spheroidal / adjoint phase in ms: 256
+// threads 65.6 / 203 / 107, 384 threads 56.2 / 210 / 99.8, 512 threads 55.3 /
+// 210 / 108; the defaults are the fastest but for the toroidal phase, where 512
+// threads are 0.9 ms faster.  The plain build tries 0..2 only.
 constexpr int FK_NSCHED = 6;
 constexpr int FK_SCHED_BLOCK[2][FK_NSCHED] = {{384, 512, 256, 384, 512, 256}, {256, 384, 512, 320, 448, 192}};
 constexpr int FK_SCHED_DEFAULT[3] = {1, 0, 1};   // toroidal, spheroidal, adjoint
 // Largest number of solves a phase of the fast build runs in the group form, 16
-// or 8 lanes per solve (models without and with a fluid core; toroidal,
-// spheroidal, adjoint).  The thread form takes the time of the longest solve
+// or 8 lanes per solve.  The thread form takes the time of the longest solve
 // whatever the number below its 37,888 lanes, the group form's grows with the
-// solves once its 3,552 groups are busy.  Thread and group form in ms:
-//   PREM to 0.2 Hz    3,206 solves 11.8 / 49 / 12.8 and 4.1 / 16.8 / 4.3,
-//                    22,278 solves 11.1 / 53 / 15.1 and 6.3 / 30 / 15.6;
-//   PREM to 0.05 Hz   4,601 solves 2.6 / 14.0 / 0.35 and 1.1 / 4.1 / 0.28,
-//                    17,961 solves 2.8 / 13.7 / 0.37 and 1.5 / 7.1 / 0.76;
-//   crust to 2 Hz     9,517 solves 2.0 / 4.7 / 7.5 and 0.9 / 3.1 / 4.4,
-//                    21,988 solves 2.1 / 4.8 / 7.7 and 1.9 / 6.7 / 9.3.
-// The lines lie where the slowest model of the kind breaks even: solves of a
-// model with a core differ more in length, and short integrations (adjoints,
-// a crust) spend more in the bookkeeping, which one lane of a group does.
-constexpr int FK_GROUP_MAX[2][3] = {{16000, 9000, 8000}, {24000, 22000, 8000}};
+// solves once its 3,552 groups are busy, so the two break even at the number
+// that the groups do in the time of the longest solve's chain.  Both forms were timed
+// on slabs of 2,000 to 65,000 solves at the top and at the middle of a band, PREM to
+// 0.02 .. 0.2 Hz and a crust to 0.4 .. 2 Hz, isotropic or not; per model the break-even lies at
+//   with a core     toroidal 36,700 .. 48,000   spheroidal 25,500 .. 49,700
+//   without         toroidal 18,100 .. 24,400   spheroidal  9,900 .. 15,500
+// and the line at or below the least of them (ms, thread and group form: PREM to 0.2 Hz, 22,278
+// solves, toroidal 11.1 and 6.1, spheroidal 55.7 and 30.1; PREM to 0.02 Hz, 26,500,
+// spheroidal break-even 25,500; crust to 1 Hz, 9,331, spheroidal 2.84 and 2.18).
+// An adjoint solve stops at every node, so the thread form's chain grows with the
+// nodes and the break-even with it: 4 nodes 7,400 .. 7,900, 11 nodes 8,300 ..
+// 10,400 (crust 11,400), 32 nodes 15,200 .. 19,800, 37 nodes 16,800 .. 21,700.  With 4 nodes
+// the group form is behind as soon as a third solve per group begins, at 7,104 (0.40 and
+// 0.35 ms); a set of sources on 11 nodes gains up to the line (7,635 positions: 7.3 and 8.6 ms for the call).
+constexpr int FK_GROUP_MAX[2][3] = {{18000, 9500, 8000}, {36000, 25000, 8000}};   // without and with a core
+constexpr int FK_GROUP_NODES = 30, FK_GROUP_MAX_ADJ = 13500;                       // adjoint phase of many nodes
+constexpr int fk_group_max(bool core, int phase, int nnod) {
+  return phase == 2 && nnod >= FK_GROUP_NODES ? FK_GROUP_MAX_ADJ : FK_GROUP_MAX[core][phase];
+}
 // candidate deferrals of the bookkeeping passes (lanes waiting, trips waited);
 // the last waits for the whole warp: its lanes, on adjacent degrees of one
 // frequency, reach their sub-interval ends within a few steps of each other
