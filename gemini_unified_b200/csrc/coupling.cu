@@ -626,12 +626,15 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   const bool fast = gem_ctx_backend(ctx) == GEM_BACKEND_GPU_FAST;   // the tensor-core sums store no coefficient rows
   const size_t b_a = fast ? 0 : align256((size_t)ao * sizeof(double));
   const size_t b_hd = align256((size_t)co * sizeof(double));
+  // the tables' exponents are done with before the products write the sums
+  const size_t texp_bytes = (size_t)npts * CPL_NKIND * lcap * sizeof(short);
+  const bool texp_in_sums = texp_bytes <= b_hd;
   const size_t b_x = align256((size_t)npts * 6 * p->nf2 * sizeof(double2));
   const size_t b_in = align256((size_t)nf * sizeof(int)) + align256((size_t)p->nf2 * sizeof(int)) +
                       3 * align256((size_t)npts * 3 * sizeof(double)) + align256(evf.size() * sizeof(double2)) +
                       align256((size_t)p->nf2 * 7 * sizeof(double2)) +
                       (fast ? align256(((size_t)2 * lcap + k) * sizeof(double)) +
-                                  align256((size_t)npts * CPL_NKIND * lcap * sizeof(short))
+                                  (texp_in_sums ? 0 : align256(texp_bytes))
                             : 0);
   char* ws = (char*)gem_ctx_aux(ctx, 12, b_tab + b_a + b_hd + b_x + b_in);
   if (!ws) return GEM_ERROR;
@@ -649,7 +652,7 @@ extern "C" int gem_coupling_run_device(gem_ctx* ctx, const gem_coupling_params* 
   double2* d_evf = (double2*)take(evf.size() * sizeof(double2));
   double2* d_zel = (double2*)take((size_t)p->nf2 * 7 * sizeof(double2));
   double* wtab = fast ? (double*)take(((size_t)2 * lcap + k) * sizeof(double)) : nullptr;
-  short* texp = fast ? (short*)take((size_t)npts * CPL_NKIND * lcap * sizeof(short)) : nullptr;
+  short* texp = !fast ? nullptr : (texp_in_sums ? (short*)C : (short*)take(texp_bytes));
   if (cudaMemcpyAsync(d_koff, koff.data(), (size_t)nf * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_nwn, nwn, (size_t)p->nf2 * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_delta, delta, (size_t)npts * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess ||

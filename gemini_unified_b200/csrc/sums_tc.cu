@@ -555,6 +555,7 @@ bool make_map(CUtensorMap* map, const signed char* base, long long rows, long lo
 
 struct TcLayout {
   int Kp;
+  bool part_in_tab;   // the partial sums take the place of the table, which is used up when they are written
   size_t off[11], total;
 };
 
@@ -566,6 +567,8 @@ TcLayout tc_layout(const TcProblem& P, long long mtot) {
   L.Kp = (K + 63) / 64 * 64;   // the slicing kernels work on 64-degree tiles
   const int bn = ns == TC_S_FINE ? TC_BN_FINE2 : TC_BN2;
   const bool two = P.ncol > (ns == TC_S_FINE ? TC_BN_FINE : TC_BN);   // launches of the products
+  const size_t part = two ? (size_t)(mtot / TC_BM + nk + 1) * ((P.ncol + bn - 1) / bn) * TC_BM * bn * sizeof(double) : 0;
+  L.part_in_tab = part <= (size_t)nk * P.lcap * P.ncol * sizeof(double);
   const size_t sz[11] = {(size_t)ns * nk * P.ncol * L.Kp,             // T8
                         (size_t)ns * mtot * L.Kp,                     // A8
                         (size_t)nk * L.Kp * sizeof(double),           // lscale
@@ -576,7 +579,7 @@ TcLayout tc_layout(const TcProblem& P, long long mtot) {
                         (size_t)3 * TC_MAX_KIND * sizeof(long long),  // per-kind tables
                         (size_t)(TC_MAX_KIND + 8) * sizeof(int),      // kind rows + error flag
                         (size_t)nk * P.ncol * sizeof(int),            // column maxima
-                        two ? (size_t)(mtot / TC_BM + nk + 1) * ((P.ncol + bn - 1) / bn) * TC_BM * bn * sizeof(double) : 0};   // part
+                        L.part_in_tab ? 0 : part};                    // partial sums
   size_t b = 0;
   for (int i = 0; i < 11; ++i) {
     L.off[i] = b;
@@ -676,16 +679,16 @@ const char* tc_slice_and_multiply(const TcProblem& P, long long mtot, int K, int
   return nullptr;
 }
 
-// Sliced-integer sums: from the FP64 tables tab[kind][l][col] with their exponents texp and the coefficient
-// rows that coefs launches, write C[kind][row][col] in FP64.  ws: device workspace of
-// sums_tc_workspace bytes; wait_ns: limit of each pipeline wait (0: 1 s).
-// Blocking (synchronises the stream).
 cudaError_t tc_exponents_launch(const double* tab, long long n, short* texp, cudaStream_t st) {
   tab_exponent_kernel<<<148 * 16, 256, 0, st>>>(tab, n, texp);
   return cudaGetLastError();
 }
 
-const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const short* texp,
+// Sliced-integer sums: from the FP64 tables tab[kind][l][col] with their exponents texp and the coefficient
+// rows that coefs launches, write C[kind][row][col] in FP64.  tab and texp hold nothing of use afterwards;
+// texp may lie in C.  ws: device workspace of sums_tc_workspace bytes; wait_ns: limit of each pipeline wait
+// (0: 1 s).  Blocking (synchronises the stream).
+const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, double* tab, const short* texp,
                         const TcCoefs& coefs,
                         double* C, void* ws, size_t ws_bytes, unsigned long long wait_ns, cudaStream_t st) {
   if (P.nkind < 1 || P.nkind > TC_MAX_KIND) return "sums_tc: table kinds outside 1..16";
@@ -709,7 +712,7 @@ const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, cons
   int* ints = (int*)(base + L.off[8]);   // [0..15] rows per kind, [16] error flag
   short* lexp = (short*)(base + L.off[5]);
   int* colmax = (int*)(base + L.off[9]);
-  double* part = (double*)(base + L.off[10]);
+  double* part = L.part_in_tab ? tab : (double*)(base + L.off[10]);
   int krows[TC_MAX_KIND + 8] = {0};
   long long htabs[3 * TC_MAX_KIND] = {0};
   std::vector<int4> htiles;

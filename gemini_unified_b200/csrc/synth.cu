@@ -791,6 +791,9 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   const long long ntr = (long long)nsta * nmt * 3;
   // all buffers of one run in one context-owned allocation, grown on demand
   const bool o_tred = o && o->tred, o_ns = o && o->nsamp_true, o_sf = o && o->stafilter;
+  // the tables' exponents are done with before the products write the sums
+  const size_t texp_bytes = (size_t)8 * S.lcap * nsta * sizeof(short);
+  const bool texp_in_sums = texp_bytes <= (size_t)co * sizeof(double);
   const size_t sizes[20] = {(size_t)8 * S.lcap * nsta * sizeof(double), fast ? 0 : (size_t)ao * sizeof(double),
                             (size_t)co * sizeof(double), (size_t)ntr * S.ldx * sizeof(double2),
                             evf.size() * sizeof(double2), tw.size() * sizeof(double2),
@@ -800,7 +803,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
                             fast_fft ? ifft_fast_twiddle_bytes(ns) : 0,
                             o_tred ? nsta * sizeof(double) : 0, o_ns ? nsta * sizeof(int) : 0,
                             o_sf ? (size_t)nsta * 3 * p->nf2 * sizeof(double2) : 0, (size_t)nstf * sizeof(float),
-                            fast ? (size_t)8 * S.lcap * nsta * sizeof(short) : 0,
+                            fast && !texp_in_sums ? texp_bytes : 0,
                             fast ? ((size_t)2 * S.lcap + kk) * sizeof(double) : 0};
   // the small inputs lie together, so that one copy brings them all (sixteen of a few KB each took
   // about a fifth of a call with 50 stations)
@@ -827,7 +830,7 @@ int synth_run(gem_ctx* ctx, const gem_synth_params* p, const int* nwn, const flo
   b.koff = (int*)parts[8]; b.theta = (double*)parts[9]; b.phi = (double*)parts[10]; b.propdir = (double*)parts[11];
   b.mt = (double*)parts[12]; b.twx = (double2*)parts[13];
   cudaMemcpyAsync(pool, in.data(), nin, cudaMemcpyHostToDevice, st);
-  short* texp = (short*)parts[18];
+  short* texp = texp_in_sums ? (short*)b.C : (short*)parts[18];
   double* wtab = (double*)parts[19];
   S.nwn = b.nwn; S.koff = b.koff;
   S.tred_sta = o_tred ? (const double*)parts[14] : nullptr;

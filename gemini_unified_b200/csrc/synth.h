@@ -106,7 +106,7 @@ TcProblem tc_problem_of(const SynthDev& S);   // the synthetics' 8 Legendre / Be
 // workspace size and run; nwn: host copy of the wavenumber counts per frequency
 // (1-based frequency index); wait_ns: limit of each pipeline wait (0: 1 s)
 size_t sums_tc_workspace(const TcProblem& P, long long mtot, int* Kp_out);
-const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, const double* tab, const short* texp,
+const char* sums_tc_run(const TcProblem& P, const int* nwn, long long mtot, double* tab, const short* texp,
                         const TcCoefs& coefs,
                         double* C, void* ws, size_t ws_bytes, unsigned long long wait_ns, cudaStream_t st);
 

@@ -69,3 +69,10 @@ def test_coupling(fk, n, npts):
     assert np.array_equal(np.isfinite(got), ok)
     top = np.where(ok, np.abs(ref), 0.0).max(axis=2, keepdims=True)
     assert np.all(np.abs(got - ref)[ok] <= np.broadcast_to(1e-8 * top, ok.shape)[ok])
+
+
+@pytest.mark.parametrize("nsta", [81, 200])
+def test_partial_sums_beside_the_tables(fk, nsta):
+    """Many frequencies of few degrees: the partial sums of the two launches do not fit the tables."""
+    test_synthetics(fk, 35, nsta)
+    test_coupling(fk, 35, nsta)

@@ -67,3 +67,34 @@ def test_wait_limit_in_the_two_launch_form(ctx):
         _synthetics(ctx, 2, 200)
     fk.tc_wait_limit(0)
     test_synthetics_at_tile_edges(ctx, 200)
+
+
+def test_device_memory_of_a_call(ctx):
+    """A call holds the FP64 tables and sums, the slices of both operands, the spectra and small
+    inputs, and no more than the coefficient rows besides (20000 stations: 1.15 GB; the tables'
+    exponents and the partial sums of the two launches would add 0.44 GB)."""
+    import ctypes
+    import torch
+    from gemini_unified_b200.fk import FrequencyTime, lib, synth_params
+    g, gr, gi, _ = ctx
+    rng = np.random.default_rng(3)
+    sp = synth_params(g, 10, 512, 1.0 / (512 * g.df), W.filspecs)
+    ft = FrequencyTime(backend=2)
+    d = [torch.from_numpy(np.ascontiguousarray(a[:10])).cuda() for a in (gr, gi)]
+    nwn, mt = np.ascontiguousarray(g.nwn, np.int32), np.ascontiguousarray(np.eye(6)[[1]])
+    vp = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    free = []
+    for n in (200, 20000):
+        out = torch.empty((n, 1, 3, 512), dtype=torch.float32, device="cuda")
+        theta = np.radians(rng.uniform(1.0, 170.0, n))
+        phi, prop = rng.uniform(-3.0, 3.0, n), rng.uniform(-3.0, 3.0, n)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+        assert lib().gem_synth_run_device(ft._h, ctypes.byref(sp), vp(nwn), d[0].data_ptr(), d[1].data_ptr(), n, vp(theta), vp(phi),
+                                          vp(prop), 1, vp(mt), out.data_ptr(), None) < 2
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    nf, lcap = g.nf2 - g.nf1 + 1, int(g.nwnmax)
+    kp, rows = -(-lcap // 64) * 64, 2 * nf * 14
+    most = n * (8 * lcap * 8 + rows * 8 + 3 * g.nf2 * 16 + 6 * 8 * kp) + rows * (6 * kp + 8 * lcap)
+    assert free[2] - free[3] <= most + (8 << 20)   # allocations come in steps of 2 MB
