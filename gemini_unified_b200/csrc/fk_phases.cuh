@@ -21,9 +21,10 @@
 // so the lockstep Bulirsch-Stoer step keeps the whole warp busy: lanes refill
 // from the phase's work queue as soon as their item is done.  Each lane walks
 // its item as a small state machine (bookkeeping runs divergently between two
-// lockstep steps).  The Neville tableau is built incrementally, one new
-// diagonal per attempt (the exact values the reference recomputes from
-// scratch), and kept in shared memory, lane-interleaved.
+// lockstep steps).  Shared memory holds, lane-interleaved, what the extrapolation
+// of a step reads: the results of the attempts 1, 2, 3 and 5 in the fast build, in
+// the plain build the Neville tableau, built incrementally, one new diagonal per
+// attempt (the exact values the reference recomputes from scratch).
 #pragma once
 #include "fk_kernel.h"
 #include "fk_solver.cuh"
